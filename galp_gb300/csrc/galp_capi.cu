@@ -409,6 +409,12 @@ int Engine::setup(const galp_csr &g, const galp_opts &o, cudaStream_t st, int64_
     if ((rc = upload(b_schunk_big, d_schunk_big, sched.schunk_big, st, h2d))) return rc;
     if ((rc = upload(b_schunk_s0, d_schunk_s0, sched.schunk_s0, st, h2d))) return rc;
     if ((rc = upload(b_schunk_s1, d_schunk_s1, sched.schunk_s1, st, h2d))) return rc;
+    for (const Scope &sc : sched.scopes)  // degree order within windows of the small-vertex lists
+        if (sc.nsv) {
+            small_window_kernel<<<(unsigned)std::min<int64_t>((sc.nsv + kSmallWindow - 1) / kSmallWindow, 4096),
+                                  kSmallWindow, 0, st>>>(d_small_v + sc.sv0, sc.nsv, (const int64_t *)b_off.p);
+            GALP_CUDA(cudaGetLastError());
+        }
     if ((rc = setup_hub_parts(variant.hub_part_shift, st, h2d))) return rc;
     // per-vertex state, spill and tied lists
     const size_t nn = (size_t)std::max<int64_t>(n, 1);
@@ -778,9 +784,10 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     if (prof.on) e0 = prof.mark(st);
     if (q.npacks && variant.small_sort == 2) {
         // one thread per small vertex, over the small-vertex list
-        const int blocks = (int)std::min<int64_t>(((int64_t)q.nsmall + 127) / 128, (int64_t)sms * kSmallLaneBlocks);
-        count_small_lane_kernel<<<blocks, 128, 0, st>>>(q);
-        launched("count_small_lane_kernel", st);
+        const int blocks = (int)std::min<int64_t>(((int64_t)q.nsmall + kSmallThreads - 1) / kSmallThreads,
+                                                  (int64_t)sms * kSmallBlocks);
+        count_small_sort_kernel<<<blocks, kSmallThreads, 0, st>>>(q);
+        launched("count_small_sort_kernel", st);
     } else if (q.npacks) {
         // several waves: blocks that finish early take up the remaining ones (pack costs vary)
         const int blocks = (int)std::min<int64_t>(((int64_t)q.npacks * 32 + 255) / 256, (int64_t)sms * small_bps);

@@ -65,7 +65,8 @@ struct Scope {
 struct Schedule {
     std::vector<int32_t> pack_v0;    // first vertex of each pack (<= 32 vertices, <= 32 edges)
     std::vector<uint8_t> pack_nv;    // vertices in each pack
-    std::vector<int32_t> small_v;    // per scope: the pack vertices one by one, in vertex order
+    std::vector<int32_t> small_v;    // per scope: the pack vertices one by one, in vertex order (the device
+                                     // copy is then ordered by degree within windows)
     std::vector<int32_t> mid_v;      // per scope: mid, large and xl vertices in ascending degree
     std::vector<int32_t> mid_deg;    // degree of each mid_v entry
     std::vector<int32_t> big_v;      // vertex of each big entry

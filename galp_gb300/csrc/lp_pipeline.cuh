@@ -26,6 +26,8 @@
 //   occupied entries unsorted (queried by order statistics).
 #pragma once
 
+#include <utility>
+
 #include "rmat_rng.h"
 #include "lp_kernels.cuh"
 #include "lp_dispatch.cuh"
@@ -56,7 +58,7 @@ struct PipeArgs {
     const int32_t *pack_v0;
     const uint8_t *pack_nv;
     int32_t npacks;
-    const int32_t *small_v; // the same vertices one by one (thread-per-vertex counting)
+    const int32_t *small_v; // the same vertices one by one, in order of degree within windows
     int32_t nsmall;
     const int32_t *mid_v;   // mid (33..256), then large (257..2048), then xl (2049..12288) vertices
     int32_t nmid_s, nmid_l, nmid_x;
@@ -89,7 +91,7 @@ struct PipeArgs {
     int32_t ngraphs;
     int32_t lab27;          // every label below 2^27 - 1 (32-bit sort keys in packs)
     int32_t small_sort;     // small vertices: 0 match-based packs, 1 sort-based packs (needs lab27),
-                            // 2 one thread per vertex
+                            // 2 one thread per vertex, sorted in registers
     int32_t narrow_cut;     // -1, or the mid-list position of the first vertex above kNarrowMax
                             // neighbours: the 128-thread CTA range is split there, its lower
                             // part going to 64-thread CTAs
@@ -602,28 +604,149 @@ __device__ __forceinline__ void tbuf_append(int32_t *buf, int *n, int32_t value,
     buf[(*n)++] = value;
 }
 
-// Small vertices (at most 32 neighbours), one thread each (`small_sort` 2): a vertex's
-// neighbour labels go to the thread's 32-entry row of shared memory (element j of lane l at
-// l * 32 + (j ^ l): the lanes' rows are bank-disjoint), are sorted there by insertion, and
-// one pass over the sorted row gives the distinct count, the runs' counts, the maximum, the
-// candidates and the ranks of the smallest and largest candidate; vertices with more than
-// two candidates spill their runs in label order, as the pack kernel does.  Against the
-// warp-per-pack kernel this spends per vertex a few instructions per neighbour instead of
-// the per-pack segment masks, matches and segmented shuffles.
-constexpr int kSmallLaneBlocks = 8;  // resident 128-thread blocks per SM (16 KB of rows each)
-__global__ void __launch_bounds__(128, kSmallLaneBlocks) count_small_lane_kernel(PipeArgs p)
+// ----- sorting networks in registers -----
+// Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their applications",
+// 1968) for the next power of two, cut to the first N wires: the wires above would hold the
+// largest keys and never exchange.  The comparators are compile-time constants, so a network
+// is straight-line code of one min and one max per comparator.
+struct NetPair {
+    int a, b;
+};
+template <int N>
+struct SortNet {
+    static __host__ __device__ constexpr int pow2()
+    {
+        int p = 1;
+        while (p < N) p *= 2;
+        return p;
+    }
+    // the c-th comparator, or with c < 0 the number of comparators in .a
+    static __host__ __device__ constexpr NetPair get(int c)
+    {
+        const int P = pow2();
+        int at = 0;
+        for (int p = 1; p < P; p *= 2)
+            for (int k = p; k >= 1; k /= 2)
+                for (int j = k % p; j + k < P; j += 2 * k)
+                    for (int i = 0; i < k && i + j + k < P; ++i)
+                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p) && i + j + k < N) {
+                            if (at == c) return NetPair{i + j, i + j + k};
+                            ++at;
+                        }
+        return NetPair{at, 0};
+    }
+    static constexpr int size = get(-1).a;
+    template <int C>
+    static __device__ __forceinline__ void step(int32_t (&x)[N])
+    {
+        constexpr NetPair q = get(C);
+        const int32_t lo = min(x[q.a], x[q.b]), hi = max(x[q.a], x[q.b]);
+        x[q.a] = lo;
+        x[q.b] = hi;
+    }
+    template <int... C>
+    static __device__ __forceinline__ void steps(int32_t (&x)[N], std::integer_sequence<int, C...>)
+    {
+        (step<C>(x), ...);
+    }
+    static __device__ __forceinline__ void sort(int32_t (&x)[N])
+    {
+        steps(x, std::make_integer_sequence<int, size>{});
+    }
+};
+
+// Row of a small vertex in its warp's shared memory: 36 words, so that the 16-byte accesses
+// of 8 lanes to their own rows fall in distinct banks.
+constexpr int kSmallRow = 36;
+
+// Sort the first N words of a lane's row in registers, write them back and return the mask
+// of positions that differ from the one before (position 0 always set).
+template <int N>
+__device__ __forceinline__ uint32_t small_sort_row(int32_t *row)
 {
-    __shared__ int32_t rows[4][32 * 32];
-    __shared__ int32_t tbuf[4][kWarpBuf];
+    int32_t x[N];
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+        const int4 q = *reinterpret_cast<const int4 *>(row + j);
+        x[j] = q.x;
+        x[j + 1] = q.y;
+        x[j + 2] = q.z;
+        x[j + 3] = q.w;
+    }
+    SortNet<N>::sort(x);
+    uint32_t h = 1u;
+#pragma unroll
+    for (int j = 1; j < N; ++j)
+        if (x[j] != x[j - 1]) h |= 1u << j;
+#pragma unroll
+    for (int j = 0; j < N; j += 4) *reinterpret_cast<int4 *>(row + j) = make_int4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+    return h;
+}
+
+// Order every window of kSmallWindow entries of a scope's small-vertex list by degree
+// (stable), once per graph: a warp's 32 vertices then have about equal degrees, while their
+// neighbour lists and per-vertex outputs stay within the window's few cache lines.
+constexpr int kSmallWindow = 128;
+__global__ void __launch_bounds__(kSmallWindow) small_window_kernel(int32_t *small_v, int nsmall, const int64_t *off)
+{
+    __shared__ uint8_t sdeg[kSmallWindow];
+    const int tid = threadIdx.x;
+    for (int64_t w0 = (int64_t)blockIdx.x * kSmallWindow; w0 < nsmall; w0 += (int64_t)gridDim.x * kSmallWindow) {
+        const int cnt = (int)min((int64_t)kSmallWindow, nsmall - w0);
+        int v = 0, deg = 0;
+        if (tid < cnt) {
+            v = small_v[w0 + tid];
+            deg = (int)(off[v + 1] - off[v]);
+            sdeg[tid] = (uint8_t)deg;
+        }
+        __syncthreads();
+        if (tid < cnt) {
+            int r = 0;
+            for (int i = 0; i < cnt; ++i) r += sdeg[i] < deg || (sdeg[i] == deg && i < tid);
+            small_v[w0 + r] = v;
+        }
+        __syncthreads();
+    }
+}
+
+// Small vertices (at most 32 neighbours; `small_sort` 2): a warp takes 32 vertices of about
+// equal degree (small_window_kernel), gathers their labels together and sorts each vertex's
+// labels in one lane's registers.
+//
+//   gather  32 CSR entries per row whatever vertices they belong to, eight rows in flight;
+//           the owner of an entry follows from the mask of vertex starts in its row; labels
+//           go to the owner's row of shared memory (padded with INT_MAX, no label).
+//   sort    a network sized to the warp's largest degree in steps of 4; the mask h of run
+//           heads gives everything else: d = popc(h), and the heads m of runs of maximum
+//           length W by W steps of m & (continuations >> W).
+//   spill   vertices with more than two candidates keep their sorted labels at their CSR
+//           positions and h, m in place of the candidate labels (SmallMaskQuery).
+//
+// Bound by the load/store pipe (70 % of its wavefronts on planted partitions of degree 15:
+// the label gathers alone are 32 per row), then by the latency of the two dependent loads.
+// A warp has the order of its vertices to itself, so there is no barrier between warps: a
+// version that ordered 128 vertices inside the block, with three barriers and per-lane
+// result selects, took 42 ms where this one takes 25.  Ten iterations, this kernel's share
+// (an insertion sort per thread in shared memory before): 1,024 planted partitions of
+// together 526 M entries 55.5 -> 24.9 ms, R-MAT 24 9.8 -> 4.4 ms, R-MAT 26 with edge
+// factor 4 20.2 -> 11.5 ms, LFR of a million vertices 2.0 -> 0.73 ms.
+constexpr int kSmallThreads = 128;
+constexpr int kSmallBlocks = 8;  // resident blocks per SM
+__global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_kernel(PipeArgs p)
+{
+    constexpr int NW = kSmallThreads / 32;
+    __shared__ __align__(16) int32_t srow[NW][32 * kSmallRow];
+    __shared__ int64_t sdlt[NW][32];   // CSR position minus slot, of the i-th vertex with neighbours
+    __shared__ int32_t sat[NW][32];    // its row minus its first slot
+    __shared__ uint32_t smask[NW][32]; // vertex starts in each row of slots
+    __shared__ int32_t tbuf[NW][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t *row = rows[w] + lane * 32;
+    int32_t *rows = srow[w];
     WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
-    const int stride = gridDim.x * 128;
-    // warp-uniform trip count: every lane runs the loop the same number of times
-    // a lane's next vertex: index, offsets, label and dirty flag load one round ahead
+    // the next round's vertex, offsets, label and dirty flag load one round ahead
     struct Head {
         int v, deg;
         int64_t o0;
@@ -631,7 +754,7 @@ __global__ void __launch_bounds__(128, kSmallLaneBlocks) count_small_lane_kernel
         int dirty;
     };
     auto head = [&](int i) {
-        Head h{0, 0, 0, 0, 1};
+        Head h{-1, 0, 0, 0, 1};
         if (i < p.nsmall) {
             h.v = p.small_v[i];
             h.o0 = __ldg(&p.off[h.v]);
@@ -641,98 +764,138 @@ __global__ void __launch_bounds__(128, kSmallLaneBlocks) count_small_lane_kernel
         }
         return h;
     };
-    Head nxt = head(blockIdx.x * 128 + w * 32 + lane);
-    for (int base = blockIdx.x * 128 + w * 32; base < p.nsmall; base += stride) {
-        const int i = base + lane;
-        const bool active = i < p.nsmall;
-        const Head h = nxt;
-        nxt = head(i + stride);
-        const int v = h.v;
+    // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
+    // window in turn, so that none has only the window's highest degrees
+    const int stride = gridDim.x * kSmallThreads;
+    int turn = w;
+    Head nxt = head(blockIdx.x * kSmallThreads + turn * 32 + lane);
+    for (int base = blockIdx.x * kSmallThreads; base < p.nsmall; base += stride) {
+        const Head hd = nxt;
+        turn = (turn + 1) & (NW - 1);
+        nxt = head(base + stride + turn * 32 + lane);
+        const int v = hd.v;
+        const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
+        // slots: lane's entries at [pos, pos + deg) of the warp's total
+        int pos = deg;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, pos, o);
+            if (lane >= o) pos += y;
+        }
+        const int total = __shfl_sync(kFull, pos, 31);
+        pos -= deg;
+        smask[w][lane] = 0u;
+        const unsigned nz = __ballot_sync(kFull, deg > 0);
+        const int rank = __popc(nz & ((1u << lane) - 1u));
+        const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
+        __syncwarp();
+        if (deg > 0) {
+            sdlt[w][rank] = hd.o0 - p.nbr_shift - pos;
+            sat[w][rank] = lane * kSmallRow - pos;
+            atomicOr(&smask[w][pos >> 5], 1u << (pos & 31));
+        }
+        for (int j = 0; j < n4; ++j)
+            *reinterpret_cast<int4 *>(rows + lane * kSmallRow + 4 * j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+        __syncwarp();
+        const uint32_t rmask = smask[w][lane];  // lane r: starts in row r ...
+        int rbefore = __popc(rmask);            // ... and in the rows before it
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, rbefore, o);
+            if (lane >= o) rbefore += y;
+        }
+        rbefore -= __popc(rmask);
+        // index of the vertex that owns slot s = row * 32 + lane (warp-collective)
+        auto owner = [&](int row) {
+            const uint32_t starts = __shfl_sync(kFull, rmask, row);
+            return __shfl_sync(kFull, rbefore, row) + __popc(starts & ((2u << lane) - 1u)) - 1;
+        };
+        constexpr int PER = 8;
+        for (int r0 = 0; r0 * 32 < total; r0 += PER) {
+            int id[PER], at[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                id[u] = -1;
+                if ((r0 + u) * 32 >= total) continue;  // warp-uniform
+                const int s = (r0 + u) * 32 + lane;
+                const int own = owner(r0 + u);
+                if (s < total) {
+                    id[u] = ld_nbr(&p.nbr[sdlt[w][own] + s]);
+                    at[u] = sat[w][own] + s;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u)
+                if (id[u] >= 0) rows[at[u]] = ld_label(&p.lab_in[id[u]]);
+        }
+        __syncwarp();
+        int32_t *row = rows + lane * kSmallRow;
+        uint32_t h = 0u;
+        switch (n4) {  // warp-uniform
+        case 0: break;
+        case 1: h = small_sort_row<4>(row); break;
+        case 2: h = small_sort_row<8>(row); break;
+        case 3: h = small_sort_row<12>(row); break;
+        case 4: h = small_sort_row<16>(row); break;
+        case 5: h = small_sort_row<20>(row); break;
+        case 6: h = small_sort_row<24>(row); break;
+        case 7: h = small_sort_row<28>(row); break;
+        default: h = small_sort_row<32>(row); break;
+        }
+        const uint32_t valid = deg >= 32 ? kFull : (1u << deg) - 1u;
+        h &= valid;
+        const uint32_t cont = ~h & valid;
+        // heads of runs of at least W labels: such a run has W - 1 continuations behind its head
+        uint32_t m = h;
+        int W = 1;
+        for (;;) {
+            const uint32_t t = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
+            if (!t) break;
+            m = t;
+            ++W;
+        }
+        const int k = __popc(m);
         bool tied = false, chg = false;
-        if (active) {
-            const int64_t o0 = h.o0;
-            const int deg = h.deg;
-            const int32_t old = h.old;
-            if (!h.dirty) {
+        if (v >= 0) {
+            if (!hd.dirty) {
                 // no label around the vertex changed: its counts carry over
-                tied = deg > 0 && (p.sm_kw[v] & 0xFFFF) > 1;
-                if (!tied) p.lab_out[v] = old;
+                tied = hd.deg > 0 && (p.sm_kw[v] & 0xFFFF) > 1;
+                if (!tied) p.lab_out[v] = hd.old;
             } else if (deg == 0) {
                 p.dcnt[v] = 0;
-                p.lab_out[v] = old;
+                p.lab_out[v] = hd.old;
             } else {
-                const int32_t *nb = p.nbr + (o0 - p.nbr_shift);
-                // gather: all of the vertex's neighbour IDs, then all its labels, in flight
-                int ids[4];
-                int j = 0;
-                for (; j + 4 <= deg; j += 4) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) ids[u] = __ldg(&nb[j + u]);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) row[(j + u) ^ lane] = ld_label(&p.lab_in[ids[u]]);
-                }
-                for (; j < deg; ++j) row[j ^ lane] = ld_label(&p.lab_in[__ldg(&nb[j])]);
-                // insertion sort of the row
-                for (int a = 1; a < deg; ++a) {
-                    const int32_t x = row[a ^ lane];
-                    int b = a - 1;
-                    while (b >= 0 && row[b ^ lane] > x) {
-                        row[(b + 1) ^ lane] = row[b ^ lane];
-                        --b;
-                    }
-                    row[(b + 1) ^ lane] = x;
-                }
-                // runs
-                int d = 0, W = 0, k = 0, rmin = 0, rmax = 0;
-                int32_t cmin = 0, cmax = 0;
-                for (int a = 0; a < deg;) {
-                    const int32_t lab = row[a ^ lane];
-                    int e = a + 1;
-                    while (e < deg && row[e ^ lane] == lab) ++e;
-                    const int c = e - a;
-                    if (c > W) {
-                        W = c;
-                        k = 1;
-                        cmin = cmax = lab;
-                        rmin = rmax = d;
-                    } else if (c == W) {
-                        ++k;
-                        cmax = lab;
-                        rmax = d;
-                    }
-                    ++d;
-                    a = e;
-                }
-                if (k > 2) {  // resolving may need the runs: spill them in label order
-                    int32_t *rl = p.run_lab + (o0 - p.nbr_shift);
-                    uint16_t *rc = p.run_cnt + (o0 - p.nbr_shift);
-                    int r = 0;
-                    for (int a = 0; a < deg;) {
-                        const int32_t lab = row[a ^ lane];
-                        int e = a + 1;
-                        while (e < deg && row[e ^ lane] == lab) ++e;
-                        rl[r] = lab;
-                        rc[r] = (uint16_t)(e - a);
-                        ++r;
-                        a = e;
-                    }
-                }
-                p.dcnt[v] = d;
+                p.dcnt[v] = __popc(h);
                 p.sm_kw[v] = k | (W << 16);
                 if (k == 1) {
-                    p.lab_out[v] = cmin;
-                    count_change(changes, cmin, old);
-                    chg = cmin != old;
+                    const int32_t nl = row[__ffs(m) - 1];
+                    p.lab_out[v] = nl;
+                    count_change(changes, nl, hd.old);
+                    chg = nl != hd.old;
                 } else {
                     tied = true;
-                    p.sm_c0[v] = cmin;
-                    p.sm_c1[v] = cmax;
-                    p.sm_r[v] = rmin | (rmax << 16);
+                    const int lo = __ffs(m) - 1, hi = 31 - __clz(m);
+                    p.sm_c0[v] = k == 2 ? row[lo] : (int32_t)h;
+                    p.sm_c1[v] = k == 2 ? row[hi] : (int32_t)m;
+                    p.sm_r[v] = __popc(h & ((1u << lo) - 1u)) | (__popc(h & ((1u << hi) - 1u)) << 16);
+                }
+            }
+        }
+        if (__any_sync(kFull, k > 2)) {
+            if (deg > 0 && k <= 2) sdlt[w][rank] = LLONG_MIN;
+            __syncwarp();
+            for (int r = 0; r * 32 < total; ++r) {
+                const int s = r * 32 + lane;
+                const int own = owner(r);
+                if (s < total) {
+                    const int64_t e = sdlt[w][own];
+                    if (e != LLONG_MIN) p.run_lab[e + s] = rows[sat[w][own] + s];
                 }
             }
         }
         tb.append(tied, v, p.tied_small, &p.ctl->tied_small);
         warp_note_changes(p, chg, v);
+        __syncwarp();
     }
     tb.flush(p.tied_small, &p.ctl->tied_small);
     flush_changes(changes, p.ctl);
@@ -1502,6 +1665,28 @@ struct SpillRunQuery {
     __device__ int tile_pick(int64_t) const { return -1; }  // d <= 32 never spans a tile
 };
 
+// A small vertex with more than two candidates as count_small_sort_kernel leaves it: h has
+// the run heads among its sorted labels (at its CSR positions), m the heads of candidates.
+struct SmallMaskQuery {
+    uint32_t h, m;
+    // position of the head of rank x (0 <= x < popc(h))
+    __device__ int at(int x) const { return (int)__fns(h, 0, x + 1); }
+    __device__ int rank(int pos) const { return __popc(h & ((1u << pos) - 1u)); }
+    __device__ int first_ge(int64_t x) const
+    {
+        if (x >= __popc(h)) return -1;
+        const uint32_t c = x <= 0 ? m : m & ~((1u << at((int)x)) - 1u);
+        return c ? rank(__ffs(c) - 1) : -1;
+    }
+    __device__ int last_lt(int64_t y) const
+    {
+        if (y <= 0) return -1;
+        const uint32_t c = y >= __popc(h) ? m : m & ((1u << at((int)y)) - 1u);
+        return c ? rank(31 - __clz(c)) : -1;
+    }
+    __device__ int tile_pick(int64_t) const { return -1; }  // d <= 32 never spans a tile
+};
+
 __global__ void __launch_bounds__(kTB) resolve_small_kernel(PipeArgs p)
 {
     if (!ctl_active(p.ctl)) return;
@@ -1515,9 +1700,19 @@ __global__ void __launch_bounds__(kTB) resolve_small_kernel(PipeArgs p)
         const RunScope rs = run_scope(p, v);
         const long long a = rs.a, N = rs.N;
         const bool is_last = rs.is_last;
+        int32_t nl;
+        if (k > 2 && p.small_sort == 2) {
+            SmallMaskQuery mq{(uint32_t)p.sm_c0[v], (uint32_t)p.sm_c1[v]};
+            const int r = resolve_rank(a, d, N, is_last, mq);
+            nl = p.run_lab[__ldg(&p.off[v]) - p.nbr_shift + mq.at(r)];
+            const int32_t old = __ldg(&p.lab_in[v]);
+            p.lab_out[v] = nl;
+            count_change(changes, nl, old);
+            note_change(p, v, nl, old);
+            continue;
+        }
         SummaryQuery q(k, d, rmin, rmax);
         int r = resolve_rank(a, d, N, is_last, q);
-        int32_t nl;
         if (!q.fail && r == rmin) {
             nl = p.sm_c0[v];
         } else if (!q.fail && r == rmax) {

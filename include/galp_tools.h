@@ -61,7 +61,7 @@ typedef struct {
     float learned_margin;  /* learned rule: predicted log gain needed to leave the fixed rule's
                               choice (default 0.03) */
     int32_t small_sort;    /* vertices of at most 32 neighbours: 2 = one thread per vertex, labels sorted
-                              in shared memory (default); 1 = packs of vertices per warp, sort-based
+                              in registers (default); 1 = packs of vertices per warp, sort-based
                               counting; 0 = packs per warp, match-based counting */
     int32_t hub_part_shift; /* hubs (above 12288 neighbours) count their labels in degree * 2^shift / 8192
                                hash partitions (default 1); a partition that overflows makes the run
