@@ -253,8 +253,14 @@ bool build_schedule(Schedule &S, int64_t n, const int64_t *off, const std::vecto
             }
             for (auto &x : th) x.join();
         }
-        sc.nnarrow = (int32_t)(std::upper_bound(S.mid_deg.begin() + (ptrdiff_t)mb, S.mid_deg.end(), kNarrowMax) -
-                               (S.mid_deg.begin() + (ptrdiff_t)mb));
+        {
+            auto cut = [&](int t) {  // mid-list entries of degree <= t
+                return (int32_t)(std::upper_bound(S.mid_deg.begin() + (ptrdiff_t)mb, S.mid_deg.end(), t) -
+                                 (S.mid_deg.begin() + (ptrdiff_t)mb));
+            };
+            for (int i = 0; i < 7; ++i) sc.gcut[i] = cut(32 << i);
+            sc.n6144 = cut(kXlAMax);
+        }
         int64_t ooff = 0;
         for (int32_t v : big) {
             const int64_t deg = off[v + 1] - off[v];
@@ -626,8 +632,9 @@ IterArgs Engine::big_args(const Scope &sc) const
     return a;
 }
 
-// Variant table rows of the in-core scope: k = 8 * aggregated + 4 * (warp/CTA split at
-// 128) + 2 * (CTA split at 1024) + frontier.  Row 0 is the fixed heuristic's dense
+// Variant table rows of the in-core scope: k = 8 * aggregated + 2 * (CTA split at 1024) +
+// frontier; rows that differ by 4 alone are the same (they split the vertices between warps
+// and CTAs, which lane groups now count up to kGroupMax in every row).  Row 0 is the fixed heuristic's dense
 // iteration and row 1 its frontier iteration.
 void Engine::build_variant_table()
 {
@@ -641,9 +648,8 @@ void Engine::build_variant_table()
     for (int k = 0; k < kVar; ++k) {
         DispatchState &d = vtab[k];
         d.agg_mode = (k & 8) ? 1 : 2;
-        d.pos1 = cut((k & 4) ? 128 : kMidSMax);
-        d.pos2 = cut((k & 2) ? 1024 : kLargeMax);
-        d.pos_a = std::max(d.pos1, cut(kLargeAMax));
+        d.pos1 = d.pos_a = cut(kGroupMax);
+        d.pos2 = cut((k & 2) ? kGroupMax : kLargeMax);
         d.pos_b = std::max(d.pos2, cut(kXlAMax));
         d.frontier = k & 1;
         d.variant = k;
@@ -657,12 +663,9 @@ std::vector<DispatchState> Engine::static_dispatch() const
     for (size_t j = 0; j < sched.scopes.size(); ++j) {
         const Scope &sc = sched.scopes[j];
         ds[j].agg_mode = variant.agg_mode;
-        ds[j].pos1 = sc.nms;
-        ds[j].pos2 = sc.nms + sc.nml;
-        const int32_t *b = sched.mid_deg.data() + sc.m0;
-        const int cnt = sc.nms + sc.nml + sc.nmx;
-        ds[j].pos_a = (int32_t)(std::upper_bound(b, b + cnt, kLargeAMax) - b);
-        ds[j].pos_b = (int32_t)(std::upper_bound(b, b + cnt, kXlAMax) - b);
+        ds[j].pos1 = ds[j].pos_a = sc.gcut[5];
+        ds[j].pos2 = sc.gcut[6];
+        ds[j].pos_b = sc.n6144;
     }
     return ds;
 }
@@ -706,29 +709,24 @@ PipeArgs Engine::pipe_args(const Scope &sc) const
     q.v1 = sc.v1;
     q.bsum = (int64_t *)b_bsum.p;
     q.last_v = sc.last_v;
-    q.narrow_cut = variant.cta_narrow ? sc.nnarrow : -1;
+    for (int i = 0; i < 6; ++i) q.gcut[i] = sc.gcut[i];
+    q.gstart = variant.mid_sort ? sc.gcut[3] : 0;
     return q;
 }
 
 // One update of one scope: reads lab_in (all vertices), writes lab_out for the scope.
 int Engine::launch_limits()
 {
-    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_mid, count_mid64_kernel, 32 * kMidWarps, 0));
+    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_group, count_group_kernel, kGroupThreads, 0));
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_mid_sort, count_mid_sort_kernel, 32 * kMidWarps, 0));
     occ_mid_sort = std::max(occ_mid_sort, 1);
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resolve, resolve_small_kernel, kTB, 0));
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resolve_mid, resolve_mid_kernel, kTB, 0));
     // the CTA kernels loop over their vertex range: a grid of exactly the resident blocks
-    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cta64, count_cta_kernel<64, 2 * kNarrowMax>, 64,
-                                                            sizeof(unsigned long long) * 2 * kNarrowMax));
-    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cta128, count_cta_kernel<128, 2 * kLargeAMax>, 128,
-                                                            sizeof(unsigned long long) * 2 * kLargeAMax));
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cta256, count_cta_kernel<kTB, 2 * kLargeMax>, kTB,
                                                             sizeof(unsigned long long) * 2 * kLargeMax));
-    occ_cta64 = std::max(occ_cta64, 1);
-    occ_cta128 = std::max(occ_cta128, 1);
     occ_cta256 = std::max(occ_cta256, 1);
-    occ_mid = std::max(occ_mid, 1);
+    occ_group = std::max(occ_group, 1);
     occ_resolve = std::max(occ_resolve, 1);
     occ_resolve_mid = std::max(occ_resolve_mid, 1);
     return GALP_OK;
@@ -737,7 +735,7 @@ int Engine::launch_limits()
 int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, const int32_t *lab_in,
                           int32_t *lab_out, const uint8_t *dirty, int32_t *changed)
 {
-    if (!occ_mid) {
+    if (!occ_group) {
         int rc = launch_limits();
         if (rc) return rc;
     }
@@ -796,47 +794,44 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     }
     if (q.nmid_s + q.nmid_l + q.nmid_x) {
         // ranges of the degree-sorted mid list come from the dispatch state
-        const int gmid = (int)std::min<int64_t>((sc.nms + kMidWarps - 1) / kMidWarps + 1,
-                                                (int64_t)sms * std::min(mid_bps, variant.mid_sort ? occ_mid_sort : occ_mid));
-        if (variant.mid_sort) {  // sort + reduce counting of the warp range
+        const int nmid = sc.nms + sc.nml + sc.nmx;
+        if (variant.mid_sort && sc.nms) {  // bitonic sort per warp, up to 256 neighbours
+            const int gmid = (int)std::min<int64_t>((sc.nms + kMidWarps - 1) / kMidWarps, (int64_t)sms * occ_mid_sort);
             count_mid_sort_kernel<<<gmid, 32 * kMidWarps, 0, st>>>(q);
             launched("count_mid_sort_kernel", st);
-        } else {
-            count_mid64_kernel<<<gmid, 32 * kMidWarps, 0, st>>>(q);
-            launched("count_mid64_kernel", st);
         }
-        const int g128 = (int)std::max<int64_t>(1, std::min<int64_t>(sc.nms + sc.nml, (int64_t)sms * occ_cta128));
-        const int g256 = (int)std::max<int64_t>(1, std::min<int64_t>(sc.nml, (int64_t)sms * occ_cta256));
-        if (q.narrow_cut > 0) {  // the lower part of the 128-thread range, in 64-thread CTAs
-            const int g64 = (int)std::min<int64_t>(q.narrow_cut, (int64_t)sms * occ_cta64);
-            count_cta_kernel<64, 2 * kNarrowMax><<<g64, 64, sizeof(unsigned long long) * 2 * kNarrowMax, st>>>(q, 4);
-            launched("count_cta_kernel<64>", st);
+        if (sc.gcut[5] > q.gstart) {
+            constexpr int gw = kGroupThreads / 32;
+            int64_t tiles = 0;
+            for (int g = 1; g <= 5; ++g)
+                tiles += (std::max(sc.gcut[g] - std::max(sc.gcut[g - 1], q.gstart), 0) + (32 >> g) - 1) / (32 >> g);
+            const int blocks = (int)std::min<int64_t>((tiles + gw - 1) / gw, (int64_t)sms * std::min(mid_bps, occ_group));
+            count_group_kernel<<<blocks, kGroupThreads, 0, st>>>(q);
+            launched("count_group_kernel", st);
         }
-        if (variant.cta_stage) {  // neighbour IDs staged by bulk copies (the stage follows the table)
-            count_cta_kernel<128, 2 * kLargeAMax, true>
-                <<<g128, 128, sizeof(unsigned long long) * 2 * kLargeAMax + sizeof(int32_t) * (kLargeAMax + 8), st>>>(
-                    q, 0);
-            launched("count_cta_kernel<128>", st);
-            count_cta_kernel<kTB, 2 * kLargeMax, true>
-                <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax + sizeof(int32_t) * (kLargeMax + 8), st>>>(
-                    q, 1);
-            launched("count_cta_kernel<256>", st);
-        } else {
-            count_cta_kernel<128, 2 * kLargeAMax><<<g128, 128, sizeof(unsigned long long) * 2 * kLargeAMax, st>>>(q, 0);
-            launched("count_cta_kernel<128>", st);
-            count_cta_kernel<kTB, 2 * kLargeMax><<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax, st>>>(q, 1);
+        if (sc.gcut[6] > sc.gcut[5]) {
+            const int g256 = (int)std::min<int64_t>(sc.gcut[6] - sc.gcut[5], (int64_t)sms * occ_cta256);
+            if (variant.cta_stage)  // neighbour IDs staged by bulk copies (the stage follows the table)
+                count_cta_kernel<kTB, 2 * kLargeMax, true>
+                    <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax + sizeof(int32_t) * (kLargeMax + 8),
+                       st>>>(q, 1);
+            else
+                count_cta_kernel<kTB, 2 * kLargeMax>
+                    <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax, st>>>(q, 1);
             launched("count_cta_kernel<256>", st);
         }
-        if (q.nmid_x + q.nmid_l) {
-            count_cta_kernel<512, 2 * kXlAMax>
-                <<<(int)std::max<int64_t>(1, std::min<int64_t>(q.nmid_x + q.nmid_l, (int64_t)sms * 2)), 512,
-                   sizeof(unsigned long long) * 2 * kXlAMax, st>>>(q, 2);
+        // rows with a CTA split at 1024 (forced or learned) send 1025..2048 here
+        const bool rows = policy == 0 && disp_mode != 0;
+        const int nxla = sc.n6144 - sc.gcut[rows ? 5 : 6];
+        if (nxla > 0) {
+            count_cta_kernel<512, 2 * kXlAMax><<<(int)std::min<int64_t>(nxla, (int64_t)sms * 2), 512,
+                                                 sizeof(unsigned long long) * 2 * kXlAMax, st>>>(q, 2);
             launched("count_cta_kernel<512>", st);
         }
-        if (q.nmid_x) {
+        if (nmid > sc.n6144) {
             count_cta_kernel<kXlThreads, kXlSlots>
-                <<<(int)std::min<int64_t>(q.nmid_x, (int64_t)sms), kXlThreads, sizeof(unsigned long long) * kXlSlots,
-                   st>>>(q, 3);
+                <<<(int)std::min<int64_t>(nmid - sc.n6144, (int64_t)sms), kXlThreads,
+                   sizeof(unsigned long long) * kXlSlots, st>>>(q, 3);
             launched("count_cta_kernel<1024>", st);
         }
     }
@@ -1349,7 +1344,7 @@ int galp_schedule_info(galp_ctx *ctx, galp_sched_info *info)
     info->nlarge = nml;
     info->nbig = (int64_t)E.sched.big_v.size();
     info->table_slots = E.sched.max_pair_slots;
-    info->launches_per_iter = 14 + (info->nbig ? 7 : 0) + (E.frontier ? 1 : 0) + (E.variant.cta_narrow ? 1 : 0);
+    info->launches_per_iter = 14 + (info->nbig ? 7 : 0) + (E.frontier ? 1 : 0);
     info->flags = (E.adj_sorted ? GALP_SCHED_SORTED : 0) | (E.symmetric ? GALP_SCHED_SYMMETRIC : 0) |
                   (E.frontier ? GALP_SCHED_FRONTIER : 0);
     info->launches = E.launches;
@@ -1426,8 +1421,8 @@ int galp_dispatch_table(galp_ctx *ctx, galp_dispatch_row *rows, int32_t cap, int
     for (int32_t k = 0; k < cap && k < *count; ++k) {
         rows[k].agg_mode = E.vtab[k].agg_mode;
         rows[k].frontier = E.vtab[k].frontier;
-        rows[k].warp_max_degree = (k & 4) ? 128 : galp::kMidSMax;
-        rows[k].cta256_max_degree = (k & 2) ? 1024 : galp::kLargeMax;
+        rows[k].warp_max_degree = galp::kGroupMax;
+        rows[k].cta256_max_degree = (k & 2) ? galp::kGroupMax : galp::kLargeMax;
         rows[k].pos1 = E.vtab[k].pos1;
         rows[k].pos2 = E.vtab[k].pos2;
     }

@@ -54,7 +54,8 @@ struct Scope {
     int32_t c0 = 0, nc = 0;    // big insert chunks
     int32_t s0 = 0, ns = 0;    // big stats chunks
     int32_t sv0 = 0, nsv = 0;  // vertices of degree <= 32 (small_v), in vertex order
-    int32_t nnarrow = 0;       // mid-list entries of at most kNarrowMax neighbours
+    int32_t gcut[7] = {};      // mid-list entries of at most 32 << i neighbours
+    int32_t n6144 = 0;         // mid-list entries of at most kXlAMax neighbours
     int32_t last_v = -1;       // last vertex of the scope that owns runs
     int32_t q0 = 0, nq = 0;    // hash partitions of the scope's big vertices
     int64_t pair_slots = 0;    // pair area of those partitions
@@ -238,12 +239,12 @@ struct Engine {
     DevBuf b_g_v0, b_g_base, b_g_last, b_g_active, b_g_iters, b_g_counts, b_gid;
     int64_t max_label = 0;    // labels stay below this (n, or the largest graph of a batch)
     // launch shapes (blocks per SM), chosen by galp_batch_tune
-    int small_bps = 16, mid_bps = 6, resolve_bps = 4;
+    int small_bps = 16, mid_bps = 8, resolve_bps = 4;
     // resident blocks per SM of the mid-vertex counting and the resolve kernels (occupancy
     // API): their grid-stride loops run as one full wave, since a partial second wave
     // would start its blocks' whole shares late
-    int occ_mid = 0, occ_mid_sort = 0, occ_resolve = 0, occ_resolve_mid = 0;
-    int occ_cta64 = 0, occ_cta128 = 0, occ_cta256 = 0;  // resident CTA-kernel blocks per SM
+    int occ_group = 0, occ_mid_sort = 0, occ_resolve = 0, occ_resolve_mid = 0;
+    int occ_cta256 = 0;
     int launch_limits();
     // hub partitions at 2^shift times the default count: plan, upload, size the pair area
     int setup_hub_parts(int shift, cudaStream_t st, int64_t &h2d);

@@ -1,12 +1,12 @@
 // lp_dispatch.cuh -- per-iteration kernel-variant dispatch (MLP inference on the device).
 //
 // Every iteration of the in-core update reads a DispatchState from device memory: how
-// mid-list vertices are split between the warp kernel and the two CTA kernels (degree
+// mid-list vertices are split between the lane-group kernel and the CTA kernels (degree
 // thresholds, as positions in the degree-sorted mid list), whether CTA-table inserts are
 // warp-aggregated, and whether the frontier is used.  Every variant computes the same
 // labels; they differ only in speed.  dispatch_kernel fills the state on the device
 // before each iteration, so no host round trip is needed:
-//   * fixed rule: CTA thresholds 256 / 2048, plain inserts, frontier when at most
+//   * fixed rule: CTA thresholds 1024 / 2048, inserts by fixed_agg, frontier when at most
 //     frontier_frac of the labels changed in the previous iteration;
 //   * learned: a 3-layer MLP (kFeat -> kHid -> kHid -> kVar, ReLU, FP32) predicts the
 //     log slowdown of every variant from the iteration's features; the argmin wins when
@@ -33,9 +33,9 @@ constexpr int kMaxLogIters = 64;
 struct DispatchState {
     int32_t agg_mode;  // CTA-table inserts: 0 auto, 1 warp-aggregated, 2 plain
     int32_t frontier;  // 1 = skip clean vertices this iteration (frontier mode only)
-    // cuts of the degree-sorted mid list: [0, pos1) one warp each; [pos1, pos_a) 128-thread
-    // CTAs (degree <= 1024); [pos_a, pos2) 256-thread CTAs; [pos2, pos_b) 512-thread CTAs
-    // (degree <= 6144); [pos_b, end) 1024-thread CTAs
+    // cuts of the degree-sorted mid list: [0, pos1) groups of lanes; [pos_a, pos2) 256-thread
+    // CTAs (pos_a = pos1); [pos2, pos_b) 512-thread CTAs (degree <= 6144); [pos_b, end)
+    // 1024-thread CTAs
     int32_t pos1, pos2, pos_a, pos_b;
     int32_t variant;   // row of the variant table
     int32_t pad;

@@ -4,11 +4,11 @@
 // One iteration over a scope (whole graph, one out-of-core batch):
 //
 //   count   vertices are degree-bucketed and counted with no dependence between blocks:
-//             small (degree <= 32, and degree 0): one warp per pack of <= 32 label
-//               slots, counting in registers (__match_any_sync on (vertex, label));
-//             mid (33..256): one warp per vertex, shared-memory hash region;
-//             large (257..2048): one CTA per vertex, shared-memory hash region;
-//             big (> 2048): global tables (big_insert/big_stats, lp_kernels.cuh).
+//             small (degree <= 32, and degree 0): one lane per vertex, labels sorted in
+//               registers (or one warp per pack of <= 32 label slots);
+//             33..1024: a group of lanes per vertex, labels sorted in registers;
+//             1025..12288: one CTA per vertex, shared-memory hash table;
+//             big (> 12288): hash partitions (big_insert, hub_count, lp_kernels.cuh).
 //           Each vertex gets its distinct-label count d; a vertex with a unique
 //           most-frequent label is final and written at once.  A tied vertex leaves a
 //           summary (smallest/largest candidate, their ranks, #candidates, max count)
@@ -21,9 +21,10 @@
 //           (resolve_rank, lp_resolve.h) from its summary, or from its spilled runs.
 //
 // Spill layout (indexed by CSR position relative to the scope's first entry):
-//   run_lab[e0 + r] label, run_cnt[e0 + r] count of the vertex's r-th run; small
-//   vertices write their runs sorted by label, mid/large vertices their table's
-//   occupied entries unsorted (queried by order statistics).
+//   run_lab[e0 + r] label, run_cnt[e0 + r] count of the vertex's r-th run; small vertices
+//   write their sorted labels (or, counted in packs, their runs in label order), vertices
+//   sorted by lane groups their runs in label order (kSpillSorted), CTA-table vertices
+//   their table's occupied entries unsorted (queried by order statistics).
 #pragma once
 
 #include <utility>
@@ -34,18 +35,14 @@
 
 namespace galp {
 
-constexpr int kMidSMax = 256;        // mid bucket: 33..256 neighbours, one warp each
-constexpr int kMidSCap = 2 * kMidSMax;
-constexpr int kMidWarps = 8;         // warps (vertices) per mid CTA
+constexpr int kMidSMax = 256;        // mid bucket: 33..256 neighbours
+constexpr int kMidWarps = 8;         // warps (vertices) per CTA of count_mid_sort_kernel
 constexpr int kScanBlock = 4096;     // vertices per scan block (256 threads x 16)
-constexpr int kLargeMax = 2048;      // large bucket: 257..2048, one 256-thread CTA each
+constexpr int kLargeMax = 2048;      // large bucket: 257..2048; above 1024 one 256-thread CTA each
 constexpr int kXlMax = 12288;        // xl bucket: 2049..12288, one CTA each (512 or 1024 threads)
 constexpr int kXlSlots = 2 * kXlMax; // 192 KB of shared-memory table (64-bit slots)
 constexpr int kXlThreads = 1024;
-constexpr int kLargeAMax = 1024;     // large vertices up to here: 128-thread CTAs, 16 KB tables
 constexpr int kXlAMax = 6144;        // xl vertices up to here: 512-thread CTAs, 96 KB tables
-constexpr int kNarrowMax = 512;      // narrow CTA variant: large vertices up to here, 64 threads,
-                                     // 8 KB tables
 
 struct PipeArgs {
     const int32_t *nbr;     // neighbour buffer holding CSR entries [nbr_shift, ...)
@@ -66,7 +63,7 @@ struct PipeArgs {
     int32_t *dcnt;          // distinct labels
     int64_t *runbase;       // run base relative to the scope
     int32_t *sm_c0, *sm_c1; // smallest / largest candidate label
-    int32_t *sm_kw;         // candidates | max count << 16
+    int32_t *sm_kw;         // candidates | max count << 16 (| kSpillSorted)
     int32_t *sm_r;          // rank of smallest | rank of largest << 16
     // spill, indexed by CSR position - nbr_shift
     int32_t *run_lab;
@@ -92,9 +89,8 @@ struct PipeArgs {
     int32_t lab27;          // every label below 2^27 - 1 (32-bit sort keys in packs)
     int32_t small_sort;     // small vertices: 0 match-based packs, 1 sort-based packs (needs lab27),
                             // 2 one thread per vertex, sorted in registers
-    int32_t narrow_cut;     // -1, or the mid-list position of the first vertex above kNarrowMax
-                            // neighbours: the 128-thread CTA range is split there, its lower
-                            // part going to 64-thread CTAs
+    int32_t gcut[6];        // mid-list positions of the first vertex above 32 << i neighbours
+    int32_t gstart;         // first mid-list position counted by lane groups (mid_sort: above 256)
 };
 
 // Graph of vertex v in batched mode: the largest g with g_v0[g] <= v.
@@ -552,11 +548,12 @@ __device__ __forceinline__ void t64_insert_row(unsigned long long *tab, uint32_t
 
 // Finish a counted vertex: per-vertex state, and its label unless it is tied.  One
 // thread; returns whether the vertex is tied (the caller appends it to the tied list).
+constexpr int kSpillSorted = 1 << 30;  // in sm_kw: the vertex's spilled runs are in label order
 __device__ __forceinline__ bool finish_counted(const PipeArgs &p, int v, const Sum5 &s, int rmin, int rmax,
-                                               unsigned long long &changes, int32_t old)
+                                               unsigned long long &changes, int32_t old, int flags = 0)
 {
     p.dcnt[v] = s.d;
-    p.sm_kw[v] = s.k | (s.W << 16);
+    p.sm_kw[v] = s.k | (s.W << 16) | flags;
     if (s.k == 1) {
         p.lab_out[v] = s.mn;
         count_change(changes, s.mn, old);
@@ -655,10 +652,6 @@ struct SortNet {
     }
 };
 
-// Row of a small vertex in its warp's shared memory: 36 words, so that the 16-byte accesses
-// of 8 lanes to their own rows fall in distinct banks.
-constexpr int kSmallRow = 36;
-
 // Sort the first N words of a lane's row in registers, write them back and return the mask
 // of positions that differ from the one before (position 0 always set).
 template <int N>
@@ -709,6 +702,84 @@ __global__ void __launch_bounds__(kSmallWindow) small_window_kernel(int32_t *sma
     }
 }
 
+// Row of a small vertex in its warp's shared memory: 36 words, so that the 16-byte accesses
+// of 8 lanes to their own rows fall in distinct banks.
+constexpr int kSmallRow = 36;
+
+// ----- a warp's tile of sorted rows -----
+//
+// One tile: the labels of up to 32 vertices (1024 CSR entries), gathered together into the
+// warp's shared memory.  The entries of the tile's vertices follow one another in slots; a
+// warp copies 32 slots at a time, whatever vertices they belong to, and the owner of a slot
+// follows from the mask of vertex starts in its row of slots.
+struct TileBuf {
+    int32_t rows[32 * kSmallRow];  // per lane: its labels, padded with INT_MAX
+    int64_t dlt[32];        // i-th vertex to count: CSR position minus slot
+    int32_t at[32];         // its row's first word minus its first slot
+    uint2 info[32];         // row of slots: mask of vertex starts, starts in earlier rows
+    // index of the vertex that owns the lane's slot in a row (lanes past the tile's total: any)
+    __device__ __forceinline__ int owner(int row) const
+    {
+        const uint2 q = info[row];
+        return (int)q.y + __popc(q.x & ((2u << (threadIdx.x & 31)) - 1u)) - 1;
+    }
+};
+
+// Gather a tile of one vertex per lane: the lane's `deg` labels, whose first entry is at e0
+// of the neighbour buffer, go to its row, padded to n words (a multiple of 4).
+__device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int deg, int64_t e0, int n)
+{
+    const int lane = threadIdx.x & 31;
+    int pos = deg;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, pos, o);
+        if (lane >= o) pos += y;
+    }
+    const int total = __shfl_sync(kFull, pos, 31);
+    pos -= deg;
+    B.info[lane] = make_uint2(0u, 0u);
+    const unsigned nz = __ballot_sync(kFull, deg > 0);
+    const int rank = __popc(nz & ((1u << lane) - 1u));
+    __syncwarp();
+    if (deg > 0) {
+        B.dlt[rank] = e0 - pos;
+        B.at[rank] = lane * kSmallRow - pos;
+        atomicOr(&B.info[pos >> 5].x, 1u << (pos & 31));
+    }
+    for (int j = 0; j < n; j += 4)
+        *reinterpret_cast<int4 *>(B.rows + lane * kSmallRow + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+    __syncwarp();
+    const int starts = __popc(B.info[lane].x);
+    int before = starts;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, before, o);
+        if (lane >= o) before += y;
+    }
+    B.info[lane].y = (uint32_t)(before - starts);
+    __syncwarp();
+    constexpr int PER = 8;  // rows in flight
+    for (int r0 = 0; r0 * 32 < total; r0 += PER) {
+        int id[PER], at[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            id[u] = -1;
+            if ((r0 + u) * 32 >= total) continue;  // warp-uniform
+            const int s = (r0 + u) * 32 + lane;
+            const int own = B.owner(r0 + u);
+            if (s < total) {
+                id[u] = ld_nbr(&p.nbr[B.dlt[own] + s]);
+                at[u] = B.at[own] + s;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+            if (id[u] >= 0) B.rows[at[u]] = ld_label(&p.lab_in[id[u]]);
+    }
+    __syncwarp();
+}
+
 // Small vertices (at most 32 neighbours; `small_sort` 2): a warp takes 32 vertices of about
 // equal degree (small_window_kernel), gathers their labels together and sorts each vertex's
 // labels in one lane's registers.
@@ -735,15 +806,11 @@ constexpr int kSmallBlocks = 8;  // resident blocks per SM
 __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_kernel(PipeArgs p)
 {
     constexpr int NW = kSmallThreads / 32;
-    __shared__ __align__(16) int32_t srow[NW][32 * kSmallRow];
-    __shared__ int64_t sdlt[NW][32];   // CSR position minus slot, of the i-th vertex with neighbours
-    __shared__ int32_t sat[NW][32];    // its row minus its first slot
-    __shared__ uint32_t smask[NW][32]; // vertex starts in each row of slots
+    __shared__ __align__(16) TileBuf stile[NW];
     __shared__ int32_t tbuf[NW][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int32_t *rows = srow[w];
     WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
     // the next round's vertex, offsets, label and dirty flag load one round ahead
@@ -767,69 +834,23 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
     // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
     // window in turn, so that none has only the window's highest degrees
     const int stride = gridDim.x * kSmallThreads;
+    int base = blockIdx.x * kSmallThreads;  // block-uniform
     int turn = w;
-    Head nxt = head(blockIdx.x * kSmallThreads + turn * 32 + lane);
-    for (int base = blockIdx.x * kSmallThreads; base < p.nsmall; base += stride) {
-        const Head hd = nxt;
+    auto ahead = [&](int from) {
+        const Head hd = head(from + turn * 32 + lane);
         turn = (turn + 1) & (NW - 1);
-        nxt = head(base + stride + turn * 32 + lane);
+        return hd;
+    };
+    TileBuf &B = stile[w];
+    Head nxt = ahead(base);
+    for (; base < p.nsmall; base += stride) {
+        const Head hd = nxt;
+        nxt = ahead(base + stride);
         const int v = hd.v;
         const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-        // slots: lane's entries at [pos, pos + deg) of the warp's total
-        int pos = deg;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, pos, o);
-            if (lane >= o) pos += y;
-        }
-        const int total = __shfl_sync(kFull, pos, 31);
-        pos -= deg;
-        smask[w][lane] = 0u;
-        const unsigned nz = __ballot_sync(kFull, deg > 0);
-        const int rank = __popc(nz & ((1u << lane) - 1u));
         const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
-        __syncwarp();
-        if (deg > 0) {
-            sdlt[w][rank] = hd.o0 - p.nbr_shift - pos;
-            sat[w][rank] = lane * kSmallRow - pos;
-            atomicOr(&smask[w][pos >> 5], 1u << (pos & 31));
-        }
-        for (int j = 0; j < n4; ++j)
-            *reinterpret_cast<int4 *>(rows + lane * kSmallRow + 4 * j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
-        __syncwarp();
-        const uint32_t rmask = smask[w][lane];  // lane r: starts in row r ...
-        int rbefore = __popc(rmask);            // ... and in the rows before it
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, rbefore, o);
-            if (lane >= o) rbefore += y;
-        }
-        rbefore -= __popc(rmask);
-        // index of the vertex that owns slot s = row * 32 + lane (warp-collective)
-        auto owner = [&](int row) {
-            const uint32_t starts = __shfl_sync(kFull, rmask, row);
-            return __shfl_sync(kFull, rbefore, row) + __popc(starts & ((2u << lane) - 1u)) - 1;
-        };
-        constexpr int PER = 8;
-        for (int r0 = 0; r0 * 32 < total; r0 += PER) {
-            int id[PER], at[PER];
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                id[u] = -1;
-                if ((r0 + u) * 32 >= total) continue;  // warp-uniform
-                const int s = (r0 + u) * 32 + lane;
-                const int own = owner(r0 + u);
-                if (s < total) {
-                    id[u] = ld_nbr(&p.nbr[sdlt[w][own] + s]);
-                    at[u] = sat[w][own] + s;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < PER; ++u)
-                if (id[u] >= 0) rows[at[u]] = ld_label(&p.lab_in[id[u]]);
-        }
-        __syncwarp();
-        int32_t *row = rows + lane * kSmallRow;
+        tile_gather(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
+        int32_t *row = B.rows + lane * kSmallRow;
         uint32_t h = 0u;
         switch (n4) {  // warp-uniform
         case 0: break;
@@ -882,14 +903,16 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
             }
         }
         if (__any_sync(kFull, k > 2)) {
-            if (deg > 0 && k <= 2) sdlt[w][rank] = LLONG_MIN;
+            const int total = __reduce_add_sync(kFull, deg);
+            const unsigned nz = __ballot_sync(kFull, deg > 0);
+            if (deg > 0 && k <= 2) B.dlt[__popc(nz & ((1u << lane) - 1u))] = LLONG_MIN;
             __syncwarp();
             for (int r = 0; r * 32 < total; ++r) {
                 const int s = r * 32 + lane;
-                const int own = owner(r);
+                const int own = B.owner(r);
                 if (s < total) {
-                    const int64_t e = sdlt[w][own];
-                    if (e != LLONG_MIN) p.run_lab[e + s] = rows[sat[w][own] + s];
+                    const int64_t e = B.dlt[own];
+                    if (e != LLONG_MIN) p.run_lab[e + s] = B.rows[B.at[own] + s];
                 }
             }
         }
@@ -927,98 +950,314 @@ __device__ __forceinline__ CtaHead cta_head(const PipeArgs &p, int first, int i,
     return h;
 }
 
-// One warp per mid vertex (33..256 neighbours): a 512-slot table of generation-tagged
-// 64-bit slots per warp (as the CTA tables: never cleared between vertices), probed over
-// up to 4 slots per neighbour.  Against 32-bit key and count arrays cleared per vertex:
-// no clear pass and one shared-memory atomic per insert.  The next vertex's head and its
-// neighbour IDs load while the current one is counted (as in the CTA kernels).
-__global__ void __launch_bounds__(32 * kMidWarps) count_mid64_kernel(PipeArgs p)
+// ----- vertices of 33..1024 neighbours sorted by groups of lanes -----
+
+// Sort x[OFF .. OFF + CNT), a bitonic sequence, within a lane: half-cleaners while the length
+// is even (they hold for any even length), a sorting network for an odd rest.
+template <int OFF, int CNT, int N, int... C>
+__device__ __forceinline__ void bitonic_rest(int32_t (&x)[N], std::integer_sequence<int, C...>)
 {
-    __shared__ unsigned long long stab[kMidWarps][kMidSCap];
-    __shared__ int32_t tbuf[kMidWarps][kWarpBuf];
+    ((void)[&] {
+        constexpr NetPair q = SortNet<CNT>::get(C);
+        const int32_t lo = min(x[OFF + q.a], x[OFF + q.b]), hi = max(x[OFF + q.a], x[OFF + q.b]);
+        x[OFF + q.a] = lo;
+        x[OFF + q.b] = hi;
+    }(), ...);
+}
+
+template <int OFF, int CNT, int N>
+__device__ __forceinline__ void bitonic_lane(int32_t (&x)[N])
+{
+    if constexpr (CNT > 1 && CNT % 2 == 0) {
+#pragma unroll
+        for (int j = 0; j < CNT / 2; ++j) {
+            const int32_t lo = min(x[OFF + j], x[OFF + j + CNT / 2]), hi = max(x[OFF + j], x[OFF + j + CNT / 2]);
+            x[OFF + j] = lo;
+            x[OFF + j + CNT / 2] = hi;
+        }
+        bitonic_lane<OFF, CNT / 2>(x);
+        bitonic_lane<OFF + CNT / 2, CNT / 2>(x);
+    } else if constexpr (CNT > 1) {
+        bitonic_rest<OFF, CNT>(x, std::make_integer_sequence<int, SortNet<CNT>::size>{});
+    }
+}
+
+// A lane's number of labels N, the words from its row to the next lane's (16-byte accesses of
+// 8 lanes to their own rows fall in distinct banks) and j / N as j * rcp >> 16 (j < 32 N).
+struct GroupShape {
+    int N, stride, rcp;
+};
+__host__ __device__ constexpr GroupShape group_shape(int N)
+{
+    return N == 20   ? GroupShape{20, 20, 3277}
+           : N == 24 ? GroupShape{24, 28, 2731}
+                     : GroupShape{32, 36, 2048};
+}
+
+// Sort the N words of every lane's row over groups of 2^g consecutive lanes (lane-major
+// order), write the rows back and return the lane's mask of positions that differ from
+// the one before (the group's first position always set).  Each lane sorts its row, then
+// level L merges pairs of sorted runs of 2^(L-1) lanes: a flip against the mirrored lane,
+// half-cleaners between lanes, and the bitonic rest within the lane.
+template <int N>
+__device__ __forceinline__ uint32_t group_sort_rows(int32_t *rows, int g)
+{
+    const int lane = threadIdx.x & 31;
+    int32_t *row = rows + lane * group_shape(N).stride;
+    int32_t x[N];
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+        const int4 q = *reinterpret_cast<const int4 *>(row + j);
+        x[j] = q.x;
+        x[j + 1] = q.y;
+        x[j + 2] = q.z;
+        x[j + 3] = q.w;
+    }
+    SortNet<N>::sort(x);
+#pragma unroll 1
+    for (int L = 1; L <= g; ++L) {
+        const int flip = (1 << L) - 1;
+        bool low = !(lane & (1 << (L - 1)));
+#pragma unroll
+        for (int j = 0; j < N / 2; ++j) {
+            const int32_t a = __shfl_xor_sync(kFull, x[N - 1 - j], flip), b = __shfl_xor_sync(kFull, x[j], flip);
+            x[j] = low ? min(x[j], a) : max(x[j], a);
+            x[N - 1 - j] = low ? min(x[N - 1 - j], b) : max(x[N - 1 - j], b);
+        }
+#pragma unroll 1
+        for (int D = 1 << (L - 1) >> 1; D >= 1; D >>= 1) {
+            low = !(lane & D);
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int32_t a = __shfl_xor_sync(kFull, x[j], D);
+                x[j] = low ? min(x[j], a) : max(x[j], a);
+            }
+        }
+        bitonic_lane<0, N>(x);
+    }
+    const int32_t before = __shfl_up_sync(kFull, x[N - 1], 1);
+    uint32_t h = (lane & ((1 << g) - 1)) == 0 || x[0] != before ? 1u : 0u;
+#pragma unroll
+    for (int j = 1; j < N; ++j)
+        if (x[j] != x[j - 1]) h |= 1u << j;
+#pragma unroll
+    for (int j = 0; j < N; j += 4) *reinterpret_cast<int4 *>(row + j) = make_int4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+    return h;
+}
+
+// Move the run heads (mask h) of every lane's row to the front of its group's rows, in order
+// (the lane's first head has rank `at` in the group), candidates (mask m) with the sign bit set.
+template <int N>
+__device__ __forceinline__ void group_compact(int32_t *rows, int g, uint32_t h, uint32_t m, int at)
+{
+    constexpr int stride = group_shape(N).stride;
+    const int lane = threadIdx.x & 31;
+    int32_t x[N];
+#pragma unroll
+    for (int j = 0; j < N; j += 4) {
+        const int4 q = *reinterpret_cast<const int4 *>(rows + lane * stride + j);
+        x[j] = q.x;
+        x[j + 1] = q.y;
+        x[j + 2] = q.z;
+        x[j + 3] = q.w;
+    }
+    __syncwarp();
+    int32_t *out = rows + (lane >> g << g) * stride + at;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+        if ((h >> j) & 1u) *out++ = x[j] | (int32_t)(((m >> j) & 1u) << 31);
+    __syncwarp();
+}
+
+// One warp per tile of 32 / G vertices of the degree-sorted mid list, G = 2^g lanes each,
+// where 16 G < degree <= 32 G: g = 1 (33..64 neighbours) to 5 (513..1024).  The labels are
+// gathered in rows of 32, spread over the group's lanes, N = 20, 24 or 32 labels each (the
+// smallest that holds the tile's largest degree), and sorted across the group; run lengths
+// come from the lanes' head masks, with the part of a run that goes on into later lanes
+// added to its head's lane.  Vertices with more than two candidates spill their runs in
+// label order, with the maximum count for candidates and 0 for others.
+//
+// About 4.5 warp instructions per entry in tie-heavy iterations, none of them divergent or
+// behind a barrier, where tables in shared memory (one warp, 64 or 128 threads per vertex)
+// took 8 to 10 at 13 to 22 active lanes; half of them are the networks' minima and maxima,
+// which run at half rate.  Ten iterations of R-MAT 24: 20.0 -> 16.6 ms here and, the spilled
+// runs being in order, 2.6 -> 0.85 ms in resolve_mid; R-MAT 26 with edge factor 4: 28.9 ->
+// 23.2 and 6.0 -> 1.8.  Longer lists stay with the tables: a warp sorting 2048 labels, 64 to
+// a lane, gained 16 % where there are tens of thousands of such vertices and lost 80 % where
+// there are a few (one warp then takes 27 us for one).  Labels brought in by asynchronous
+// copies, the next tile's during the sort, were slower (4-byte copies run at half the rate
+// of loads: 17.1 ms here, and 33 instead of 25 for the small vertices above).
+constexpr int kGroupMax = 1024;
+constexpr int kGroupThreads = 128;
+constexpr int kGroupBlocks = 5;  // resident blocks per SM: 6, 4 and 8 were 1 to 9 % slower
+__global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) count_group_kernel(PipeArgs p)
+{
+    constexpr int NW = kGroupThreads / 32;
+    __shared__ __align__(16) int32_t srow[NW][32 * 36];
+    __shared__ int64_t sent[NW][16];  // the tile's vertices: first entry in the neighbour buffer,
+    __shared__ int32_t sdeg[NW][16];  // labels to gather
+    __shared__ int32_t tbuf[NW][kWarpBuf];
+    __shared__ int sfirst[6], slast[6], supto[7];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int gw = blockIdx.x * kMidWarps + w;
-    const int nw = gridDim.x * kMidWarps;
-    unsigned long long changes = 0;
-    unsigned long long *tab = stab[w];
     WarpBuf tb{tbuf[w]};
-    for (int s = lane; s < kMidSCap; s += 32) tab[s] = 0ull;
-    uint32_t gen = 0;
-    __syncwarp();
-    const int nwarp_v = p.disp->pos1;  // the degree-sorted mid list's prefix of warp vertices
-    constexpr int PER = kMidSMax / 32;
-    // the next vertex's head and neighbour IDs load while the current one is counted
-    auto ids_ahead = [&](int (&nb)[PER], const CtaHead &h) {
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int e = lane + u * 32;
-            nb[u] = (h.v >= 0 && h.dirty && e < h.deg) ? ld_nbr(&p.nbr[h.o0 + e - p.nbr_shift]) : -1;
+    unsigned long long changes = 0;
+    // the classes' list ranges and tiles, largest degrees first
+    if (threadIdx.x == 0) {
+        int tiles = 0;
+        const int pos1 = p.disp->pos1;
+        for (int g = 5; g >= 1; --g) {
+            const int f = max(p.gcut[g - 1], p.gstart), l = min(p.gcut[g], pos1), per = 32 >> g;
+            tiles += (max(l - f, 0) + per - 1) / per;
+            sfirst[g] = f;
+            slast[g] = l;
+            supto[g] = tiles;
         }
+        supto[6] = 0;
+    }
+    __syncthreads();
+    const int tiles = supto[1];
+    struct Head {
+        int v, deg, g;
+        int64_t o0;
+        int32_t old;
+        int dirty;
     };
-    CtaHead nxt = cta_head(p, 0, gw, nwarp_v, fr);
-    int nbn[PER];
-    ids_ahead(nbn, nxt);
-    for (int i = gw; i < nwarp_v; i += nw) {
-        const CtaHead h = nxt;
-        const int v = h.v;
-        int nb[PER];
-#pragma unroll
-        for (int u = 0; u < PER; ++u) nb[u] = nbn[u];
-        nxt = cta_head(p, 0, i + nw, nwarp_v, fr);
-        if (!h.dirty) {
-            tb.append(lane == 0 && carry_clean(p, v), v, p.tied_mid, &p.ctl->tied_mid);
-            ids_ahead(nbn, nxt);
-            continue;
-        }
-        if (++gen > kT64GenMax) {
-            for (int s = lane; s < kMidSCap; s += 32) tab[s] = 0ull;
-            __syncwarp();
-            gen = 1;
-        }
-        const int64_t o0 = h.o0;
-        const int deg = h.deg;
-        const uint32_t cap = (uint32_t)min(kMidSCap, 4 * pad32(deg));
-        uint32_t lb[PER];
-#pragma unroll
-        for (int u = 0; u < PER; ++u) lb[u] = (nb[u] >= 0) ? (uint32_t)ld_label(&p.lab_in[nb[u]]) : kEmpty;
-        Sum5 part = sum5_empty();  // observed counts (sum5_observe); d = claims
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            if (u * 32 >= deg) break;  // warp-uniform
-            // lanes holding the same label add once (heavy labels would serialise)
-            t64_insert_row(tab, cap, gen, lb[u], true, part);
-        }
-        ids_ahead(nbn, nxt);
-        __syncwarp();
-        const Sum5 sm = sum5_warp(part);
-        int rmin = 0, rmax = sm.d - 1;  // when every distinct label is a candidate
-        if (sm.k > 1) {
-            if (sm.k < sm.d) {
-                t64_ranks(tab, (int)cap, lane, 32, gen, sm.mn, sm.mx, rmin, rmax);
-                rmin = __reduce_add_sync(kFull, rmin);
-                rmax = __reduce_add_sync(kFull, rmax);
+    auto head = [&](int t) {
+        Head h{-1, 0, 1, 0, 0, 1};
+        if (t < tiles) {
+            h.g = 5;
+            while (t >= supto[h.g]) --h.g;  // the class whose tiles end above t
+            const int i = sfirst[h.g] + (t - supto[h.g + 1]) * (32 >> h.g) + (lane >> h.g);
+            if (i < slast[h.g]) {
+                h.v = p.mid_v[i];
+                h.o0 = __ldg(&p.off[h.v]);
+                h.deg = (int)(__ldg(&p.off[h.v + 1]) - h.o0);
+                h.old = __ldg(&p.lab_in[h.v]);
+                h.dirty = fr ? (int)p.dirty[h.v] : 1;
             }
-            if (sm.k > 2) {  // resolving may need the runs themselves (unsorted)
-                int32_t *rl = p.run_lab + (o0 - p.nbr_shift);
-                uint16_t *rc = p.run_cnt + (o0 - p.nbr_shift);
-                int base = 0;
-                for (int s0 = 0; s0 < (int)cap; s0 += 32) {  // cap is a multiple of 128
-                    const unsigned long long x = tab[s0 + lane];
-                    const bool occ = (uint32_t)(x >> kT64GenShift) == gen;
-                    const unsigned m = __ballot_sync(kFull, occ);
-                    if (occ) {
-                        const int at = base + __popc(m & ((1u << lane) - 1));
-                        rl[at] = (int32_t)((x >> 14) & 0x7FFFFFFF);
-                        rc[at] = (uint16_t)(x & kT64CntMask);
-                    }
-                    base += __popc(m);
+        }
+        return h;
+    };
+    const int nw = gridDim.x * NW;
+    int t = blockIdx.x * NW + w;
+    int32_t *rows = srow[w];
+    Head nxt = head(t);
+    for (; t < tiles; t += nw) {
+        const Head hd = nxt;
+        nxt = head(t + nw);
+        const int v = hd.v, g = hd.g, G = 1 << g, sub = lane & (G - 1);
+        const bool leader = sub == 0;
+        const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
+        const int n = (__reduce_max_sync(kFull, deg) + G - 1) >> g;
+        const GroupShape sh = n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
+        const int N = sh.N, stride = sh.stride;
+        if (leader) {
+            sent[w][lane >> g] = hd.o0 - p.nbr_shift;
+            sdeg[w][lane >> g] = deg;
+        }
+        for (int j = 0; j < N; j += 4)
+            *reinterpret_cast<int4 *>(rows + lane * stride + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+        __syncwarp();
+        // gather: row r holds entries 32 (r mod G) ... of the tile's vertex r / G
+        constexpr int PER = 8;  // rows in flight
+        for (int r0 = 0; r0 < 32; r0 += PER) {
+            int id[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+                id[u] = j < sdeg[w][q] ? ld_nbr(&p.nbr[sent[w][q] + j]) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+                if (id[u] >= 0)
+                    rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] = ld_label(&p.lab_in[id[u]]);
+            }
+        }
+        __syncwarp();
+        uint32_t h;
+        if (N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
+        else if (N == 24) h = group_sort_rows<24>(rows, g);
+        else h = group_sort_rows<32>(rows, g);
+        const int cnt = min(max(deg - sub * N, 0), N);  // labels in this lane
+        const uint32_t valid = cnt >= 32 ? kFull : (1u << cnt) - 1u;
+        h &= valid;
+        const uint32_t cont = ~h & valid;
+        // labels of the following lanes that continue this lane's last run: sums of the lanes'
+        // leading continuations up to and with the first lane that has a head
+        int ext = h ? __ffs(h) - 1 : cnt;
+        bool stop = h != 0u;
+        for (int o = 1; o < G; o <<= 1) {
+            const int e2 = __shfl_down_sync(kFull, ext, o);
+            const bool s2 = __shfl_down_sync(kFull, (int)stop, o);
+            if (sub + o < G && !stop) {
+                ext += e2;
+                stop = s2;
+            }
+        }
+        ext = __shfl_down_sync(kFull, ext, 1);
+        if (sub == G - 1) ext = 0;
+        const int lp = h ? 31 - __clz(h) : 0;     // the last head of the lane ...
+        const int tail = h ? cnt - lp + ext : 0;  // ... and the length of its run
+        uint32_t m = h & ~(1u << lp);             // the other heads, as for small vertices
+        int W = m ? 1 : 0;
+        while (m) {
+            const uint32_t more = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
+            if (!more) break;
+            m = more;
+            ++W;
+        }
+        int top = max(W, tail);
+        for (int o = G >> 1; o; o >>= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
+        m = (W == top ? m : 0u) | (tail == top && h ? 1u << lp : 0u);
+        // distinct labels and candidates of the group, and the rank of the lane's first head
+        int k = __popc(m), d = __popc(h);
+        for (int o = 1; o < G; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, d, o);
+            if (sub >= o) d += y;
+        }
+        const int rank0 = d - __popc(h);
+        for (int o = G >> 1; o; o >>= 1) k += __shfl_xor_sync(kFull, k, o);
+        d = __shfl_sync(kFull, d, lane | (G - 1));
+        // the smallest and largest candidate and their ranks, from the lanes that hold them
+        const unsigned gm = (G == 32 ? kFull : ((1u << G) - 1u)) << (lane - sub);
+        const unsigned holders = __ballot_sync(kFull, m != 0u) & gm;
+        const int lo = m ? __ffs(m) - 1 : 0, hi = m ? 31 - __clz(m) : 0;
+        const int l0 = holders ? __ffs(holders) - 1 : lane, l1 = holders ? 31 - __clz(holders) : lane;
+        Sum5 sm;
+        sm.d = d;
+        sm.W = top;
+        sm.k = k;
+        sm.mn = __shfl_sync(kFull, rows[lane * stride + lo], l0);
+        sm.mx = __shfl_sync(kFull, rows[lane * stride + hi], l1);
+        const int rmin = __shfl_sync(kFull, rank0 + __popc(h & ((1u << lo) - 1u)), l0);
+        const int rmax = __shfl_sync(kFull, rank0 + __popc(h & ((1u << hi) - 1u)), l1);
+        bool tied = false;
+        if (leader && v >= 0) {
+            if (!hd.dirty) tied = carry_clean(p, v);
+            else tied = finish_counted(p, v, sm, rmin, rmax, changes, hd.old, kSpillSorted);
+        }
+        tb.append(tied, v, p.tied_mid, &p.ctl->tied_mid);
+        unsigned spill = __ballot_sync(kFull, leader && deg > 0 && k > 2);
+        if (spill) {
+            if (N == 20) group_compact<20>(rows, g, h, m, rank0);
+            else if (N == 24) group_compact<24>(rows, g, h, m, rank0);
+            else group_compact<32>(rows, g, h, m, rank0);
+            const int64_t e0 = hd.o0 - p.nbr_shift;
+            while (spill) {  // one vertex after the other, coalesced
+                const int src = __ffs(spill) - 1;
+                spill &= spill - 1;
+                const int64_t e = __shfl_sync(kFull, e0, src);
+                const int dd = __shfl_sync(kFull, d, src), ww = __shfl_sync(kFull, top, src);
+                for (int r = lane; r < dd; r += 32) {
+                    const int32_t x = rows[src * stride + r];
+                    p.run_lab[e + r] = x & INT_MAX;
+                    p.run_cnt[e + r] = x < 0 ? (uint16_t)ww : (uint16_t)0;
                 }
             }
         }
-        const bool tied = lane == 0 && finish_counted(p, v, sm, rmin, rmax, changes, h.old);
-        tb.append(tied, v, p.tied_mid, &p.ctl->tied_mid);
         __syncwarp();
     }
     tb.flush(p.tied_mid, &p.ctl->tied_mid);
@@ -1074,7 +1313,7 @@ __global__ void __launch_bounds__(32 * kMidWarps) count_mid_sort_kernel(PipeArgs
     const int nw = gridDim.x * kMidWarps;
     unsigned long long changes = 0;
     WarpBuf tb{tbuf[w]};
-    const int nwarp_v = p.disp->pos1;  // the degree-sorted mid list's prefix of warp vertices
+    const int nwarp_v = p.gstart;  // the degree-sorted mid list's prefix of up to 256 neighbours
     for (int i = gw; i < nwarp_v; i += nw) {
         const int v = p.mid_v[i];
         if (fr && !p.dirty[v]) {
@@ -1286,16 +1525,10 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : THREADS >= 512 
     __shared__ int ctn;
     if (!ctl_active(p.ctl)) return;
     if (threadIdx.x == 0) ctn = 0;  // ordered before thread 0's own uses
-    // ranges of the degree-sorted mid list: 0 [pos1, pos_a), 1 [pos_a, pos2), 2 [pos2, pos_b),
-    // 3 [pos_b, end); with a narrow cut c, 0 is [max(pos1, c), pos_a) and 4 [pos1, min(pos_a, c))
+    // ranges of the degree-sorted mid list: 1 [pos_a, pos2), 2 [pos2, pos_b), 3 [pos_b, end)
     const DispatchState &ds = *p.disp;
-    int first = which == 0 ? ds.pos1 : which == 1 ? ds.pos_a : which == 2 ? ds.pos2 : which == 3 ? ds.pos_b : ds.pos1;
-    int end = which == 0 ? ds.pos_a : which == 1 ? ds.pos2 : which == 2 ? ds.pos_b : which == 3 ? p.nmid_s + p.nmid_l + p.nmid_x
-                                                                                            : ds.pos_a;
-    if (p.narrow_cut >= 0) {
-        if (which == 0) first = max(first, p.narrow_cut);
-        if (which == 4) end = min(end, p.narrow_cut);
-    }
+    const int first = which == 1 ? ds.pos_a : which == 2 ? ds.pos2 : ds.pos_b;
+    const int end = which == 1 ? ds.pos2 : which == 2 ? ds.pos_b : p.nmid_s + p.nmid_l + p.nmid_x;
     const int count = end - first;
     const bool fr = frontier_on(p);
     const int tid = threadIdx.x;
@@ -1842,6 +2075,35 @@ struct SpillTableQuery {
     }
 };
 
+// Spilled runs in label order (vertices counted by lane groups), one warp: the run of
+// rank r is entry r.
+struct SpillSortedQuery {
+    const uint16_t *cnt;
+    int d, W, rmin, rmax;
+    int lane;
+    __device__ int first_ge(int64_t x) const
+    {
+        if (x <= rmin) return rmin;
+        if (x > rmax) return -1;
+        for (int r0 = (int)x;; r0 += 32) {  // rank rmax is a candidate
+            const int r = r0 + lane;
+            const unsigned m = __ballot_sync(kFull, r <= rmax && (int)cnt[r] == W);
+            if (m) return r0 + __ffs(m) - 1;
+        }
+    }
+    __device__ int last_lt(int64_t y) const
+    {
+        if (y > rmax) return rmax;
+        if (y <= rmin) return -1;
+        for (int r0 = (int)y - 32;; r0 -= 32) {  // rank rmin is a candidate
+            const int r = r0 + lane;
+            const unsigned m = __ballot_sync(kFull, r >= rmin && (int)cnt[r] == W);
+            if (m) return r0 + 31 - __clz(m);
+        }
+    }
+    __device__ int tile_pick(int64_t) const { return -1; }  // d <= kGroupMax never spans a tile
+};
+
 __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
 {
     __shared__ int hist[kNW][256];
@@ -1852,7 +2114,7 @@ __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
     for (int i = blockIdx.x * kNW + w; i < nt; i += gridDim.x * kNW) {
         const int v = p.tied_mid[i];
         const int kw = p.sm_kw[v], rr = p.sm_r[v];
-        const int k = kw & 0xFFFF, W = kw >> 16, rmin = rr & 0xFFFF, rmax = rr >> 16;
+        const int k = kw & 0xFFFF, W = (kw >> 16) & 0x3FFF, rmin = rr & 0xFFFF, rmax = rr >> 16;
         const int d = p.dcnt[v];
         const RunScope rs = run_scope(p, v);
         const long long a = rs.a, N = rs.N;
@@ -1866,9 +2128,15 @@ __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
             nl = p.sm_c1[v];
         } else {
             const int64_t e = __ldg(&p.off[v]) - p.nbr_shift;
-            SpillTableQuery tq{p.run_lab + e, p.run_cnt + e, d, W, rmin, rmax, hist[w], lane};
-            if (q.fail) r = resolve_rank(a, d, N, is_last, tq);
-            nl = (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : (int32_t)tq.select(r);
+            if (kw & kSpillSorted) {
+                SpillSortedQuery sq{p.run_cnt + e, d, W, rmin, rmax, lane};
+                if (q.fail) r = resolve_rank(a, d, N, is_last, sq);
+                nl = (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : p.run_lab[e + r];
+            } else {
+                SpillTableQuery tq{p.run_lab + e, p.run_cnt + e, d, W, rmin, rmax, hist[w], lane};
+                if (q.fail) r = resolve_rank(a, d, N, is_last, tq);
+                nl = (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : (int32_t)tq.select(r);
+            }
         }
         if (lane == 0) {
             const int32_t old = __ldg(&p.lab_in[v]);

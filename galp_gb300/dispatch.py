@@ -1,9 +1,9 @@
 """Learned per-iteration dispatch: timing sweeps, training and evaluation.
 
 Every in-core iteration runs one row of a 16-entry variant table (include/galp_tools.h
-galp_dispatch_row): CTA-table inserts plain or warp-aggregated, the warp/CTA degree split
-at 128 or 256, the 256/1024-thread CTA split at 1024 or 2048, and the frontier on or off.
-All rows compute the same labels.  The fixed rule runs row 0 (row 1 once at most 5 % of
+galp_dispatch_row): CTA-table inserts plain or warp-aggregated, the 256/512-thread CTA
+split at 1024 or 2048, and the frontier on or off (rows that differ by 4 alone are the
+same).  All rows compute the same labels.  The fixed rule runs row 0 (row 1 once at most 5 % of
 the labels changed, in frontier mode); the learned rule runs the row an MLP predicts to be
 fastest from the iteration's features (degree histogram, changed fraction, distinct
 labels per CSR entry, iteration index).

@@ -19,8 +19,8 @@ typedef struct {
     int64_t n, m;          /* vertices, CSR entries */
     int64_t m_big;         /* CSR entries of vertices above 12288 neighbours (global-table path) */
     int64_t npacks;        /* packs of vertices with <= 32 neighbours (one warp each) */
-    int64_t nmid;          /* vertices with 33..256 neighbours (one warp each) */
-    int64_t nlarge;        /* vertices with 257..12288 neighbours (one CTA each, on-chip table) */
+    int64_t nmid;          /* vertices with 33..256 neighbours */
+    int64_t nlarge;        /* vertices with 257..12288 neighbours (above 1024 one CTA each, on-chip table) */
     int64_t nbig;          /* vertices on the global-table path */
     int64_t table_slots;   /* pair slots of those vertices' hash partitions (largest scope) */
     int32_t launches_per_iter; /* kernels launched per dense iteration (upper bound) */
@@ -68,24 +68,23 @@ typedef struct {
                                redo itself with the shift raised by one (up to 6).  Shift 0 counts a
                                partition in a 1024-thread CTA with a 128 KB table, 1 in 512 threads
                                with 64 KB (three per SM), 2 and above in 256 threads with 32 KB (six) */
-    int32_t cta_stage;      /* CTA counting of 257..2048 neighbours: 1 = the next vertex's neighbour IDs
+    int32_t cta_stage;      /* CTA counting of 1025..2048 neighbours: 1 = the next vertex's neighbour IDs
                                staged in shared memory by a bulk copy, 0 = global loads (default: the
                                stage takes unified L1 from the label gathers; 1.7x slower on R-MAT 26) */
-    int32_t cta_narrow;     /* 1 = vertices of 257..512 neighbours counted by 64-thread CTAs with 8 KB
-                               tables, split off the 128-thread CTA range (default); 0 = all of that
-                               range in 128-thread CTAs */
-    int32_t mid_sort;       /* vertices of 33..256 neighbours (the warp range): 1 = the segmented
-                               sort + reduce way (a 256-key bitonic sort per warp, runs from the
-                               sorted keys: the reference's method-0 counting), 0 = hash tables
-                               (default) */
+    int32_t cta_narrow;     /* 0 or 1 (default), without effect: it chose a CTA shape for 257..512
+                               neighbours, which groups of lanes now sort */
+    int32_t mid_sort;       /* vertices of 33..256 neighbours: 1 = the segmented sort + reduce way (a
+                               256-key bitonic sort per warp, runs from the sorted keys: the
+                               reference's method-0 counting), 0 = sorted by groups of lanes, as up
+                               to 1024 (default) */
 } galp_variant;
 
 /* One row of the in-core variant table (every row computes the same labels). */
 typedef struct {
     int32_t agg_mode;          /* CTA-table inserts: 1 warp-aggregated, 2 plain */
     int32_t frontier;          /* 1 = skip vertices whose neighbour labels did not change */
-    int32_t warp_max_degree;   /* mid vertices up to this degree: one warp each */
-    int32_t cta256_max_degree; /* then 256-thread CTAs up to this degree, 1024-thread CTAs above */
+    int32_t warp_max_degree;   /* mid vertices up to this degree: sorted by groups of lanes */
+    int32_t cta256_max_degree; /* then 256-thread CTAs up to this degree, larger CTAs above */
     int32_t pos1, pos2;        /* the same split as positions in the degree-sorted mid list */
 } galp_dispatch_row;
 
