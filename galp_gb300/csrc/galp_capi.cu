@@ -21,6 +21,7 @@
 
 #include "../../include/galp.h"
 #include "lp_kernels.cuh"
+#include "lp_fused.cuh"
 #include "galp_ctx.h"
 #include "dispatch_weights.inc"
 #include "../../include/galp_tools.h"
@@ -494,6 +495,7 @@ int Engine::setup(const galp_csr &g, const galp_opts &o, cudaStream_t st, int64_
         symmetric = frontier && chk[1] == 0 && chk[2] == 0;
         if (!symmetric) frontier = false;
     }
+    if (fused_fits() && (rc = setup_fused(st))) return rc;
     if (frontier) {
         GALP_CUDA(b_dirty.alloc(nn));
         GALP_CUDA(b_changed.alloc(sizeof(int32_t) * nn));
@@ -914,8 +916,107 @@ DispatchArgs Engine::dispatch_args(int it) const
     return a;
 }
 
+// Whether runs of this graph or batch may be one cooperative kernel: small ones, whose
+// iterations the launches of the separate kernels would bound.
+bool Engine::fused_fits() const
+{
+    return policy == 0 && (batched ? G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries : m <= kFusedMaxEntries) &&
+           n > 0 && n <= kFusedMaxVertices && sched.big_v.empty();
+}
+
+// ... and whether this run is: under the default kernels and the fixed rule, not in a stream
+// capture (the caller's graph gets the separate kernels).
+bool Engine::fused_run(cudaStream_t st, int niter) const
+{
+    if (!b_fused.p || niter < 1 || frontier || disp_mode != 0 || prof.on || variant.small_sort != 2 ||
+        variant.mid_sort || variant.cta_stage)
+        return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
+// Buffers and launch shape of one-kernel runs (once per graph).
+int Engine::setup_fused(cudaStream_t st)
+{
+    const Scope &sc = sched.scopes[0];
+    const int nmid = sc.nms + sc.nml + sc.nmx, ncta = nmid - sc.gcut[5];
+    fused_slots = ncta ? std::min(kXlSlots, 4 * ((sched.mid_deg[(size_t)(sc.m0 + nmid - 1)] + 31) & ~31)) : 0;
+    const bool narrow = m <= kFusedNarrowEntries;
+    fused_threads = narrow ? kFusedNarrow : kFusedWide;
+    fused_smem = std::max(narrow ? kFusedSmem<kFusedNarrow> : kFusedSmem<kFusedWide>,
+                          sizeof(unsigned long long) * (size_t)fused_slots);
+    fused_kernel = batched ? (narrow ? fused_run_kernel<true, kFusedNarrow> : fused_run_kernel<true, kFusedWide>)
+                           : (narrow ? fused_run_kernel<false, kFusedNarrow> : fused_run_kernel<false, kFusedWide>);
+    int64_t tiles = (sc.nsv + 31) / 32 + ncta;
+    for (int g = 1; g <= 5; ++g) tiles += (sc.gcut[g] - sc.gcut[g - 1] + (32 >> g) - 1) / (32 >> g);
+    fused_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, std::min(sms, kFusedMaxBlocks)));
+    GALP_CUDA(cudaFuncSetAttribute(fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sizeof(unsigned long long) * kXlSlots)));
+    const size_t graphs = batched ? (size_t)G : 1;
+    GALP_CUDA(b_fused.alloc(sizeof(FusedState) + sizeof(long long) * 3 * (kFusedMaxBlocks + graphs) +
+                            (batched ? sizeof(unsigned long long) * 3 * graphs : 0)));
+    return reset_fused(st);
+}
+
+// The barriers and sums of one-kernel runs as the first run finds them.
+int Engine::reset_fused(cudaStream_t st)
+{
+    GALP_CUDA(cudaMemsetAsync(b_fused.p, 0, b_fused.bytes, st));
+    return GALP_OK;
+}
+
+int Engine::enqueue_run_fused(cudaStream_t st, int niter, long long thr)
+{
+    const Scope &sc = sched.scopes[0];
+    FusedArgs a{};
+    a.p = pipe_args(sc);
+    a.p.nbr = (const int32_t *)b_nbr[0].p;
+    a.lab0 = (int32_t *)b_lab0.p;
+    a.lab1 = (int32_t *)b_lab1.p;
+    a.state = (FusedState *)b_fused.p;
+    a.d = dispatch_args(0);
+    a.n = n;
+    a.m = m;
+    a.thr = thr;
+    a.niter = niter;
+    a.shortcut = adj_sorted ? 1 : 0;
+    a.chunk = (int)((n + fused_blocks - 1) / fused_blocks);
+    a.slots = fused_slots;
+    a.agg_mode = variant.agg_mode;
+    a.pieces = kFusedMaxBlocks + (batched ? G : 1);
+    a.sums = (long long *)((FusedState *)b_fused.p + 1);
+    if (batched) {
+        a.g_changes = (unsigned long long *)(a.sums + 3 * (size_t)a.pieces);
+        a.g_active = (int32_t *)b_g_active.p;
+        a.g_iters = (int32_t *)b_g_iters.p;
+        a.g_counts = (long long *)b_g_counts.p;
+        a.g_max_iter = batch_max_iter;
+        a.early_exit = early_exit;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)fused_blocks);
+    cfg.blockDim = dim3((unsigned)fused_threads);
+    cfg.dynamicSmemBytes = fused_smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {  // not all of the device is ours
+        (void)cudaGetLastError();
+        b_fused.release();
+        return enqueue_run_incore(st, niter, thr);
+    }
+    GALP_CUDA(e);
+    launched("fused_run_kernel", st);
+    return GALP_OK;
+}
+
 int Engine::enqueue_run_incore(cudaStream_t st, int niter, long long thr)
 {
+    if (fused_run(st, niter)) return enqueue_run_fused(st, niter, thr);
     int32_t *lab[2] = {(int32_t *)b_lab0.p, (int32_t *)b_lab1.p};
     int rc = enqueue_init(st, niter, thr);
     if (rc) return rc;
@@ -1170,7 +1271,7 @@ int galp_enqueue(galp_ctx *ctx, int32_t niter)
     GALP_CUDA(cudaSetDevice(ctx->opts.device));
     GALP_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
     int rc;
-    if (ctx->eng.batched && !ctx->eng.prof.on) {
+    if (ctx->eng.batched && !ctx->eng.prof.on && !ctx->eng.fused_run(ctx->stream, niter)) {
         // the whole run (every iteration of every graph) as one CUDA-graph launch
         if (ctx->graph_iters != niter) {
             if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
@@ -1234,6 +1335,10 @@ int galp_sync(galp_ctx *ctx, galp_stats *st)
         st->err = c.err;
         st->runs_last = c.N;
         for (int i = 0; i < GALP_MAX_ITERS; ++i) st->updates[i] = (int64_t)c.counts[i];
+    }
+    if ((c.err & kErrLookback) && ctx->eng.b_fused.p) {  // barriers given up half-way
+        const int rc = ctx->eng.reset_fused(ctx->stream);
+        if (rc) return rc;
     }
     if (c.err & kErrFormat) return GALP_EFORMAT;
     if (c.err & kErrHubOverflow) return GALP_ENOMEM;

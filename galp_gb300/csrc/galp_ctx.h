@@ -9,6 +9,7 @@
 
 #include "../../include/galp.h"
 #include "../../include/galp_tools.h"
+#include "lp_fused.cuh"
 #include "lp_pipeline.cuh"
 
 namespace galp {
@@ -196,6 +197,11 @@ struct Engine {
     DevBuf b_lab0, b_lab1, b_ctl, b_bstat, b_big_a, b_bad;
     DevBuf b_dcnt, b_runbase, b_c0, b_c1, b_kw, b_r, b_run_lab, b_run_cnt, b_tsmall, b_tmid, b_bsum;
     DevBuf b_dirty, b_changed, b_chk;  // frontier mode; setup adjacency checks
+    // one-kernel runs (b_fused.p null: not for this graph): barriers, sums, changes per graph
+    DevBuf b_fused;
+    void (*fused_kernel)(FusedArgs) = nullptr;
+    int fused_blocks = 0, fused_threads = 0, fused_slots = 0;
+    size_t fused_smem = 0;
     DevBuf b_static_feat, b_vtab, b_disp, b_feat_log, b_var_log, b_weights;  // dispatch
     float static_feat[kDegBins + 3] = {};
     std::vector<DispatchState> vtab;   // variant table of the in-core scope
@@ -266,6 +272,11 @@ struct Engine {
     int enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, const int32_t *lab_in,
                       int32_t *lab_out, const uint8_t *dirty = nullptr, int32_t *changed = nullptr);
     int enqueue_run_incore(cudaStream_t st, int niter, long long thr);
+    bool fused_fits() const;
+    bool fused_run(cudaStream_t st, int niter) const;
+    int setup_fused(cudaStream_t st);
+    int reset_fused(cudaStream_t st);
+    int enqueue_run_fused(cudaStream_t st, int niter, long long thr);
     int run_outofcore(cudaStream_t st, int niter, long long thr);
     int enqueue_init(cudaStream_t st, int niter, long long thr);
     const int32_t *final_labels(int iters) const;

@@ -65,20 +65,16 @@ struct DispatchArgs {
 // / 40, log2 n / 40, log2 mean degree / 16, fraction of labels changed in the previous
 // iteration, distinct labels per CSR entry in the previous iteration (runs / m),
 // iteration / 16, frontier mode, constant 1, padding.
-__device__ __forceinline__ void dispatch_features(const DispatchArgs &a, float *f)
+// Feature i (0 <= i < kFeat) of iteration `it`, `changed` labels and `runs` after the one before
+__device__ __forceinline__ float dispatch_feature(const DispatchArgs &a, int i, int it, long long changed,
+                                                  long long runs)
 {
-    for (int i = 0; i < kDegBins + 3; ++i) f[i] = a.static_feat[i];
-    float chg = 1.f, dist = 1.f;
-    if (a.it > 0) {
-        chg = (float)((double)a.ctl->counts[a.it - 1] / (double)(a.n > 0 ? a.n : 1));
-        dist = (float)((double)a.ctl->N / (double)(a.m > 0 ? a.m : 1));
-    }
-    f[kDegBins + 3] = chg;
-    f[kDegBins + 4] = dist;
-    f[kDegBins + 5] = (float)a.it / 16.f;
-    f[kDegBins + 6] = a.frontier_mode ? 1.f : 0.f;
-    f[kDegBins + 7] = 1.f;
-    for (int i = kDegBins + 8; i < kFeat; ++i) f[i] = 0.f;
+    if (i < kDegBins + 3) return a.static_feat[i];
+    if (i == kDegBins + 3) return it > 0 ? (float)((double)changed / (double)(a.n > 0 ? a.n : 1)) : 1.f;
+    if (i == kDegBins + 4) return it > 0 ? (float)((double)runs / (double)(a.m > 0 ? a.m : 1)) : 1.f;
+    if (i == kDegBins + 5) return (float)it / 16.f;
+    if (i == kDegBins + 6) return a.frontier_mode ? 1.f : 0.f;
+    return i == kDegBins + 7 ? 1.f : 0.f;
 }
 
 // One block of kHid threads.
@@ -87,8 +83,10 @@ __global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
     __shared__ float x[kFeat], h1[kHid], h2[kHid], y[kVar];
     __shared__ int pick;
     const int t = threadIdx.x;
+    if (t < kFeat)
+        x[t] = dispatch_feature(a, t, a.it, a.it > 0 ? (long long)a.ctl->counts[a.it - 1] : 0, a.ctl->N);
+    __syncthreads();
     if (t == 0) {
-        dispatch_features(a, x);
         int v;
         if (a.mode == 2) {
             v = a.forced;
@@ -131,11 +129,10 @@ __global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
         if (!a.frontier_mode) d.frontier = 0;
         *a.out = d;
         if (a.it < kMaxLogIters) {
-            if (a.feat_log)
-                for (int i = 0; i < kFeat; ++i) a.feat_log[a.it * kFeat + i] = x[i];
             if (a.var_log) a.var_log[a.it] = pick;
         }
     }
+    if (t < kFeat && a.it < kMaxLogIters && a.feat_log) a.feat_log[a.it * kFeat + t] = x[t];
 }
 
 }  // namespace galp

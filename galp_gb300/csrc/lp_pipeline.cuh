@@ -131,6 +131,32 @@ __device__ __forceinline__ bool frontier_on(const PipeArgs &p)
     return p.dirty && !*((volatile int *)&p.ctl->frontier_off);
 }
 
+// Loads of the current labels.  LIVE: the running kernel itself wrote them in an earlier phase
+// (a grid-wide barrier lies between), so the non-coherent path must not be used.
+template <bool LIVE>
+__device__ __forceinline__ int32_t get_label(const int32_t *p)
+{
+    if constexpr (LIVE) {
+        int32_t v;
+        asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        return v;
+    } else {
+        return __ldg(p);
+    }
+}
+template <bool LIVE>
+__device__ __forceinline__ int32_t gather_label(const int32_t *p)
+{
+    if constexpr (LIVE) {
+        int32_t v;
+        asm volatile("{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_last.b64 pol, 1.0;\n\t"
+            "ld.global.L2::cache_hint.b32 %0, [%1], pol;\n\t}" : "=r"(v) : "l"(p));
+        return v;
+    } else {
+        return ld_label(p);
+    }
+}
+
 // Record a changed vertex for the next iteration's frontier (single thread).
 __device__ __forceinline__ void note_change(const PipeArgs &p, int32_t v, int32_t nl, int32_t old)
 {
@@ -727,6 +753,7 @@ struct TileBuf {
 
 // Gather a tile of one vertex per lane: the lane's `deg` labels, whose first entry is at e0
 // of the neighbour buffer, go to its row, padded to n words (a multiple of 4).
+template <bool LIVE>
 __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int deg, int64_t e0, int n)
 {
     const int lane = threadIdx.x & 31;
@@ -775,7 +802,7 @@ __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int d
         }
 #pragma unroll
         for (int u = 0; u < PER; ++u)
-            if (id[u] >= 0) B.rows[at[u]] = ld_label(&p.lab_in[id[u]]);
+            if (id[u] >= 0) B.rows[at[u]] = gather_label<LIVE>(&p.lab_in[id[u]]);
     }
     __syncwarp();
 }
@@ -801,6 +828,105 @@ __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int d
 // (an insertion sort per thread in shared memory before): 1,024 planted partitions of
 // together 526 M entries 55.5 -> 24.9 ms, R-MAT 24 9.8 -> 4.4 ms, R-MAT 26 with edge
 // factor 4 20.2 -> 11.5 ms, LFR of a million vertices 2.0 -> 0.73 ms.
+// What a lane needs of its vertex before counting it: loaded one tile ahead.
+struct TileHead {
+    int v, deg, g;  // vertex (-1 = none), its neighbours, log2 of its lanes
+    int64_t o0;     // first CSR entry
+    int32_t old;    // current label
+    int dirty;      // 0: frontier mode and no neighbour label changed
+};
+
+template <bool LIVE>
+__device__ __forceinline__ void tile_head(const PipeArgs &p, TileHead &h, int v, bool fr)
+{
+    h.v = v;
+    h.o0 = __ldg(&p.off[v]);
+    h.deg = (int)(__ldg(&p.off[v + 1]) - h.o0);
+    h.old = get_label<LIVE>(&p.lab_in[v]);
+    h.dirty = fr ? (int)p.dirty[v] : 1;
+}
+
+// Count the warp's 32 small vertices (one per lane), with the tile buffer B.  Writes their state
+// and the labels of untied ones; returns the lane's distinct count.
+template <bool LIVE>
+__device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const TileHead &hd,
+                                          unsigned long long &changes, bool &tied, bool &chg)
+{
+    const int lane = threadIdx.x & 31;
+    const int v = hd.v;
+    const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
+    const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
+    tile_gather<LIVE>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
+    int32_t *row = B.rows + lane * kSmallRow;
+    uint32_t h = 0u;
+    switch (n4) {  // warp-uniform
+    case 0: break;
+    case 1: h = small_sort_row<4>(row); break;
+    case 2: h = small_sort_row<8>(row); break;
+    case 3: h = small_sort_row<12>(row); break;
+    case 4: h = small_sort_row<16>(row); break;
+    case 5: h = small_sort_row<20>(row); break;
+    case 6: h = small_sort_row<24>(row); break;
+    case 7: h = small_sort_row<28>(row); break;
+    default: h = small_sort_row<32>(row); break;
+    }
+    const uint32_t valid = deg >= 32 ? kFull : (1u << deg) - 1u;
+    h &= valid;
+    const uint32_t cont = ~h & valid;
+    // heads of runs of at least W labels: such a run has W - 1 continuations behind its head
+    uint32_t m = h;
+    int W = 1;
+    for (;;) {
+        const uint32_t t = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
+        if (!t) break;
+        m = t;
+        ++W;
+    }
+    const int k = __popc(m);
+    tied = chg = false;
+    if (v >= 0) {
+        if (!hd.dirty) {
+            // no label around the vertex changed: its counts carry over
+            tied = hd.deg > 0 && (p.sm_kw[v] & 0xFFFF) > 1;
+            if (!tied) p.lab_out[v] = hd.old;
+        } else if (deg == 0) {
+            p.dcnt[v] = 0;
+            p.lab_out[v] = hd.old;
+        } else {
+            p.dcnt[v] = __popc(h);
+            p.sm_kw[v] = k | (W << 16);
+            if (k == 1) {
+                const int32_t nl = row[__ffs(m) - 1];
+                p.lab_out[v] = nl;
+                count_change(changes, nl, hd.old);
+                chg = nl != hd.old;
+            } else {
+                tied = true;
+                const int lo = __ffs(m) - 1, hi = 31 - __clz(m);
+                p.sm_c0[v] = k == 2 ? row[lo] : (int32_t)h;
+                p.sm_c1[v] = k == 2 ? row[hi] : (int32_t)m;
+                p.sm_r[v] = __popc(h & ((1u << lo) - 1u)) | (__popc(h & ((1u << hi) - 1u)) << 16);
+            }
+        }
+    }
+    if (__any_sync(kFull, k > 2)) {
+        const int total = __reduce_add_sync(kFull, deg);
+        const unsigned nz = __ballot_sync(kFull, deg > 0);
+        if (deg > 0 && k <= 2) B.dlt[__popc(nz & ((1u << lane) - 1u))] = LLONG_MIN;
+        __syncwarp();
+        for (int r = 0; r * 32 < total; ++r) {
+            const int s = r * 32 + lane;
+            const int own = B.owner(r);
+            if (s < total) {
+                const int64_t e = B.dlt[own];
+                if (e != LLONG_MIN) p.run_lab[e + s] = B.rows[B.at[own] + s];
+            }
+        }
+    }
+    __syncwarp();  // the tile buffer may be written again
+    return __popc(h);
+}
+
 constexpr int kSmallThreads = 128;
 constexpr int kSmallBlocks = 8;  // resident blocks per SM
 __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_kernel(PipeArgs p)
@@ -813,112 +939,26 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
-    // the next round's vertex, offsets, label and dirty flag load one round ahead
-    struct Head {
-        int v, deg;
-        int64_t o0;
-        int32_t old;
-        int dirty;
-    };
-    auto head = [&](int i) {
-        Head h{-1, 0, 0, 0, 1};
-        if (i < p.nsmall) {
-            h.v = p.small_v[i];
-            h.o0 = __ldg(&p.off[h.v]);
-            h.deg = (int)(__ldg(&p.off[h.v + 1]) - h.o0);
-            h.old = __ldg(&p.lab_in[h.v]);
-            h.dirty = fr ? (int)p.dirty[h.v] : 1;
-        }
-        return h;
-    };
     // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
     // window in turn, so that none has only the window's highest degrees
     const int stride = gridDim.x * kSmallThreads;
     int base = blockIdx.x * kSmallThreads;  // block-uniform
     int turn = w;
     auto ahead = [&](int from) {
-        const Head hd = head(from + turn * 32 + lane);
+        TileHead h{-1, 0, 0, 0, 0, 1};
+        const int i = from + turn * 32 + lane;
+        if (i < p.nsmall) tile_head<false>(p, h, p.small_v[i], fr);
         turn = (turn + 1) & (NW - 1);
-        return hd;
+        return h;
     };
-    TileBuf &B = stile[w];
-    Head nxt = ahead(base);
+    TileHead nxt = ahead(base);
     for (; base < p.nsmall; base += stride) {
-        const Head hd = nxt;
+        const TileHead hd = nxt;
         nxt = ahead(base + stride);
-        const int v = hd.v;
-        const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-        const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
-        tile_gather(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
-        int32_t *row = B.rows + lane * kSmallRow;
-        uint32_t h = 0u;
-        switch (n4) {  // warp-uniform
-        case 0: break;
-        case 1: h = small_sort_row<4>(row); break;
-        case 2: h = small_sort_row<8>(row); break;
-        case 3: h = small_sort_row<12>(row); break;
-        case 4: h = small_sort_row<16>(row); break;
-        case 5: h = small_sort_row<20>(row); break;
-        case 6: h = small_sort_row<24>(row); break;
-        case 7: h = small_sort_row<28>(row); break;
-        default: h = small_sort_row<32>(row); break;
-        }
-        const uint32_t valid = deg >= 32 ? kFull : (1u << deg) - 1u;
-        h &= valid;
-        const uint32_t cont = ~h & valid;
-        // heads of runs of at least W labels: such a run has W - 1 continuations behind its head
-        uint32_t m = h;
-        int W = 1;
-        for (;;) {
-            const uint32_t t = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
-            if (!t) break;
-            m = t;
-            ++W;
-        }
-        const int k = __popc(m);
-        bool tied = false, chg = false;
-        if (v >= 0) {
-            if (!hd.dirty) {
-                // no label around the vertex changed: its counts carry over
-                tied = hd.deg > 0 && (p.sm_kw[v] & 0xFFFF) > 1;
-                if (!tied) p.lab_out[v] = hd.old;
-            } else if (deg == 0) {
-                p.dcnt[v] = 0;
-                p.lab_out[v] = hd.old;
-            } else {
-                p.dcnt[v] = __popc(h);
-                p.sm_kw[v] = k | (W << 16);
-                if (k == 1) {
-                    const int32_t nl = row[__ffs(m) - 1];
-                    p.lab_out[v] = nl;
-                    count_change(changes, nl, hd.old);
-                    chg = nl != hd.old;
-                } else {
-                    tied = true;
-                    const int lo = __ffs(m) - 1, hi = 31 - __clz(m);
-                    p.sm_c0[v] = k == 2 ? row[lo] : (int32_t)h;
-                    p.sm_c1[v] = k == 2 ? row[hi] : (int32_t)m;
-                    p.sm_r[v] = __popc(h & ((1u << lo) - 1u)) | (__popc(h & ((1u << hi) - 1u)) << 16);
-                }
-            }
-        }
-        if (__any_sync(kFull, k > 2)) {
-            const int total = __reduce_add_sync(kFull, deg);
-            const unsigned nz = __ballot_sync(kFull, deg > 0);
-            if (deg > 0 && k <= 2) B.dlt[__popc(nz & ((1u << lane) - 1u))] = LLONG_MIN;
-            __syncwarp();
-            for (int r = 0; r * 32 < total; ++r) {
-                const int s = r * 32 + lane;
-                const int own = B.owner(r);
-                if (s < total) {
-                    const int64_t e = B.dlt[own];
-                    if (e != LLONG_MIN) p.run_lab[e + s] = B.rows[B.at[own] + s];
-                }
-            }
-        }
-        tb.append(tied, v, p.tied_small, &p.ctl->tied_small);
-        warp_note_changes(p, chg, v);
-        __syncwarp();
+        bool tied, chg;
+        small_tile<false>(p, stile[w], hd, changes, tied, chg);
+        tb.append(tied, hd.v, p.tied_small, &p.ctl->tied_small);
+        warp_note_changes(p, chg, hd.v);
     }
     tb.flush(p.tied_small, &p.ctl->tied_small);
     flush_changes(changes, p.ctl);
@@ -1088,177 +1128,191 @@ __device__ __forceinline__ void group_compact(int32_t *rows, int g, uint32_t h, 
 // copies, the next tile's during the sort, were slower (4-byte copies run at half the rate
 // of loads: 17.1 ms here, and 33 instead of 25 for the small vertices above).
 constexpr int kGroupMax = 1024;
+struct GroupBuf {
+    int32_t rows[32 * 36];
+    int64_t ent[16];  // the tile's vertices: first entry in the neighbour buffer,
+    int32_t deg[16];  // labels to gather
+};
+
+// The classes' list ranges and tiles, largest degrees first: tile t of a class g is the one with
+// upto[g + 1] <= t < upto[g], list entries first[g] + (t - upto[g + 1]) * (32 >> g) ...
+struct GroupTiles {
+    int first[6], last[6], upto[7];
+    __device__ void set(const PipeArgs &p, int pos1)  // one thread
+    {
+        int tiles = 0;
+        for (int g = 5; g >= 1; --g) {
+            const int f = max(p.gcut[g - 1], p.gstart), l = min(p.gcut[g], pos1), per = 32 >> g;
+            tiles += (max(l - f, 0) + per - 1) / per;
+            first[g] = f;
+            last[g] = l;
+            upto[g] = tiles;
+        }
+        upto[6] = 0;
+    }
+    __device__ __forceinline__ int count() const { return upto[1]; }
+};
+
+template <bool LIVE>
+__device__ __forceinline__ TileHead group_head(const PipeArgs &p, const GroupTiles &T, int t, bool fr)
+{
+    TileHead h{-1, 0, 1, 0, 0, 1};
+    if (t < T.count()) {
+        h.g = 5;
+        while (t >= T.upto[h.g]) --h.g;
+        const int i = T.first[h.g] + (t - T.upto[h.g + 1]) * (32 >> h.g) + ((int)(threadIdx.x & 31) >> h.g);
+        if (i < T.last[h.g]) tile_head<LIVE>(p, h, p.mid_v[i], fr);
+    }
+    return h;
+}
+
+// Count the warp's tile of vertices (one per group of lanes).  Writes their state and the
+// labels of untied ones; returns the group's distinct count.  tied: in the groups' first
+// lanes.
+template <bool LIVE>
+__device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const TileHead &hd,
+                                          unsigned long long &changes, bool &tied)
+{
+    const int lane = threadIdx.x & 31;
+    int32_t *rows = B.rows;
+    const int v = hd.v, g = hd.g, G = 1 << g, sub = lane & (G - 1);
+    const bool leader = sub == 0;
+    const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
+    const int n = (__reduce_max_sync(kFull, deg) + G - 1) >> g;
+    const GroupShape sh = n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
+    const int N = sh.N, stride = sh.stride;
+    if (leader) {
+        B.ent[lane >> g] = hd.o0 - p.nbr_shift;
+        B.deg[lane >> g] = deg;
+    }
+    for (int j = 0; j < N; j += 4)
+        *reinterpret_cast<int4 *>(rows + lane * stride + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+    __syncwarp();
+    // gather: row r holds entries 32 (r mod G) ... of the tile's vertex r / G
+    constexpr int PER = 8;  // rows in flight
+    for (int r0 = 0; r0 < 32; r0 += PER) {
+        int id[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+            id[u] = j < B.deg[q] ? ld_nbr(&p.nbr[B.ent[q] + j]) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+            if (id[u] >= 0)
+                rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] = gather_label<LIVE>(&p.lab_in[id[u]]);
+        }
+    }
+    __syncwarp();
+    uint32_t h;
+    if (N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
+    else if (N == 24) h = group_sort_rows<24>(rows, g);
+    else h = group_sort_rows<32>(rows, g);
+    const int cnt = min(max(deg - sub * N, 0), N);  // labels in this lane
+    const uint32_t valid = cnt >= 32 ? kFull : (1u << cnt) - 1u;
+    h &= valid;
+    const uint32_t cont = ~h & valid;
+    // labels of the following lanes that continue this lane's last run: sums of the lanes'
+    // leading continuations up to and with the first lane that has a head
+    int ext = h ? __ffs(h) - 1 : cnt;
+    bool stop = h != 0u;
+    for (int o = 1; o < G; o <<= 1) {
+        const int e2 = __shfl_down_sync(kFull, ext, o);
+        const bool s2 = __shfl_down_sync(kFull, (int)stop, o);
+        if (sub + o < G && !stop) {
+            ext += e2;
+            stop = s2;
+        }
+    }
+    ext = __shfl_down_sync(kFull, ext, 1);
+    if (sub == G - 1) ext = 0;
+    const int lp = h ? 31 - __clz(h) : 0;     // the last head of the lane ...
+    const int tail = h ? cnt - lp + ext : 0;  // ... and the length of its run
+    uint32_t m = h & ~(1u << lp);             // the other heads, as for small vertices
+    int W = m ? 1 : 0;
+    while (m) {
+        const uint32_t more = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
+        if (!more) break;
+        m = more;
+        ++W;
+    }
+    int top = max(W, tail);
+    for (int o = G >> 1; o; o >>= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
+    m = (W == top ? m : 0u) | (tail == top && h ? 1u << lp : 0u);
+    // distinct labels and candidates of the group, and the rank of the lane's first head
+    int k = __popc(m), d = __popc(h);
+    for (int o = 1; o < G; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, d, o);
+        if (sub >= o) d += y;
+    }
+    const int rank0 = d - __popc(h);
+    for (int o = G >> 1; o; o >>= 1) k += __shfl_xor_sync(kFull, k, o);
+    d = __shfl_sync(kFull, d, lane | (G - 1));
+    // the smallest and largest candidate and their ranks, from the lanes that hold them
+    const unsigned gm = (G == 32 ? kFull : ((1u << G) - 1u)) << (lane - sub);
+    const unsigned holders = __ballot_sync(kFull, m != 0u) & gm;
+    const int lo = m ? __ffs(m) - 1 : 0, hi = m ? 31 - __clz(m) : 0;
+    const int l0 = holders ? __ffs(holders) - 1 : lane, l1 = holders ? 31 - __clz(holders) : lane;
+    Sum5 sm;
+    sm.d = d;
+    sm.W = top;
+    sm.k = k;
+    sm.mn = __shfl_sync(kFull, rows[lane * stride + lo], l0);
+    sm.mx = __shfl_sync(kFull, rows[lane * stride + hi], l1);
+    const int rmin = __shfl_sync(kFull, rank0 + __popc(h & ((1u << lo) - 1u)), l0);
+    const int rmax = __shfl_sync(kFull, rank0 + __popc(h & ((1u << hi) - 1u)), l1);
+    tied = false;
+    if (leader && v >= 0) {
+        if (!hd.dirty) tied = carry_clean(p, v);
+        else tied = finish_counted(p, v, sm, rmin, rmax, changes, hd.old, kSpillSorted);
+    }
+    unsigned spill = __ballot_sync(kFull, leader && deg > 0 && k > 2);
+    if (spill) {
+        if (N == 20) group_compact<20>(rows, g, h, m, rank0);
+        else if (N == 24) group_compact<24>(rows, g, h, m, rank0);
+        else group_compact<32>(rows, g, h, m, rank0);
+        const int64_t e0 = hd.o0 - p.nbr_shift;
+        while (spill) {  // one vertex after the other, coalesced
+            const int src = __ffs(spill) - 1;
+            spill &= spill - 1;
+            const int64_t e = __shfl_sync(kFull, e0, src);
+            const int dd = __shfl_sync(kFull, d, src), ww = __shfl_sync(kFull, top, src);
+            for (int r = lane; r < dd; r += 32) {
+                const int32_t x = rows[src * stride + r];
+                p.run_lab[e + r] = x & INT_MAX;
+                p.run_cnt[e + r] = x < 0 ? (uint16_t)ww : (uint16_t)0;
+            }
+        }
+    }
+    __syncwarp();  // the tile buffer may be written again
+    return d;
+}
+
 constexpr int kGroupThreads = 128;
 constexpr int kGroupBlocks = 5;  // resident blocks per SM: 6, 4 and 8 were 1 to 9 % slower
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) count_group_kernel(PipeArgs p)
 {
     constexpr int NW = kGroupThreads / 32;
-    __shared__ __align__(16) int32_t srow[NW][32 * 36];
-    __shared__ int64_t sent[NW][16];  // the tile's vertices: first entry in the neighbour buffer,
-    __shared__ int32_t sdeg[NW][16];  // labels to gather
+    __shared__ __align__(16) GroupBuf stile[NW];
     __shared__ int32_t tbuf[NW][kWarpBuf];
-    __shared__ int sfirst[6], slast[6], supto[7];
+    __shared__ GroupTiles T;
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int w = threadIdx.x >> 5;
     WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
-    // the classes' list ranges and tiles, largest degrees first
-    if (threadIdx.x == 0) {
-        int tiles = 0;
-        const int pos1 = p.disp->pos1;
-        for (int g = 5; g >= 1; --g) {
-            const int f = max(p.gcut[g - 1], p.gstart), l = min(p.gcut[g], pos1), per = 32 >> g;
-            tiles += (max(l - f, 0) + per - 1) / per;
-            sfirst[g] = f;
-            slast[g] = l;
-            supto[g] = tiles;
-        }
-        supto[6] = 0;
-    }
+    if (threadIdx.x == 0) T.set(p, p.disp->pos1);
     __syncthreads();
-    const int tiles = supto[1];
-    struct Head {
-        int v, deg, g;
-        int64_t o0;
-        int32_t old;
-        int dirty;
-    };
-    auto head = [&](int t) {
-        Head h{-1, 0, 1, 0, 0, 1};
-        if (t < tiles) {
-            h.g = 5;
-            while (t >= supto[h.g]) --h.g;  // the class whose tiles end above t
-            const int i = sfirst[h.g] + (t - supto[h.g + 1]) * (32 >> h.g) + (lane >> h.g);
-            if (i < slast[h.g]) {
-                h.v = p.mid_v[i];
-                h.o0 = __ldg(&p.off[h.v]);
-                h.deg = (int)(__ldg(&p.off[h.v + 1]) - h.o0);
-                h.old = __ldg(&p.lab_in[h.v]);
-                h.dirty = fr ? (int)p.dirty[h.v] : 1;
-            }
-        }
-        return h;
-    };
     const int nw = gridDim.x * NW;
     int t = blockIdx.x * NW + w;
-    int32_t *rows = srow[w];
-    Head nxt = head(t);
-    for (; t < tiles; t += nw) {
-        const Head hd = nxt;
-        nxt = head(t + nw);
-        const int v = hd.v, g = hd.g, G = 1 << g, sub = lane & (G - 1);
-        const bool leader = sub == 0;
-        const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-        const int n = (__reduce_max_sync(kFull, deg) + G - 1) >> g;
-        const GroupShape sh = n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
-        const int N = sh.N, stride = sh.stride;
-        if (leader) {
-            sent[w][lane >> g] = hd.o0 - p.nbr_shift;
-            sdeg[w][lane >> g] = deg;
-        }
-        for (int j = 0; j < N; j += 4)
-            *reinterpret_cast<int4 *>(rows + lane * stride + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
-        __syncwarp();
-        // gather: row r holds entries 32 (r mod G) ... of the tile's vertex r / G
-        constexpr int PER = 8;  // rows in flight
-        for (int r0 = 0; r0 < 32; r0 += PER) {
-            int id[PER];
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
-                id[u] = j < sdeg[w][q] ? ld_nbr(&p.nbr[sent[w][q] + j]) : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
-                if (id[u] >= 0)
-                    rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] = ld_label(&p.lab_in[id[u]]);
-            }
-        }
-        __syncwarp();
-        uint32_t h;
-        if (N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
-        else if (N == 24) h = group_sort_rows<24>(rows, g);
-        else h = group_sort_rows<32>(rows, g);
-        const int cnt = min(max(deg - sub * N, 0), N);  // labels in this lane
-        const uint32_t valid = cnt >= 32 ? kFull : (1u << cnt) - 1u;
-        h &= valid;
-        const uint32_t cont = ~h & valid;
-        // labels of the following lanes that continue this lane's last run: sums of the lanes'
-        // leading continuations up to and with the first lane that has a head
-        int ext = h ? __ffs(h) - 1 : cnt;
-        bool stop = h != 0u;
-        for (int o = 1; o < G; o <<= 1) {
-            const int e2 = __shfl_down_sync(kFull, ext, o);
-            const bool s2 = __shfl_down_sync(kFull, (int)stop, o);
-            if (sub + o < G && !stop) {
-                ext += e2;
-                stop = s2;
-            }
-        }
-        ext = __shfl_down_sync(kFull, ext, 1);
-        if (sub == G - 1) ext = 0;
-        const int lp = h ? 31 - __clz(h) : 0;     // the last head of the lane ...
-        const int tail = h ? cnt - lp + ext : 0;  // ... and the length of its run
-        uint32_t m = h & ~(1u << lp);             // the other heads, as for small vertices
-        int W = m ? 1 : 0;
-        while (m) {
-            const uint32_t more = m & __funnelshift_rc(cont, 0u, W);  // a shift of 32 gives 0
-            if (!more) break;
-            m = more;
-            ++W;
-        }
-        int top = max(W, tail);
-        for (int o = G >> 1; o; o >>= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
-        m = (W == top ? m : 0u) | (tail == top && h ? 1u << lp : 0u);
-        // distinct labels and candidates of the group, and the rank of the lane's first head
-        int k = __popc(m), d = __popc(h);
-        for (int o = 1; o < G; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, d, o);
-            if (sub >= o) d += y;
-        }
-        const int rank0 = d - __popc(h);
-        for (int o = G >> 1; o; o >>= 1) k += __shfl_xor_sync(kFull, k, o);
-        d = __shfl_sync(kFull, d, lane | (G - 1));
-        // the smallest and largest candidate and their ranks, from the lanes that hold them
-        const unsigned gm = (G == 32 ? kFull : ((1u << G) - 1u)) << (lane - sub);
-        const unsigned holders = __ballot_sync(kFull, m != 0u) & gm;
-        const int lo = m ? __ffs(m) - 1 : 0, hi = m ? 31 - __clz(m) : 0;
-        const int l0 = holders ? __ffs(holders) - 1 : lane, l1 = holders ? 31 - __clz(holders) : lane;
-        Sum5 sm;
-        sm.d = d;
-        sm.W = top;
-        sm.k = k;
-        sm.mn = __shfl_sync(kFull, rows[lane * stride + lo], l0);
-        sm.mx = __shfl_sync(kFull, rows[lane * stride + hi], l1);
-        const int rmin = __shfl_sync(kFull, rank0 + __popc(h & ((1u << lo) - 1u)), l0);
-        const int rmax = __shfl_sync(kFull, rank0 + __popc(h & ((1u << hi) - 1u)), l1);
-        bool tied = false;
-        if (leader && v >= 0) {
-            if (!hd.dirty) tied = carry_clean(p, v);
-            else tied = finish_counted(p, v, sm, rmin, rmax, changes, hd.old, kSpillSorted);
-        }
-        tb.append(tied, v, p.tied_mid, &p.ctl->tied_mid);
-        unsigned spill = __ballot_sync(kFull, leader && deg > 0 && k > 2);
-        if (spill) {
-            if (N == 20) group_compact<20>(rows, g, h, m, rank0);
-            else if (N == 24) group_compact<24>(rows, g, h, m, rank0);
-            else group_compact<32>(rows, g, h, m, rank0);
-            const int64_t e0 = hd.o0 - p.nbr_shift;
-            while (spill) {  // one vertex after the other, coalesced
-                const int src = __ffs(spill) - 1;
-                spill &= spill - 1;
-                const int64_t e = __shfl_sync(kFull, e0, src);
-                const int dd = __shfl_sync(kFull, d, src), ww = __shfl_sync(kFull, top, src);
-                for (int r = lane; r < dd; r += 32) {
-                    const int32_t x = rows[src * stride + r];
-                    p.run_lab[e + r] = x & INT_MAX;
-                    p.run_cnt[e + r] = x < 0 ? (uint16_t)ww : (uint16_t)0;
-                }
-            }
-        }
-        __syncwarp();
+    TileHead nxt = group_head<false>(p, T, t, fr);
+    for (; t < T.count(); t += nw) {
+        const TileHead hd = nxt;
+        nxt = group_head<false>(p, T, t + nw, fr);
+        bool tied;
+        group_tile<false>(p, stile[w], hd, changes, tied);
+        tb.append(tied, hd.v, p.tied_mid, &p.ctl->tied_mid);
     }
     tb.flush(p.tied_mid, &p.ctl->tied_mid);
     flush_changes(changes, p.ctl);
@@ -1920,6 +1974,41 @@ struct SmallMaskQuery {
     __device__ int tile_pick(int64_t) const { return -1; }  // d <= 32 never spans a tile
 };
 
+// State of a small vertex: read where it is needed, or loaded beforehand in one round trip.
+struct SmallStateMem {
+    const PipeArgs &p;
+    int v;
+    __device__ int kw() const { return p.sm_kw[v]; }
+    __device__ int d() const { return p.dcnt[v]; }
+    __device__ int32_t c0() const { return p.sm_c0[v]; }
+    __device__ int32_t c1() const { return p.sm_c1[v]; }
+    __device__ int r() const { return p.sm_r[v]; }
+    __device__ int64_t o0() const { return __ldg(&p.off[v]); }
+};
+
+// New label of a tied small vertex with run scope rs (one thread).
+template <class State>
+__device__ __forceinline__ int32_t resolve_small(const PipeArgs &p, const RunScope &rs, const State &x)
+{
+    const int kw = x.kw(), d = x.d();
+    const int k = kw & 0xFFFF, W = kw >> 16;
+    if (k > 2 && p.small_sort == 2) {
+        SmallMaskQuery mq{(uint32_t)x.c0(), (uint32_t)x.c1()};
+        const int r = resolve_rank(rs.a, d, rs.N, rs.is_last, mq);
+        return p.run_lab[x.o0() - p.nbr_shift + mq.at(r)];
+    }
+    const int rr = x.r();
+    const int rmin = rr & 0xFFFF, rmax = rr >> 16;
+    SummaryQuery q(k, d, rmin, rmax);
+    int r = resolve_rank(rs.a, d, rs.N, rs.is_last, q);
+    if (!q.fail && r == rmin) return x.c0();
+    if (!q.fail && r == rmax) return x.c1();
+    const int64_t e = x.o0() - p.nbr_shift;
+    SpillRunQuery sq{p.run_lab + e, p.run_cnt + e, d, W};
+    if (q.fail) r = resolve_rank(rs.a, d, rs.N, rs.is_last, sq);
+    return p.run_lab[e + r];
+}
+
 __global__ void __launch_bounds__(kTB) resolve_small_kernel(PipeArgs p)
 {
     if (!ctl_active(p.ctl)) return;
@@ -1927,35 +2016,7 @@ __global__ void __launch_bounds__(kTB) resolve_small_kernel(PipeArgs p)
     unsigned long long changes = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
         const int v = p.tied_small[i];
-        const int kw = p.sm_kw[v], rr = p.sm_r[v];
-        const int k = kw & 0xFFFF, W = kw >> 16, rmin = rr & 0xFFFF, rmax = rr >> 16;
-        const int d = p.dcnt[v];
-        const RunScope rs = run_scope(p, v);
-        const long long a = rs.a, N = rs.N;
-        const bool is_last = rs.is_last;
-        int32_t nl;
-        if (k > 2 && p.small_sort == 2) {
-            SmallMaskQuery mq{(uint32_t)p.sm_c0[v], (uint32_t)p.sm_c1[v]};
-            const int r = resolve_rank(a, d, N, is_last, mq);
-            nl = p.run_lab[__ldg(&p.off[v]) - p.nbr_shift + mq.at(r)];
-            const int32_t old = __ldg(&p.lab_in[v]);
-            p.lab_out[v] = nl;
-            count_change(changes, nl, old);
-            note_change(p, v, nl, old);
-            continue;
-        }
-        SummaryQuery q(k, d, rmin, rmax);
-        int r = resolve_rank(a, d, N, is_last, q);
-        if (!q.fail && r == rmin) {
-            nl = p.sm_c0[v];
-        } else if (!q.fail && r == rmax) {
-            nl = p.sm_c1[v];
-        } else {
-            const int64_t e = __ldg(&p.off[v]) - p.nbr_shift;
-            SpillRunQuery sq{p.run_lab + e, p.run_cnt + e, d, W};
-            if (q.fail) r = resolve_rank(a, d, N, is_last, sq);
-            nl = p.run_lab[e + r];
-        }
+        const int32_t nl = resolve_small(p, run_scope(p, v), SmallStateMem{p, v});
         const int32_t old = __ldg(&p.lab_in[v]);
         p.lab_out[v] = nl;
         count_change(changes, nl, old);
@@ -2104,6 +2165,29 @@ struct SpillSortedQuery {
     __device__ int tile_pick(int64_t) const { return -1; }  // d <= kGroupMax never spans a tile
 };
 
+// New label of a tied mid-list vertex with run scope rs (one warp; hist: 256 ints of its shared
+// memory).
+__device__ __forceinline__ int32_t resolve_mid(const PipeArgs &p, int v, const RunScope &rs, int *hist)
+{
+    const int lane = threadIdx.x & 31;
+    const int kw = p.sm_kw[v], rr = p.sm_r[v];
+    const int k = kw & 0xFFFF, W = (kw >> 16) & 0x3FFF, rmin = rr & 0xFFFF, rmax = rr >> 16;
+    const int d = p.dcnt[v];
+    SummaryQuery q(k, d, rmin, rmax);
+    int r = resolve_rank(rs.a, d, rs.N, rs.is_last, q);
+    if (!q.fail && r == rmin) return p.sm_c0[v];
+    if (!q.fail && r == rmax) return p.sm_c1[v];
+    const int64_t e = __ldg(&p.off[v]) - p.nbr_shift;
+    if (kw & kSpillSorted) {
+        SpillSortedQuery sq{p.run_cnt + e, d, W, rmin, rmax, lane};
+        if (q.fail) r = resolve_rank(rs.a, d, rs.N, rs.is_last, sq);
+        return (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : p.run_lab[e + r];
+    }
+    SpillTableQuery tq{p.run_lab + e, p.run_cnt + e, d, W, rmin, rmax, hist, lane};
+    if (q.fail) r = resolve_rank(rs.a, d, rs.N, rs.is_last, tq);
+    return (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : (int32_t)tq.select(r);
+}
+
 __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
 {
     __shared__ int hist[kNW][256];
@@ -2113,31 +2197,7 @@ __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
     unsigned long long changes = 0;
     for (int i = blockIdx.x * kNW + w; i < nt; i += gridDim.x * kNW) {
         const int v = p.tied_mid[i];
-        const int kw = p.sm_kw[v], rr = p.sm_r[v];
-        const int k = kw & 0xFFFF, W = (kw >> 16) & 0x3FFF, rmin = rr & 0xFFFF, rmax = rr >> 16;
-        const int d = p.dcnt[v];
-        const RunScope rs = run_scope(p, v);
-        const long long a = rs.a, N = rs.N;
-        const bool is_last = rs.is_last;
-        SummaryQuery q(k, d, rmin, rmax);
-        int r = resolve_rank(a, d, N, is_last, q);
-        int32_t nl;
-        if (!q.fail && r == rmin) {
-            nl = p.sm_c0[v];
-        } else if (!q.fail && r == rmax) {
-            nl = p.sm_c1[v];
-        } else {
-            const int64_t e = __ldg(&p.off[v]) - p.nbr_shift;
-            if (kw & kSpillSorted) {
-                SpillSortedQuery sq{p.run_cnt + e, d, W, rmin, rmax, lane};
-                if (q.fail) r = resolve_rank(a, d, N, is_last, sq);
-                nl = (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : p.run_lab[e + r];
-            } else {
-                SpillTableQuery tq{p.run_lab + e, p.run_cnt + e, d, W, rmin, rmax, hist[w], lane};
-                if (q.fail) r = resolve_rank(a, d, N, is_last, tq);
-                nl = (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : (int32_t)tq.select(r);
-            }
-        }
+        const int32_t nl = resolve_mid(p, v, run_scope(p, v), hist[w]);
         if (lane == 0) {
             const int32_t old = __ldg(&p.lab_in[v]);
             p.lab_out[v] = nl;

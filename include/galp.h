@@ -138,7 +138,7 @@ int galp_run_noalloc(const galp_csr *graph, int32_t niter, int32_t early_exit, i
  * together, each with exactly the labels, iteration count and change counts of its own
  * in-core run (policy 0): labels start at graph-local IDs, run positions and the early
  * exit are per graph, and a graph that has exited keeps its labels while the others go
- * on.  A run is one CUDA-graph launch.  Vertices above 12288 neighbours are not
+ * on.  A run is one launch: a CUDA graph, or for small batches one kernel.  Vertices above 12288 neighbours are not
  * supported here (GALP_EUNSUPPORTED).
  *
  * galp_run_batch: one call over `count` host graphs; labels_out = int32[sum of n] in

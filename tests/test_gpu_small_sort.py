@@ -6,6 +6,7 @@ import pytest
 
 import galp_gb300
 import oracle
+from galp_gb300 import tools
 
 pytestmark = pytest.mark.gpu
 
@@ -23,6 +24,7 @@ def _graph(degs, pool, seed):
 
 def _check(g, niter=4, **opts):
     with galp_gb300.Propagator(g, early_exit=0, **opts) as p:
+        tools.profile(p, 1)  # the separate kernels, whatever the size
         for k in range(1, niter + 1):
             p.run(k)
             got = p.get_labels()
