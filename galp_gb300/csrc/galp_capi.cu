@@ -290,7 +290,6 @@ bool build_schedule(Schedule &S, int64_t n, const int64_t *off, const std::vecto
         sc.occ_slots = ooff;
         S.max_occ_slots = std::max(S.max_occ_slots, ooff);
         S.max_scope_edges = std::max(S.max_scope_edges, sc.e1 - sc.e0);
-        S.max_scope_small = std::max(S.max_scope_small, nsmall);
         S.max_scope_mid = std::max<int64_t>(S.max_scope_mid, (int64_t)sc.nms + sc.nml + sc.nmx);
         S.max_scope_vertices = std::max(S.max_scope_vertices, sc.v1 - sc.v0);
         S.scopes.push_back(sc);
@@ -430,13 +429,15 @@ int Engine::setup(const galp_csr &g, const galp_opts &o, cudaStream_t st, int64_
     GALP_CUDA(b_c0.alloc(sizeof(int32_t) * nn));
     GALP_CUDA(b_c1.alloc(sizeof(int32_t) * nn));
     GALP_CUDA(b_kw.alloc(sizeof(int32_t) * nn));
+    GALP_CUDA(cudaMemsetAsync(b_kw.p, 0, sizeof(int32_t) * nn, st));  // 0 stays in hubs (resolve_kernel)
     GALP_CUDA(b_r.alloc(sizeof(int32_t) * nn));
     const size_t ms = (size_t)std::max<int64_t>(sched.max_scope_edges, 1);
     GALP_CUDA(b_run_lab.alloc(sizeof(int32_t) * ms));
     GALP_CUDA(b_run_cnt.alloc(sizeof(uint16_t) * ms));
-    GALP_CUDA(b_tsmall.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(sched.max_scope_small, 1)));
     GALP_CUDA(b_tmid.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(sched.max_scope_mid, 1)));
-    GALP_CUDA(b_bsum.alloc(sizeof(int64_t) * (size_t)std::max<int64_t>((sched.max_scope_vertices + kScanBlock - 1) / kScanBlock, 1)));
+    const size_t pieces = (size_t)(sched.max_scope_vertices / kRunBlock + 1 + (batched ? G : 0));
+    GALP_CUDA(b_bsum.alloc(sizeof(long long) * 2 * pieces));
+    GALP_CUDA(cudaMemsetAsync(b_bsum.p, 0, sizeof(long long) * pieces, st));  // sums; then their scan
     GALP_CUDA(cudaStreamSynchronize(st));
     phase(2);
     // dispatch: static features, variant table, per-scope state, logs
@@ -544,6 +545,7 @@ int Engine::setup_batch(const galp_csr &g, const int64_t *graph_v0, int32_t coun
     if ((rc = upload(b_g_v0, dv0, g_v0_h, st, h2d))) return rc;
     if ((rc = upload(b_g_last, dummy, g_last_h, st, h2d))) return rc;
     GALP_CUDA(b_g_base.alloc(sizeof(int64_t) * (count + 1)));
+    GALP_CUDA(b_g_changes.alloc(sizeof(unsigned long long) * count));
     GALP_CUDA(b_gid.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(g.n, 1)));
     batch_gid_kernel<<<(unsigned)std::min<int64_t>(count, 4096), kTB, 0, st>>>(dv0, count, (int32_t *)b_gid.p);
     max_label = 0;
@@ -680,7 +682,9 @@ PipeArgs Engine::pipe_args(const Scope &sc) const
     q.small_sort = variant.small_sort;
     if (batched) {
         q.g_v0 = (const int64_t *)b_g_v0.p;
-        q.g_base = (const int64_t *)b_g_base.p;
+        q.g_base = (int64_t *)b_g_base.p;
+        q.g_active = (const int32_t *)b_g_active.p;
+        q.g_changes = (unsigned long long *)b_g_changes.p;
         q.g_last = (const int32_t *)b_g_last.p;
         q.gid = (const int32_t *)b_gid.p;
         q.ngraphs = G;
@@ -705,11 +709,11 @@ PipeArgs Engine::pipe_args(const Scope &sc) const
     q.sm_r = (int32_t *)b_r.p;
     q.run_lab = (int32_t *)b_run_lab.p;
     q.run_cnt = (uint16_t *)b_run_cnt.p;
-    q.tied_small = (int32_t *)b_tsmall.p;
     q.tied_mid = (int32_t *)b_tmid.p;
     q.v0 = sc.v0;
     q.v1 = sc.v1;
-    q.bsum = (int64_t *)b_bsum.p;
+    q.sums = (long long *)b_bsum.p;
+    q.run_at = q.sums + b_bsum.bytes / (2 * sizeof(long long));
     q.last_v = sc.last_v;
     for (int i = 0; i < 6; ++i) q.gcut[i] = sc.gcut[i];
     q.gstart = variant.mid_sort ? sc.gcut[3] : 0;
@@ -722,14 +726,12 @@ int Engine::launch_limits()
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_group, count_group_kernel, kGroupThreads, 0));
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_mid_sort, count_mid_sort_kernel, 32 * kMidWarps, 0));
     occ_mid_sort = std::max(occ_mid_sort, 1);
-    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resolve, resolve_small_kernel, kTB, 0));
-    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resolve_mid, resolve_mid_kernel, kTB, 0));
+    GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_resolve_mid, resolve_mid_kernel<false>, kTB, 0));
     // the CTA kernels loop over their vertex range: a grid of exactly the resident blocks
     GALP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_cta256, count_cta_kernel<kTB, 2 * kLargeMax>, kTB,
                                                             sizeof(unsigned long long) * 2 * kLargeMax));
     occ_cta256 = std::max(occ_cta256, 1);
     occ_group = std::max(occ_group, 1);
-    occ_resolve = std::max(occ_resolve, 1);
     occ_resolve_mid = std::max(occ_resolve_mid, 1);
     return GALP_OK;
 }
@@ -752,9 +754,6 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     q.lab_out = lab_out;
     q.dirty = dirty;
     q.changed = changed;
-    Ctl *ctl = (Ctl *)b_ctl.p;
-    GALP_CUDA(cudaMemsetAsync(&ctl->tied_small, 0, 2 * sizeof(int), st));
-    prof.kmark("memset", st);
     int e0 = -1;
     if (a.nbig) {
         if (prof.on) e0 = prof.mark(st);
@@ -773,12 +772,10 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
             hub_count_kernel<kHubCountThreads, kHubTab>
                 <<<std::min(a.nparts, hub_count_blocks), kHubCountThreads, sizeof(uint32_t) * 2 * kHubTab, st>>>(a);
         launched("hub_count_kernel", st);
-        big_combine_kernel<<<(a.nbig + 7) / 8, 256, 0, st>>>(a);
+        big_combine_kernel<<<(a.nbig + 7) / 8, 256, 0, st>>>(a, q);
         launched("big_combine_kernel", st);
         big_stats_kernel<<<a.nschunks, kTB, 0, st>>>(a);
         launched("big_stats_kernel", st);
-        big_dcnt_kernel<<<(a.nbig + 255) / 256, 256, 0, st>>>(a, q.dcnt);
-        launched("big_dcnt_kernel", st);
         if (prof.on) prof.spans[1].push_back({e0, prof.mark(st)});
     }
     if (prof.on) e0 = prof.mark(st);
@@ -839,23 +836,17 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     }
     const int64_t nv = sc.v1 - sc.v0;
     if (nv > 0) {
-        const int nblk = (int)((nv + kScanBlock - 1) / kScanBlock);
-        scan_reduce_kernel<<<nblk, kTB, 0, st>>>(q);
-        launched("scan_reduce_kernel", st);
-        scan_spine_kernel<<<1, kTB, 0, st>>>(q, nblk);
-        launched("scan_spine_kernel", st);
-        scan_apply_kernel<<<nblk, kTB, 0, st>>>(q);
-        launched("scan_apply_kernel", st);
+        const int blocks = (int)((nv + kRunBlock - 1) / kRunBlock);
+        scan_kernel<<<1, kScanThreads, 0, st>>>(q, blocks + (batched ? G : 0));
+        launched("scan_kernel", st);
+        if (batched) resolve_kernel<true><<<blocks, kTB, 0, st>>>(q);
+        else resolve_kernel<false><<<blocks, kTB, 0, st>>>(q);
+        launched("resolve_kernel", st);
     }
-    if (batched) {
-        batch_bases_kernel<<<(G + 1 + 255) / 256, 256, 0, st>>>((const int64_t *)b_g_v0.p, G, q.runbase, n,
-                                                                (const Ctl *)b_ctl.p, (int64_t *)b_g_base.p);
-        launched("batch_bases_kernel", st);
-    }
-    resolve_small_kernel<<<sms * std::min(resolve_bps, occ_resolve), kTB, 0, st>>>(q);
-    launched("resolve_small_kernel", st);
     if (q.nmid_s + q.nmid_l + q.nmid_x) {
-        resolve_mid_kernel<<<sms * occ_resolve_mid, kTB, 0, st>>>(q);
+        const int blocks = sms * std::min(resolve_bps, occ_resolve_mid);
+        if (batched) resolve_mid_kernel<true><<<blocks, kTB, 0, st>>>(q);
+        else resolve_mid_kernel<false><<<blocks, kTB, 0, st>>>(q);
         launched("resolve_mid_kernel", st);
     }
     if (prof.on) prof.spans[0].push_back({e0, prof.mark(st)});
@@ -863,8 +854,6 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
         if (prof.on) e0 = prof.mark(st);
         big_resolve_kernel<<<a.nbig, 32, sizeof(uint32_t) * kPickScratch, st>>>(a);
         launched("big_resolve_kernel", st);
-        big_reset_kernel<<<(a.nbig + 255) / 256, 256, 0, st>>>(a);
-        launched("big_reset_kernel", st);
         if (prof.on) prof.spans[2].push_back({e0, prof.mark(st)});
     }
     GALP_CUDA(cudaGetLastError());
@@ -878,8 +867,8 @@ int Engine::enqueue_init(cudaStream_t st, int niter, long long thr)
         batch_init_labels_kernel<<<(unsigned)std::min<int64_t>(G, (int64_t)sms * 8), kTB, 0, st>>>(
             (const int64_t *)b_g_v0.p, G, (int32_t *)b_lab0.p);
         launched("batch_init_labels_kernel", st);
-        batch_init_kernel<<<(G + 255) / 256, 256, 0, st>>>((int32_t *)b_g_active.p, (int32_t *)b_g_iters.p, G,
-                                                           niter > 0 ? 1 : 0);
+        batch_init_kernel<<<(G + 255) / 256, 256, 0, st>>>((int32_t *)b_g_active.p, (int32_t *)b_g_iters.p,
+                                                           (unsigned long long *)b_g_changes.p, G, niter > 0 ? 1 : 0);
         launched("batch_init_kernel", st);
     } else if (n > 0) {
         const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 4096);
@@ -1029,8 +1018,9 @@ int Engine::enqueue_run_incore(cudaStream_t st, int niter, long long thr)
     for (int it = 0; it < niter; ++it) {
         const int it0 = prof.on ? prof.mark(st) : -1;
         const bool shortcut = it == 0 && adj_sorted && n > 0;
-        if (!shortcut) {
-            // this iteration's kernel variant, decided on the device
+        if (!shortcut && it == 0) {
+            // the first iteration's kernel variant, decided on the device; later ones are decided
+            // at the end of the iteration before
             dispatch_kernel<<<1, kHid, 0, st>>>(dispatch_args(it));
             launched("dispatch_kernel", st);
         }
@@ -1066,12 +1056,14 @@ int Engine::enqueue_run_incore(cudaStream_t st, int niter, long long thr)
             full_state = true;
         }
         if (batched) {  // per-graph change counts, early exits and frozen graphs
-            batch_commit_kernel<<<(unsigned)std::min<int64_t>(G, (int64_t)sms * 8), kTB, 0, st>>>(
-                ctl, (const int64_t *)b_g_v0.p, G, lab[it & 1], lab[(it + 1) & 1], (int32_t *)b_g_active.p,
-                (int32_t *)b_g_iters.p, (long long *)b_g_counts.p, batch_max_iter, it, early_exit);
-            launched("batch_commit_kernel", st);
-            batch_finalize_kernel<<<1, 1024, 0, st>>>(ctl, (const int32_t *)b_g_active.p, G);
+            batch_finalize_kernel<<<1, 1024, 0, st>>>(ctl, (const int64_t *)b_g_v0.p, (int32_t *)b_g_active.p,
+                                                      (int32_t *)b_g_iters.p, (long long *)b_g_counts.p,
+                                                      (unsigned long long *)b_g_changes.p, G, batch_max_iter, it,
+                                                      early_exit, it + 1 < niter ? dispatch_args(it + 1) : DispatchArgs{});
             launched("batch_finalize_kernel", st);
+        } else if (it + 1 < niter) {
+            finalize_dispatch_kernel<<<1, kHid, 0, st>>>(ctl, dispatch_args(it + 1));
+            launched("finalize_dispatch_kernel", st);
         } else {
             finalize_kernel<<<1, 1, 0, st>>>(ctl);
             launched("finalize_kernel", st);
@@ -1449,7 +1441,7 @@ int galp_schedule_info(galp_ctx *ctx, galp_sched_info *info)
     info->nlarge = nml;
     info->nbig = (int64_t)E.sched.big_v.size();
     info->table_slots = E.sched.max_pair_slots;
-    info->launches_per_iter = 14 + (info->nbig ? 7 : 0) + (E.frontier ? 1 : 0);
+    info->launches_per_iter = 11 + (info->nbig ? 5 : 0) + (E.frontier ? 1 : 0);
     info->flags = (E.adj_sorted ? GALP_SCHED_SORTED : 0) | (E.symmetric ? GALP_SCHED_SYMMETRIC : 0) |
                   (E.frontier ? GALP_SCHED_FRONTIER : 0);
     info->launches = E.launches;

@@ -86,7 +86,7 @@ struct Schedule {
     int hub_shift = 0;               // partitions per hub: degree * 2^hub_shift / kHubPartPairs
     std::vector<Scope> scopes;
     int64_t max_pair_slots = 0, max_occ_slots = 0, max_scope_edges = 0, m_big = 0;
-    int64_t max_scope_small = 0, max_scope_mid = 0, max_scope_vertices = 0;
+    int64_t max_scope_mid = 0, max_scope_vertices = 0;
     double deg_hist[kDegBins] = {};  // CSR entries by log2 degree (dispatch features)
 };
 
@@ -195,7 +195,7 @@ struct Engine {
     DevBuf b_chunk_big, b_chunk_e0, b_chunk_e1, b_schunk_big, b_schunk_s0, b_schunk_s1, b_big_ooff;
     DevBuf b_hub_p0, b_hub_pbase, b_hub_pcap, b_part_big, b_pfill, b_psum, b_pairs, b_big_list;
     DevBuf b_lab0, b_lab1, b_ctl, b_bstat, b_big_a, b_bad;
-    DevBuf b_dcnt, b_runbase, b_c0, b_c1, b_kw, b_r, b_run_lab, b_run_cnt, b_tsmall, b_tmid, b_bsum;
+    DevBuf b_dcnt, b_runbase, b_c0, b_c1, b_kw, b_r, b_run_lab, b_run_cnt, b_tmid, b_bsum;
     DevBuf b_dirty, b_changed, b_chk;  // frontier mode; setup adjacency checks
     // one-kernel runs (b_fused.p null: not for this graph): barriers, sums, changes per graph
     DevBuf b_fused;
@@ -242,14 +242,14 @@ struct Engine {
     int batch_max_iter = 0;   // row length of b_g_counts
     std::vector<int64_t> g_v0_h;
     std::vector<int32_t> g_last_h;
-    DevBuf b_g_v0, b_g_base, b_g_last, b_g_active, b_g_iters, b_g_counts, b_gid;
+    DevBuf b_g_v0, b_g_base, b_g_changes, b_g_last, b_g_active, b_g_iters, b_g_counts, b_gid;
     int64_t max_label = 0;    // labels stay below this (n, or the largest graph of a batch)
     // launch shapes (blocks per SM), chosen by galp_batch_tune
     int small_bps = 16, mid_bps = 8, resolve_bps = 4;
     // resident blocks per SM of the mid-vertex counting and the resolve kernels (occupancy
     // API): their grid-stride loops run as one full wave, since a partial second wave
     // would start its blocks' whole shares late
-    int occ_group = 0, occ_mid_sort = 0, occ_resolve = 0, occ_resolve_mid = 0;
+    int occ_group = 0, occ_mid_sort = 0, occ_resolve_mid = 0;
     int occ_cta256 = 0;
     int launch_limits();
     // hub partitions at 2^shift times the default count: plan, upload, size the pair area

@@ -77,8 +77,9 @@ __device__ __forceinline__ float dispatch_feature(const DispatchArgs &a, int i, 
     return i == kDegBins + 7 ? 1.f : 0.f;
 }
 
-// One block of kHid threads.
-__global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
+// The state of the iteration about to run, by one block of at least kHid threads (all of
+// them call it); what it reads of *ctl the block's earlier writes may have written.
+__device__ __forceinline__ void dispatch_step(const DispatchArgs &a)
 {
     __shared__ float x[kFeat], h1[kHid], h2[kHid], y[kVar];
     __shared__ int pick;
@@ -100,16 +101,20 @@ __global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
     if (a.mode == 1) {
         const float *W1 = a.weights, *b1 = W1 + kFeat * kHid, *W2 = b1 + kHid, *b2 = W2 + kHid * kHid;
         const float *W3 = b2 + kHid, *b3 = W3 + kHid * kVar;
-        float s = b1[t];
-        for (int i = 0; i < kFeat; ++i) s += x[i] * W1[i * kHid + t];
-        h1[t] = fmaxf(s, 0.f);
+        if (t < kHid) {
+            float s = b1[t];
+            for (int i = 0; i < kFeat; ++i) s += x[i] * W1[i * kHid + t];
+            h1[t] = fmaxf(s, 0.f);
+        }
         __syncthreads();
-        s = b2[t];
-        for (int i = 0; i < kHid; ++i) s += h1[i] * W2[i * kHid + t];
-        h2[t] = fmaxf(s, 0.f);
+        if (t < kHid) {
+            float s = b2[t];
+            for (int i = 0; i < kHid; ++i) s += h1[i] * W2[i * kHid + t];
+            h2[t] = fmaxf(s, 0.f);
+        }
         __syncthreads();
         if (t < kVar) {
-            s = b3[t];
+            float s = b3[t];
             for (int i = 0; i < kHid; ++i) s += h2[i] * W3[i * kVar + t];
             y[t] = s;
         }
@@ -128,11 +133,24 @@ __global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
         if (a.mode == 0) d.agg_mode = a.fixed_agg;
         if (!a.frontier_mode) d.frontier = 0;
         *a.out = d;
-        if (a.it < kMaxLogIters) {
-            if (a.var_log) a.var_log[a.it] = pick;
-        }
+        if (a.it < kMaxLogIters && a.var_log) a.var_log[a.it] = pick;
     }
     if (t < kFeat && a.it < kMaxLogIters && a.feat_log) a.feat_log[a.it * kFeat + t] = x[t];
+}
+
+// Before the first iteration that needs a state; later states follow the iteration's end
+// (finalize_dispatch_kernel).
+__global__ void __launch_bounds__(kHid) dispatch_kernel(DispatchArgs a)
+{
+    dispatch_step(a);
+}
+
+// End of an iteration (finalize_kernel) and the next one's state.
+__global__ void __launch_bounds__(kHid) finalize_dispatch_kernel(Ctl *ctl, DispatchArgs a)
+{
+    if (threadIdx.x == 0) finalize_iteration(ctl);
+    __syncthreads();
+    dispatch_step(a);
 }
 
 }  // namespace galp

@@ -93,18 +93,6 @@ __device__ __forceinline__ bool grid_barrier(FusedState *st, Ctl *ctl, int *fail
     return !*failed;
 }
 
-// Add the distinct counts of a warp's vertices (0 in lanes without one) to their pieces' sums.
-__device__ __forceinline__ void add_piece(long long *sums, int piece, int d)
-{
-    const int c0 = __reduce_max_sync(kFull, d ? piece : 0);
-    if (__all_sync(kFull, !d || piece == c0)) {
-        const int all = __reduce_add_sync(kFull, d);
-        if ((threadIdx.x & 31) == 0 && all) atomicAdd((unsigned long long *)&sums[c0], (unsigned long long)all);
-    } else if (d) {
-        atomicAdd((unsigned long long *)&sums[piece], (unsigned long long)d);
-    }
-}
-
 // Dynamic shared memory: the warps' tile buffers, or the block's hash table, or the resolve
 // phase's buffers.
 template <int THREADS>
@@ -131,15 +119,9 @@ static_assert(sizeof(FusedResolve<kFusedNarrow>) <= kFusedSmem<kFusedNarrow> &&
 
 // State of a vertex in the resolve phase, loaded in one round trip whether it is tied or not.
 struct FusedVertex {
-    int d_, kw_, r_, g, gprev;  // g: its graph, gprev: the graph of the vertex before
-    int32_t c0_, c1_, old, now; // its label before, and after the count where it is not tied
-    int64_t o0_, o1;
-    __device__ int kw() const { return kw_; }
-    __device__ int d() const { return d_; }
-    __device__ int32_t c0() const { return c0_; }
-    __device__ int32_t c1() const { return c1_; }
-    __device__ int r() const { return r_; }
-    __device__ int64_t o0() const { return o0_; }
+    int d, kw, r, g, gprev;    // g: its graph, gprev: the graph of the vertex before
+    int32_t c0, c1, old, now;  // its label before, and after the count where it is not tied
+    int64_t o0;
 };
 
 template <bool BATCH, int kFusedThreads>
@@ -176,7 +158,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             ctl->changes = 0;
             ctl->changed_n = 0;
             ctl->frontier_off = 0;
-            ctl->tied_small = ctl->tied_mid = 0;
+            ctl->tied_mid = 0;
             st->changes[0] = 0;
         }
         if (tid < 64) ctl->counts[tid] = 0;
@@ -340,19 +322,18 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 TileHead hd = group0;
                 if (r != w) hd = group_head<true>(p, T, tile_of(r), false);
                 else if (hd.v >= 0) hd.old = get_label<true>(&p.lab_in[hd.v]);
-                bool tied;
-                const int d = group_tile<true>(p, tiles[w].group, hd, changes, tied);
+                const int d = group_tile<true>(p, tiles[w].group, hd, changes);
                 const bool leader = (lane & ((1 << hd.g) - 1)) == 0;
-                add_piece(sums, piece_of(hd.v), leader && hd.v >= 0 ? d : 0);
+                add_runs(sums, piece_of(hd.v), leader && hd.v >= 0 ? d : 0);
                 if (leader && hd.v >= 0) counted += (unsigned)d;
             }
             for (int r = w; r * nb < nsmall; r += kFusedWarps) {
                 TileHead hd = small0;
                 if (r != w) hd = small_head(r);
                 else if (hd.v >= 0) hd.old = get_label<true>(&p.lab_in[hd.v]);
-                bool tied, chg;
-                const int d = small_tile<true>(p, tiles[w].small, hd, changes, tied, chg);
-                add_piece(sums, piece_of(hd.v), d);
+                bool chg;
+                const int d = small_tile<true>(p, tiles[w].small, hd, changes, chg);
+                add_runs(sums, piece_of(hd.v), d);
                 counted += (unsigned)d;
             }
             if (BATCH) {
@@ -386,14 +367,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                     const int64_t v = vb + (w * kPer + u) * 32 + lane;
                     x[u] = FusedVertex{};
                     if (v < v1) {
-                        x[u].d_ = p.dcnt[v];
-                        x[u].kw_ = p.sm_kw[v];
-                        x[u].c0_ = p.sm_c0[v];
-                        x[u].c1_ = p.sm_c1[v];
-                        x[u].r_ = p.sm_r[v];
+                        x[u].d = p.dcnt[v];
+                        x[u].kw = p.sm_kw[v];
+                        x[u].c0 = p.sm_c0[v];
+                        x[u].c1 = p.sm_c1[v];
+                        x[u].r = p.sm_r[v];
                         x[u].old = get_label<true>(&p.lab_in[v]);
-                        x[u].o0_ = __ldg(&p.off[v]);
-                        x[u].o1 = __ldg(&p.off[v + 1]);
+                        x[u].o0 = __ldg(&p.off[v]);
                         if (BATCH) {
                             x[u].now = get_label<true>(&p.lab_out[v]);
                             x[u].g = __ldg(&p.gid[v]);
@@ -446,7 +426,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 int wtotal = 0;
 #pragma unroll
                 for (int u = 0; u < kPer; ++u) {
-                    incl[u] = x[u].d_;
+                    incl[u] = x[u].d;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
                         const int y = __shfl_up_sync(kFull, incl[u], o);
@@ -473,7 +453,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                     for (int u = 0; u < kPer; ++u) {
                         const int64_t v = vb + (w * kPer + u) * 32 + lane;
                         const bool starts = v < v1 && v > v0 && x[u].g != x[u].gprev;
-                        s0[u] = starts ? before + incl[u] - x[u].d_ : LLONG_MIN;
+                        s0[u] = starts ? before + incl[u] - x[u].d : LLONG_MIN;
 #pragma unroll
                         for (int o = 1; o < 32; o <<= 1) {
                             const long long y = __shfl_up_sync(kFull, s0[u], o);
@@ -495,8 +475,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
 #pragma unroll
                 for (int u = 0; u < kPer; ++u) {
                     const int64_t v = vb + (w * kPer + u) * 32 + lane;
-                    const bool tied = x[u].d_ > 0 && (x[u].kw_ & 0xFFFF) > 1;
-                    long long at = before + incl[u] - x[u].d_, N = runs_first;
+                    const bool tied = x[u].d > 0 && (x[u].kw & 0xFFFF) > 1;
+                    long long at = before + incl[u] - x[u].d, N = runs_first;
                     bool is_last = v == p.last_v, run = true;
                     if (BATCH && v < v1) {
                         const int j = x[u].g - gf;
@@ -512,7 +492,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                     int32_t nl = x[u].now;
                     bool queued = false;
                     if (tied) {
-                        if (x[u].o1 - x[u].o0_ > kSmallMax) {
+                        if (x[u].kw >= 0) {
                             const int q = atomicAdd(&qn, 1);
                             R.qv[q] = (int)v;
                             R.qa[q] = at;
@@ -522,7 +502,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                             }
                             queued = true;
                         } else {
-                            nl = resolve_small(p, RunScope{at, N, is_last}, x[u]);
+                            int64_t from = -1;
+                            nl = resolve_small(p, RunScope{at, N, is_last}, x[u].kw, x[u].d, x[u].c0, x[u].c1, x[u].r,
+                                               x[u].o0, from);
+                            if (from >= 0) nl = p.run_lab[from];
                             if (run) p.lab_out[v] = nl;
                             count_change(changes, nl, x[u].old);
                         }

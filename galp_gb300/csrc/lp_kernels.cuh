@@ -63,8 +63,8 @@ struct Ctl {
     int max_iter;               // iterations requested
     int pad1;
     unsigned long long counts[64];  // changes per iteration
-    int tied_small;             // tied vertices listed by the count kernels (per scope)
-    int tied_mid;
+    int tied_mid;               // tied vertices above 32 neighbours (per scope)
+    int pad2;
     int changed_n;              // vertices whose label changed (frontier mode)
     int frontier_off;           // frontier mode: this iteration recounts every vertex
 };
@@ -1073,48 +1073,6 @@ __global__ void __launch_bounds__(kTB) big_stats_kernel(IterArgs p)
     }
 }
 
-// One warp per big vertex: fold its partitions' summaries; when every distinct label is
-// a candidate the ranks are 0 and d - 1.
-__global__ void big_combine_kernel(IterArgs p)
-{
-    if (!ctl_active(p.ctl)) return;
-    const int lane = threadIdx.x & 31;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < p.nbig; i += nw) {
-        const int bi = p.b0 + i;
-        int W = 0, k = 0, mn = INT_MAX, mx = -1;
-        for (int c = p.hub_p0[bi] + lane; c < p.hub_p0[bi + 1]; c += 32) {
-            const int4 o = p.psum[c];
-            if (o.x > W) {
-                W = o.x;
-                k = o.y;
-                mn = o.z;
-                mx = o.w;
-            } else if (o.x == W) {
-                k += o.y;
-                mn = min(mn, o.z);
-                mx = max(mx, o.w);
-            }
-        }
-        const int Ww = __reduce_max_sync(kFull, W);
-        const bool top = W == Ww;
-        k = __reduce_add_sync(kFull, top ? k : 0);
-        mn = __reduce_min_sync(kFull, top ? mn : INT_MAX);
-        mx = __reduce_max_sync(kFull, top ? mx : -1);
-        if (lane == 0) {
-            BigStat &st = p.bstat[bi];
-            st.W = Ww;
-            st.k = k;
-            st.cmin = mn;
-            st.cmax = mx;
-            if (k == st.d) {
-                st.rmin = 0;
-                st.rmax = st.d - 1;
-            }
-        }
-    }
-}
-
 // One warp per big vertex: resolve its winner (its run base is known now), write the
 // label and count the change.
 __global__ void __launch_bounds__(32) big_resolve_kernel(IterArgs p)
@@ -1147,6 +1105,7 @@ __global__ void __launch_bounds__(32) big_resolve_kernel(IterArgs p)
             label = (r == st.rmin) ? st.cmin : (r == st.rmax) ? st.cmax : (int32_t)q.select(r);
         }
     }
+    __syncwarp();  // every lane has read the statistics
     if (lane == 0) {
         const int32_t old = p.lab_in[v];
         p.lab_out[v] = label;
@@ -1154,29 +1113,14 @@ __global__ void __launch_bounds__(32) big_resolve_kernel(IterArgs p)
             atomicAdd(&p.ctl->changes, 1ull);
             if (p.changed) p.changed[atomicAdd(&p.ctl->changed_n, 1)] = v;
         }
-    }
-}
-
-// Reset the per-big-vertex statistics for the next iteration.
-__global__ void big_reset_kernel(IterArgs p)
-{
-    if (!ctl_active(p.ctl)) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.nbig; i += gridDim.x * blockDim.x) {
-        BigStat &b = p.bstat[p.b0 + i];
-        b.d = 0;
-        b.W = 0;
-        b.k = 0;
-        b.cmin = INT_MAX;
-        b.cmax = -1;
-        b.rmin = 0;
-        b.rmax = 0;
+        st = BigStat{0, 0, 0, INT_MAX, -1, 0, 0, 0};  // for the next iteration
     }
 }
 
 // End of an iteration: record the change count, apply the early exit
 // (DPPBase::run, dpp.cuh:83-90: break once count <= n * 1e-5) and reset the
 // per-launch counters.
-__global__ void finalize_kernel(Ctl *ctl)
+__device__ __forceinline__ void finalize_iteration(Ctl *ctl)  // one thread
 {
     if (ctl->active) {
         const unsigned long long c = ctl->changes;
@@ -1187,6 +1131,8 @@ __global__ void finalize_kernel(Ctl *ctl)
     ctl->changes = 0;
     ctl->ticket = 0;
 }
+
+__global__ void finalize_kernel(Ctl *ctl) { finalize_iteration(ctl); }
 
 __global__ void init_labels_kernel(int32_t *lab, int64_t n)
 {

@@ -12,13 +12,15 @@
 //           Each vertex gets its distinct-label count d; a vertex with a unique
 //           most-frequent label is final and written at once.  A tied vertex leaves a
 //           summary (smallest/largest candidate, their ranks, #candidates, max count)
-//           and its (label, count) runs in a spill area at its own CSR positions,
-//           and joins a list of tied vertices.
-//   scan    exclusive scan of d over the scope's vertices: each vertex's run base,
-//           the position of its first run in the reference's run array
-//           (label_propagation/src/dpp/kernel.cuh:66-82 scatter_indexes).
-//   resolve each tied vertex picks its winner by the reference's positional tie rule
-//           (resolve_rank, lp_resolve.h) from its summary, or from its spilled runs.
+//           and its (label, count) runs in a spill area at its own CSR positions.
+//           Its d joins the sum of its block of vertices.
+//   scan    exclusive scan of those sums (the run base of a vertex is the position of its
+//           first run in the reference's run array,
+//           label_propagation/src/dpp/kernel.cuh:66-82 scatter_indexes).
+//   resolve goes over the vertices in order with their run bases: each tied vertex picks
+//           its winner by the reference's positional tie rule (resolve_rank, lp_resolve.h)
+//           from its summary, or from its spilled runs; those above 32 neighbours in a
+//           kernel of their own, one warp each.
 //
 // Spill layout (indexed by CSR position relative to the scope's first entry):
 //   run_lab[e0 + r] label, run_cnt[e0 + r] count of the vertex's r-th run; small vertices
@@ -37,7 +39,7 @@ namespace galp {
 
 constexpr int kMidSMax = 256;        // mid bucket: 33..256 neighbours
 constexpr int kMidWarps = 8;         // warps (vertices) per CTA of count_mid_sort_kernel
-constexpr int kScanBlock = 4096;     // vertices per scan block (256 threads x 16)
+constexpr int kRunBlock = 1024;      // vertices per sum of distinct counts, and per resolve block
 constexpr int kLargeMax = 2048;      // large bucket: 257..2048; above 1024 one 256-thread CTA each
 constexpr int kXlMax = 12288;        // xl bucket: 2049..12288, one CTA each (512 or 1024 threads)
 constexpr int kXlSlots = 2 * kXlMax; // 192 KB of shared-memory table (64-bit slots)
@@ -61,19 +63,20 @@ struct PipeArgs {
     int32_t nmid_s, nmid_l, nmid_x;
     // per-vertex state (global vertex index)
     int32_t *dcnt;          // distinct labels
-    int64_t *runbase;       // run base relative to the scope
+    int64_t *runbase;       // run base (in its scope or graph) of hubs and of listed tied vertices
     int32_t *sm_c0, *sm_c1; // smallest / largest candidate label
-    int32_t *sm_kw;         // candidates | max count << 16 (| kSpillSorted)
+    int32_t *sm_kw;         // candidates | max count << 16 (| kSmallVertex or kSpillSorted)
     int32_t *sm_r;          // rank of smallest | rank of largest << 16
     // spill, indexed by CSR position - nbr_shift
     int32_t *run_lab;
     uint16_t *run_cnt;
-    // tied lists
-    int32_t *tied_small;
-    int32_t *tied_mid;
+    int32_t *tied_mid;      // tied vertices above 32 neighbours (listed by resolve_kernel)
     // scan
     int64_t v0, v1;         // scope vertices
-    int64_t *bsum;          // per scan block
+    // distinct counts summed per block of kRunBlock vertices (batches: per piece of a block that
+    // lies in one graph, see run_piece), zero between iterations; and their exclusive scan
+    long long *sums;
+    long long *run_at;
     int32_t last_v;
     // frontier mode (null = every vertex is recounted and no changes are recorded)
     const uint8_t *dirty;   // 1 = a neighbour's label changed in the previous iteration
@@ -82,7 +85,9 @@ struct PipeArgs {
     // batched mode (null g_v0 = one graph): graph g owns vertices [g_v0[g], g_v0[g+1]), its
     // own run positions (g_base[g] = run base of its first vertex), labels and last vertex
     const int64_t *g_v0;
-    const int64_t *g_base;
+    int64_t *g_base;
+    const int32_t *g_active;          // 0: the graph has ended and keeps its labels
+    unsigned long long *g_changes;    // labels changed per graph in this iteration
     const int32_t *g_last;
     const int32_t *gid;     // graph of every vertex
     int32_t ngraphs;
@@ -93,17 +98,7 @@ struct PipeArgs {
     int32_t gstart;         // first mid-list position counted by lane groups (mid_sort: above 256)
 };
 
-// Graph of vertex v in batched mode: the largest g with g_v0[g] <= v.
-__device__ __forceinline__ int find_graph(const int64_t *g_v0, int ngraphs, int64_t v)
-{
-    int lo = 0, hi = ngraphs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&g_v0[mid]) <= v) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
+constexpr int kSmallVertex = (int)0x80000000u;  // in sm_kw: at most 32 neighbours
 
 // Run position scope of a vertex: its run base a, the scope's run count N, and whether it
 // is the scope's last run-owning vertex (the whole graph, or its graph in batched mode).
@@ -112,12 +107,13 @@ struct RunScope {
     bool is_last;
 };
 
-__device__ __forceinline__ RunScope run_scope(const PipeArgs &p, int v)
+// of vertex v, whose run base is a in the scope
+__device__ __forceinline__ RunScope run_scope(const PipeArgs &p, int v, long long a)
 {
-    if (!p.g_v0) return RunScope{p.runbase[v], p.ctl->N, v == p.last_v};
+    if (!p.g_v0) return RunScope{a, p.ctl->N, v == p.last_v};
     const int g = __ldg(&p.gid[v]);
     const long long base = p.g_base[g];
-    return RunScope{p.runbase[v] - base, p.g_base[g + 1] - base, v == p.g_last[g]};
+    return RunScope{a - base, p.g_base[g + 1] - base, v == p.g_last[g]};
 }
 
 __device__ __forceinline__ void count_change(unsigned long long &changes, int32_t nl, int32_t old)
@@ -171,6 +167,29 @@ __device__ __forceinline__ void flush_changes(unsigned long long changes, Ctl *c
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(&ctl->changes, c);
 }
 
+// Sum that vertex v's distinct count belongs to.  Blocks and graphs cut the vertices into
+// pieces; block + graph numbers them in vertex order (with gaps, whose sums stay 0).
+__device__ __forceinline__ int run_piece(const PipeArgs &p, int v)
+{
+    return (int)((v - p.v0) / kRunBlock) + (p.g_v0 ? __ldg(&p.gid[v]) : 0);
+}
+
+// Add a warp's distinct counts d (0 in lanes without one) to their sums.
+__device__ __forceinline__ void add_runs(long long *sums, int piece, int d)
+{
+    const int c0 = __reduce_max_sync(kFull, d ? piece : 0);
+    if (__all_sync(kFull, !d || piece == c0)) {
+        const int all = __reduce_add_sync(kFull, d);
+        if ((threadIdx.x & 31) == 0 && all) atomicAdd((unsigned long long *)&sums[c0], (unsigned long long)all);
+    } else if (d) {
+        atomicAdd((unsigned long long *)&sums[piece], (unsigned long long)d);
+    }
+}
+__device__ __forceinline__ void add_runs(const PipeArgs &p, int v, int d)  // one thread
+{
+    atomicAdd((unsigned long long *)&p.sums[run_piece(p, v)], (unsigned long long)d);
+}
+
 // warp-aggregated append of the lanes with `pred` to list[ctr++]
 __device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t *list, int *ctr)
 {
@@ -184,11 +203,9 @@ __device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t *l
 }
 
 // Warp-private shared-memory buffer in front of a shared append-only list (the tied
-// lists): a warp appends with one ballot, and the buffer reaches the list with one global
-// atomic per kWarpBuf entries instead of one per append.  In the tie-heavy iterations
-// nearly every pack and vertex appends, and atomics on the one list counter serialise in L2.
+// vertices above 32 neighbours): a warp appends with one ballot, and the buffer reaches the
+// list with one global atomic per kWarpBuf entries instead of one per append.
 constexpr int kWarpBuf = 64;
-constexpr int kCtaBuf = 16;
 struct WarpBuf {
     int32_t *buf;  // kWarpBuf entries of this warp's shared memory
     int n = 0;     // warp-uniform fill
@@ -225,7 +242,7 @@ __device__ __forceinline__ void warp_note_changes(const PipeArgs &p, bool change
 // and move to the vertex lanes, which write the vertex state (all lanes call this).
 __device__ __forceinline__ void finish_small_pack(const PipeArgs &p, bool vl, int v, int deg, int pos, int d, int k,
                                                   int W, int cmin, int cmax, int rmin, int rmax,
-                                                  unsigned long long &changes, WarpBuf &tb)
+                                                  unsigned long long &changes)
 {
     const int lane = threadIdx.x & 31;
     // results live at each vertex's first slot lane; bring them to the vertex lanes
@@ -243,7 +260,7 @@ __device__ __forceinline__ void finish_small_pack(const PipeArgs &p, bool vl, in
     if (vl) {
         p.dcnt[v] = deg > 0 ? d_v : 0;
         const int32_t old = __ldg(&p.lab_in[v]);
-        if (deg > 0) p.sm_kw[v] = k_v | (W_v << 16);
+        if (deg > 0) p.sm_kw[v] = k_v | (W_v << 16) | kSmallVertex;
         if (!tied) {
             const int32_t nl = deg > 0 ? c0_v : old;
             p.lab_out[v] = nl;
@@ -255,7 +272,7 @@ __device__ __forceinline__ void finish_small_pack(const PipeArgs &p, bool vl, in
             p.sm_r[v] = r0_v | (r1_v << 16);
         }
     }
-    tb.append(tied, v, p.tied_small, &p.ctl->tied_small);
+    add_runs(p.sums, vl && deg > 0 ? run_piece(p, v) : 0, vl && deg > 0 ? d_v : 0);
     warp_note_changes(p, chg, v);
 }
 
@@ -264,14 +281,12 @@ __device__ __forceinline__ void finish_small_pack(const PipeArgs &p, bool vl, in
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 6) count_small_kernel(PipeArgs p)
 {
-    __shared__ int32_t tbuf[8][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     unsigned long long changes = 0;
-    WarpBuf tb{tbuf[threadIdx.x >> 5]};
     for (int pk = gw; pk < p.npacks; pk += nw) {
         const int v0 = p.pack_v0[pk], nv = p.pack_nv[pk];
         // vertex lanes: offsets, degrees, slot positions
@@ -283,7 +298,7 @@ __global__ void __launch_bounds__(256, 6) count_small_kernel(PipeArgs p)
             bool tied = false;
             if (vl && (__ldg(&p.off[v + 1]) > __ldg(&p.off[v]))) tied = (p.sm_kw[v] & 0xFFFF) > 1;
             if (vl && !tied) p.lab_out[v] = __ldg(&p.lab_in[v]);
-            tb.append(tied, v, p.tied_small, &p.ctl->tied_small);
+            add_runs(p.sums, vl ? run_piece(p, v) : 0, vl ? p.dcnt[v] : 0);
             continue;
         }
         // The pack's CSR entries are contiguous: slot lane i holds entry obase + i.  Vertex
@@ -341,7 +356,7 @@ __global__ void __launch_bounds__(256, 6) count_small_kernel(PipeArgs p)
                 p.run_lab[e] = slab;
                 p.run_cnt[e] = (uint16_t)cnt;
             }
-            finish_small_pack(p, vl, v, deg, pos, d, k, W, cmin, cmax, rmin, rmax, changes, tb);
+            finish_small_pack(p, vl, v, deg, pos, d, k, W, cmin, cmax, rmin, rmax, changes);
             continue;
         }
         const unsigned eq = __match_any_sync(kFull, valid ? (uint32_t)lab : (0x80000000u | (uint32_t)lane)) & vm;
@@ -420,9 +435,8 @@ __global__ void __launch_bounds__(256, 6) count_small_kernel(PipeArgs p)
                 }
             }
         }
-        finish_small_pack(p, vl, v, deg, pos, d, k, W, cmin, cmax, rmin, rmax, changes, tb);
+        finish_small_pack(p, vl, v, deg, pos, d, k, W, cmin, cmax, rmin, rmax, changes);
     }
-    tb.flush(p.tied_small, &p.ctl->tied_small);
     flush_changes(changes, p.ctl);
 }
 
@@ -572,10 +586,9 @@ __device__ __forceinline__ void t64_insert_row(unsigned long long *tab, uint32_t
     }
 }
 
-// Finish a counted vertex: per-vertex state, and its label unless it is tied.  One
-// thread; returns whether the vertex is tied (the caller appends it to the tied list).
+// Finish a counted vertex: per-vertex state, and its label unless it is tied.  One thread.
 constexpr int kSpillSorted = 1 << 30;  // in sm_kw: the vertex's spilled runs are in label order
-__device__ __forceinline__ bool finish_counted(const PipeArgs &p, int v, const Sum5 &s, int rmin, int rmax,
+__device__ __forceinline__ void finish_counted(const PipeArgs &p, int v, const Sum5 &s, int rmin, int rmax,
                                                unsigned long long &changes, int32_t old, int flags = 0)
 {
     p.dcnt[v] = s.d;
@@ -584,47 +597,18 @@ __device__ __forceinline__ bool finish_counted(const PipeArgs &p, int v, const S
         p.lab_out[v] = s.mn;
         count_change(changes, s.mn, old);
         note_change(p, v, s.mn, old);
-        return false;
+        return;
     }
     p.sm_c0[v] = s.mn;
     p.sm_c1[v] = s.mx;
     p.sm_r[v] = rmin | (rmax << 16);
-    return true;
-}
-
-__device__ __forceinline__ bool finish_counted(const PipeArgs &p, int v, const Sum5 &s, int rmin, int rmax,
-                                               unsigned long long &changes)
-{
-    return finish_counted(p, v, s, rmin, rmax, changes, __ldg(&p.lab_in[v]));
 }
 
 // Frontier: a clean vertex keeps its counts; it is re-resolved if tied, else keeps its
-// label.  One thread; returns whether the vertex is tied.
-__device__ __forceinline__ bool carry_clean(const PipeArgs &p, int v)
+// label.  One thread.
+__device__ __forceinline__ void carry_clean(const PipeArgs &p, int v)
 {
-    if ((p.sm_kw[v] & 0xFFFF) > 1) return true;
-    p.lab_out[v] = __ldg(&p.lab_in[v]);
-    return false;
-}
-
-// One thread's buffer of tied vertices in shared memory (thread 0 finishes every vertex of
-// a CTA counting kernel): one list reservation per kCtaBuf vertices.  Buffer and fill
-// live in shared memory, so the CTA's other threads carry no registers for it; 16 entries
-// keep two 96 KB-table CTAs inside the 196 KB shared-memory carve-out (more would leave
-// the label gathers almost no L1).
-__device__ __forceinline__ void tbuf_flush(int32_t *buf, int *n, int32_t *list, int *ctr)
-{
-    const int c = *n;
-    if (!c) return;
-    const int base = atomicAdd(ctr, c);
-    for (int i = 0; i < c; ++i) list[base + i] = buf[i];
-    *n = 0;
-}
-
-__device__ __forceinline__ void tbuf_append(int32_t *buf, int *n, int32_t value, int32_t *list, int *ctr)
-{
-    if (*n == kCtaBuf) tbuf_flush(buf, n, list, ctr);
-    buf[(*n)++] = value;
+    if ((p.sm_kw[v] & 0xFFFF) <= 1) p.lab_out[v] = __ldg(&p.lab_in[v]);
 }
 
 // ----- sorting networks in registers -----
@@ -847,10 +831,10 @@ __device__ __forceinline__ void tile_head(const PipeArgs &p, TileHead &h, int v,
 }
 
 // Count the warp's 32 small vertices (one per lane), with the tile buffer B.  Writes their state
-// and the labels of untied ones; returns the lane's distinct count.
+// and the labels of untied ones (chg: it changed); returns the lane's distinct count.
 template <bool LIVE>
 __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const TileHead &hd,
-                                          unsigned long long &changes, bool &tied, bool &chg)
+                                          unsigned long long &changes, bool &chg)
 {
     const int lane = threadIdx.x & 31;
     const int v = hd.v;
@@ -883,25 +867,23 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
         ++W;
     }
     const int k = __popc(m);
-    tied = chg = false;
+    chg = false;
     if (v >= 0) {
         if (!hd.dirty) {
             // no label around the vertex changed: its counts carry over
-            tied = hd.deg > 0 && (p.sm_kw[v] & 0xFFFF) > 1;
-            if (!tied) p.lab_out[v] = hd.old;
+            if (hd.deg == 0 || (p.sm_kw[v] & 0xFFFF) <= 1) p.lab_out[v] = hd.old;
         } else if (deg == 0) {
             p.dcnt[v] = 0;
             p.lab_out[v] = hd.old;
         } else {
             p.dcnt[v] = __popc(h);
-            p.sm_kw[v] = k | (W << 16);
+            p.sm_kw[v] = k | (W << 16) | kSmallVertex;
             if (k == 1) {
                 const int32_t nl = row[__ffs(m) - 1];
                 p.lab_out[v] = nl;
                 count_change(changes, nl, hd.old);
                 chg = nl != hd.old;
             } else {
-                tied = true;
                 const int lo = __ffs(m) - 1, hi = 31 - __clz(m);
                 p.sm_c0[v] = k == 2 ? row[lo] : (int32_t)h;
                 p.sm_c1[v] = k == 2 ? row[hi] : (int32_t)m;
@@ -933,11 +915,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
 {
     constexpr int NW = kSmallThreads / 32;
     __shared__ __align__(16) TileBuf stile[NW];
-    __shared__ int32_t tbuf[NW][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
     // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
     // window in turn, so that none has only the window's highest degrees
@@ -955,12 +935,12 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
     for (; base < p.nsmall; base += stride) {
         const TileHead hd = nxt;
         nxt = ahead(base + stride);
-        bool tied, chg;
-        small_tile<false>(p, stile[w], hd, changes, tied, chg);
-        tb.append(tied, hd.v, p.tied_small, &p.ctl->tied_small);
+        bool chg;
+        int d = small_tile<false>(p, stile[w], hd, changes, chg);
+        if (!hd.dirty) d = p.dcnt[hd.v];
+        add_runs(p.sums, d ? run_piece(p, hd.v) : 0, d);
         warp_note_changes(p, chg, hd.v);
     }
-    tb.flush(p.tied_small, &p.ctl->tied_small);
     flush_changes(changes, p.ctl);
 }
 
@@ -1167,11 +1147,10 @@ __device__ __forceinline__ TileHead group_head(const PipeArgs &p, const GroupTil
 }
 
 // Count the warp's tile of vertices (one per group of lanes).  Writes their state and the
-// labels of untied ones; returns the group's distinct count.  tied: in the groups' first
-// lanes.
+// labels of untied ones; returns the group's distinct count.
 template <bool LIVE>
 __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const TileHead &hd,
-                                          unsigned long long &changes, bool &tied)
+                                          unsigned long long &changes)
 {
     const int lane = threadIdx.x & 31;
     int32_t *rows = B.rows;
@@ -1262,10 +1241,9 @@ __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const 
     sm.mx = __shfl_sync(kFull, rows[lane * stride + hi], l1);
     const int rmin = __shfl_sync(kFull, rank0 + __popc(h & ((1u << lo) - 1u)), l0);
     const int rmax = __shfl_sync(kFull, rank0 + __popc(h & ((1u << hi) - 1u)), l1);
-    tied = false;
     if (leader && v >= 0) {
-        if (!hd.dirty) tied = carry_clean(p, v);
-        else tied = finish_counted(p, v, sm, rmin, rmax, changes, hd.old, kSpillSorted);
+        if (!hd.dirty) carry_clean(p, v);
+        else finish_counted(p, v, sm, rmin, rmax, changes, hd.old, kSpillSorted);
     }
     unsigned spill = __ballot_sync(kFull, leader && deg > 0 && k > 2);
     if (spill) {
@@ -1295,12 +1273,10 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) count_group_kerne
 {
     constexpr int NW = kGroupThreads / 32;
     __shared__ __align__(16) GroupBuf stile[NW];
-    __shared__ int32_t tbuf[NW][kWarpBuf];
     __shared__ GroupTiles T;
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int w = threadIdx.x >> 5;
-    WarpBuf tb{tbuf[w]};
     unsigned long long changes = 0;
     if (threadIdx.x == 0) T.set(p, p.disp->pos1);
     __syncthreads();
@@ -1310,11 +1286,10 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks) count_group_kerne
     for (; t < T.count(); t += nw) {
         const TileHead hd = nxt;
         nxt = group_head<false>(p, T, t + nw, fr);
-        bool tied;
-        group_tile<false>(p, stile[w], hd, changes, tied);
-        tb.append(tied, hd.v, p.tied_mid, &p.ctl->tied_mid);
+        int d = group_tile<false>(p, stile[w], hd, changes);
+        if (!hd.dirty) d = p.dcnt[hd.v];
+        if ((threadIdx.x & ((1 << hd.g) - 1)) == 0 && hd.v >= 0) add_runs(p, hd.v, d);
     }
-    tb.flush(p.tied_mid, &p.ctl->tied_mid);
     flush_changes(changes, p.ctl);
 }
 
@@ -1359,19 +1334,20 @@ __device__ __forceinline__ void warp_bitonic256(uint32_t (&a)[8], int lane)
 
 __global__ void __launch_bounds__(32 * kMidWarps) count_mid_sort_kernel(PipeArgs p)
 {
-    __shared__ int32_t tbuf[kMidWarps][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int gw = blockIdx.x * kMidWarps + w;
     const int nw = gridDim.x * kMidWarps;
     unsigned long long changes = 0;
-    WarpBuf tb{tbuf[w]};
     const int nwarp_v = p.gstart;  // the degree-sorted mid list's prefix of up to 256 neighbours
     for (int i = gw; i < nwarp_v; i += nw) {
         const int v = p.mid_v[i];
         if (fr && !p.dirty[v]) {
-            tb.append(lane == 0 && carry_clean(p, v), v, p.tied_mid, &p.ctl->tied_mid);
+            if (lane == 0) {
+                carry_clean(p, v);
+                add_runs(p, v, p.dcnt[v]);
+            }
             continue;
         }
         const int64_t o0 = __ldg(&p.off[v]);
@@ -1457,11 +1433,12 @@ __global__ void __launch_bounds__(32 * kMidWarps) count_mid_sort_kernel(PipeArgs
                     }
             }
         }
-        const bool tied = lane == 0 && finish_counted(p, v, sm, rmin, rmax, changes);
-        tb.append(tied, v, p.tied_mid, &p.ctl->tied_mid);
+        if (lane == 0) {
+            finish_counted(p, v, sm, rmin, rmax, changes, __ldg(&p.lab_in[v]));
+            add_runs(p, v, sm.d);
+        }
         __syncwarp();
     }
-    tb.flush(p.tied_mid, &p.ctl->tied_mid);
     flush_changes(changes, p.ctl);
 }
 
@@ -1575,10 +1552,7 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : THREADS >= 512 
     __shared__ int sctr;
     __shared__ __align__(8) unsigned long long stage_bar;
     __shared__ int stage_ok;
-    __shared__ int32_t ctbuf[kCtaBuf];  // thread 0's tied vertices
-    __shared__ int ctn;
     if (!ctl_active(p.ctl)) return;
-    if (threadIdx.x == 0) ctn = 0;  // ordered before thread 0's own uses
     // ranges of the degree-sorted mid list: 1 [pos_a, pos2), 2 [pos2, pos_b), 3 [pos_b, end)
     const DispatchState &ds = *p.disp;
     const int first = which == 1 ? ds.pos_a : which == 2 ? ds.pos2 : ds.pos_b;
@@ -1635,7 +1609,10 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : THREADS >= 512 
         for (int u = 0; u < PER; ++u) nb0[u] = nbn[u];
         nxt = cta_head(p, first, i + gridDim.x, count, fr);
         if (!h.dirty) {
-            if (tid == 0 && carry_clean(p, v)) tbuf_append(ctbuf, &ctn, v, p.tied_mid, &p.ctl->tied_mid);
+            if (tid == 0) {
+                carry_clean(p, v);
+                add_runs(p, v, h.dcnt);
+            }
             ids_ahead(nbn, nxt);
             continue;
         }
@@ -1707,11 +1684,12 @@ __global__ void __launch_bounds__(THREADS, THREADS >= 1024 ? 1 : THREADS >= 512 
                           p.run_cnt + (o0 - p.nbr_shift), &sctr);
             }
         }
-        if (tid == 0 && finish_counted(p, v, s, rmin, rmax, changes, h.old))
-            tbuf_append(ctbuf, &ctn, v, p.tied_mid, &p.ctl->tied_mid);
+        if (tid == 0) {
+            finish_counted(p, v, s, rmin, rmax, changes, h.old);
+            add_runs(p, v, s.d);
+        }
         __syncthreads();
     }
-    if (tid == 0) tbuf_flush(ctbuf, &ctn, p.tied_mid, &p.ctl->tied_mid);
     // a copy that a wait gave up on still lands in this CTA's shared memory: wait for it
     // (bounded) before the CTA exits
     if (staged && lost_parity < 2) (void)mbar_wait(&stage_bar, lost_parity);
@@ -1831,101 +1809,110 @@ __global__ void __launch_bounds__(kTB) gather_probe_kernel(const int32_t *nbr, i
     if ((threadIdx.x & 31) == 0 && x) atomicXor(acc, (unsigned long long)x);
 }
 
-__global__ void big_dcnt_kernel(IterArgs a, int32_t *dcnt)
+// One warp per big vertex: fold its partitions' summaries; when every distinct label is
+// a candidate the ranks are 0 and d - 1.  Its distinct count joins the others.
+__global__ void big_combine_kernel(IterArgs p, PipeArgs q)
 {
-    if (!ctl_active(a.ctl)) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.nbig; i += gridDim.x * blockDim.x)
-        dcnt[a.big_v[a.b0 + i]] = a.bstat[a.b0 + i].d;
+    if (!ctl_active(p.ctl)) return;
+    const int lane = threadIdx.x & 31;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < p.nbig; i += nw) {
+        const int bi = p.b0 + i;
+        int W = 0, k = 0, mn = INT_MAX, mx = -1;
+        for (int c = p.hub_p0[bi] + lane; c < p.hub_p0[bi + 1]; c += 32) {
+            const int4 o = p.psum[c];
+            if (o.x > W) {
+                W = o.x;
+                k = o.y;
+                mn = o.z;
+                mx = o.w;
+            } else if (o.x == W) {
+                k += o.y;
+                mn = min(mn, o.z);
+                mx = max(mx, o.w);
+            }
+        }
+        const int Ww = __reduce_max_sync(kFull, W);
+        const bool top = W == Ww;
+        k = __reduce_add_sync(kFull, top ? k : 0);
+        mn = __reduce_min_sync(kFull, top ? mn : INT_MAX);
+        mx = __reduce_max_sync(kFull, top ? mx : -1);
+        if (lane == 0) {
+            BigStat &st = p.bstat[bi];
+            st.W = Ww;
+            st.k = k;
+            st.cmin = mn;
+            st.cmax = mx;
+            if (k == st.d) {
+                st.rmin = 0;
+                st.rmax = st.d - 1;
+            }
+            const int v = p.big_v[bi];
+            q.dcnt[v] = st.d;
+            add_runs(q, v, st.d);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
-// scan of distinct counts -> run bases (reduce, spine, apply)
+// scan of the distinct counts' sums
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kTB) scan_reduce_kernel(PipeArgs p)
-{
-    __shared__ long long ws[kNW];
-    if (!ctl_active(p.ctl)) return;
-    const int64_t b0 = p.v0 + (int64_t)blockIdx.x * kScanBlock;
-    long long s = 0;
-    for (int i = threadIdx.x; i < kScanBlock; i += kTB) {
-        const int64_t v = b0 + i;
-        if (v < p.v1) s += p.dcnt[v];
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        long long t = 0;
-        for (int w = 0; w < kNW; ++w) t += ws[w];
-        p.bsum[blockIdx.x] = t;
-    }
-}
 
-// one CTA: exclusive scan of the block sums in place; total -> ctl->N
-__global__ void __launch_bounds__(kTB) scan_spine_kernel(PipeArgs p, int nblocks)
+// One block: exclusive scan of the sums (which are zero again afterwards), the scope's number of
+// runs, the graphs' run bases, an empty tied list.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(PipeArgs p, int npieces)
 {
-    __shared__ long long ws[kNW];
-    __shared__ long long carry;
+    constexpr int NW = kScanThreads / 32, PER = 8;
+    __shared__ long long ws[NW];
     if (!ctl_active(p.ctl)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nblocks; base += kTB) {
-        const int i = base + threadIdx.x;
-        const long long x = i < nblocks ? p.bsum[i] : 0;
-        long long incl = x;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    long long base = 0;
+    // rounds of kScanThreads * PER sums; a warp takes 32 * PER consecutive ones, row after row
+    for (int i0 = 0; i0 < npieces; i0 += kScanThreads * PER) {
+        long long x[PER], s = 0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const long long o = __shfl_up_sync(kFull, incl, off);
-            if (lane >= off) incl += o;
+        for (int u = 0; u < PER; ++u) {
+            const int i = i0 + (w * PER + u) * 32 + lane;
+            x[u] = i < npieces ? p.sums[i] : 0;
         }
-        if (lane == 31) ws[warp] = incl;
-        __syncthreads();
-        long long wb = 0, tot = 0;
-        for (int w = 0; w < kNW; ++w) {
-            if (w < warp) wb += ws[w];
-            tot += ws[w];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const long long own = x[u];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(kFull, x[u], o);
+                if (lane >= o) x[u] += y;
+            }
+            const long long row = __shfl_sync(kFull, x[u], 31);
+            x[u] += s - own;
+            s += row;
         }
-        const long long c = carry;
-        if (i < nblocks) p.bsum[i] = c + wb + incl - x;
+        if (lane == 0) ws[w] = s;
         __syncthreads();
-        if (threadIdx.x == 0) carry = c + tot;
+        long long before = base, all = ws[lane];
+        for (int i = 0; i < w; ++i) before += ws[i];
+        all = warp_sum_ll(all);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int i = i0 + (w * PER + u) * 32 + lane;
+            if (i < npieces) {
+                p.run_at[i] = before + x[u];
+                p.sums[i] = 0;
+            }
+        }
+        base += all;
         __syncthreads();
     }
-    if (threadIdx.x == 0) p.ctl->N = carry;
-}
-
-__global__ void __launch_bounds__(kTB) scan_apply_kernel(PipeArgs p)
-{
-    __shared__ long long ws[kNW];
-    if (!ctl_active(p.ctl)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int PER = kScanBlock / kTB;
-    const int64_t b0 = p.v0 + (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * PER;
-    int x[PER];
-    long long s = 0;
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-        x[u] = (b0 + u < p.v1) ? p.dcnt[b0 + u] : 0;
-        s += x[u];
+    if (tid == 0) {
+        p.ctl->N = base;
+        p.ctl->tied_mid = 0;
     }
-    long long incl = s;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const long long o = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += o;
-    }
-    if (lane == 31) ws[warp] = incl;
-    __syncthreads();
-    long long wb = 0;
-    for (int w = 0; w < warp; ++w) wb += ws[w];
-    long long run = p.bsum[blockIdx.x] + wb + incl - s;
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-        if (b0 + u < p.v1) p.runbase[b0 + u] = run;
-        run += x[u];
-    }
+    if (p.g_v0)
+        for (int g = tid; g <= p.ngraphs; g += kScanThreads) {
+            const int64_t v = p.g_v0[g];
+            p.g_base[g] = v < p.v1 ? p.run_at[run_piece(p, (int)v)] : base;
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -1956,16 +1943,35 @@ struct SpillRunQuery {
 // the run heads among its sorted labels (at its CSR positions), m the heads of candidates.
 struct SmallMaskQuery {
     uint32_t h, m;
+    int pos = 0;  // head of the candidate that the last query found
     // position of the head of rank x (0 <= x < popc(h))
-    __device__ int at(int x) const { return (int)__fns(h, 0, x + 1); }
-    __device__ int rank(int pos) const { return __popc(h & ((1u << pos) - 1u)); }
-    __device__ int first_ge(int64_t x) const
+    __device__ int at(int x) const
+    {
+        uint32_t b = h;
+        int r = 0;
+#pragma unroll
+        for (int step = 16; step; step >>= 1) {
+            const int c = __popc(b & ((1u << step) - 1u));
+            if (x >= c) {
+                x -= c;
+                r += step;
+                b >>= step;
+            }
+        }
+        return r;
+    }
+    __device__ int rank(int head)
+    {
+        pos = head;
+        return __popc(h & ((1u << head) - 1u));
+    }
+    __device__ int first_ge(int64_t x)
     {
         if (x >= __popc(h)) return -1;
         const uint32_t c = x <= 0 ? m : m & ~((1u << at((int)x)) - 1u);
         return c ? rank(__ffs(c) - 1) : -1;
     }
-    __device__ int last_lt(int64_t y) const
+    __device__ int last_lt(int64_t y)
     {
         if (y <= 0) return -1;
         const uint32_t c = y >= __popc(h) ? m : m & ((1u << at((int)y)) - 1u);
@@ -1974,55 +1980,27 @@ struct SmallMaskQuery {
     __device__ int tile_pick(int64_t) const { return -1; }  // d <= 32 never spans a tile
 };
 
-// State of a small vertex: read where it is needed, or loaded beforehand in one round trip.
-struct SmallStateMem {
-    const PipeArgs &p;
-    int v;
-    __device__ int kw() const { return p.sm_kw[v]; }
-    __device__ int d() const { return p.dcnt[v]; }
-    __device__ int32_t c0() const { return p.sm_c0[v]; }
-    __device__ int32_t c1() const { return p.sm_c1[v]; }
-    __device__ int r() const { return p.sm_r[v]; }
-    __device__ int64_t o0() const { return __ldg(&p.off[v]); }
-};
-
-// New label of a tied small vertex with run scope rs (one thread).
-template <class State>
-__device__ __forceinline__ int32_t resolve_small(const PipeArgs &p, const RunScope &rs, const State &x)
+// New label of a tied small vertex with run scope rs, from its state (one thread); e: its first
+// entry in the spill area.  Where that holds the label, its entry is left in `from`.
+__device__ __forceinline__ int32_t resolve_small(const PipeArgs &p, const RunScope &rs, int kw, int d, int32_t c0,
+                                                 int32_t c1, int rr, int64_t e, int64_t &from)
 {
-    const int kw = x.kw(), d = x.d();
-    const int k = kw & 0xFFFF, W = kw >> 16;
+    const int k = kw & 0xFFFF, W = (kw >> 16) & 0x3FFF;
     if (k > 2 && p.small_sort == 2) {
-        SmallMaskQuery mq{(uint32_t)x.c0(), (uint32_t)x.c1()};
-        const int r = resolve_rank(rs.a, d, rs.N, rs.is_last, mq);
-        return p.run_lab[x.o0() - p.nbr_shift + mq.at(r)];
+        SmallMaskQuery mq{(uint32_t)c0, (uint32_t)c1};
+        (void)resolve_rank(rs.a, d, rs.N, rs.is_last, mq);  // its result is the last query's
+        from = e + mq.pos;
+        return 0;
     }
-    const int rr = x.r();
     const int rmin = rr & 0xFFFF, rmax = rr >> 16;
     SummaryQuery q(k, d, rmin, rmax);
     int r = resolve_rank(rs.a, d, rs.N, rs.is_last, q);
-    if (!q.fail && r == rmin) return x.c0();
-    if (!q.fail && r == rmax) return x.c1();
-    const int64_t e = x.o0() - p.nbr_shift;
+    if (!q.fail && r == rmin) return c0;
+    if (!q.fail && r == rmax) return c1;
     SpillRunQuery sq{p.run_lab + e, p.run_cnt + e, d, W};
     if (q.fail) r = resolve_rank(rs.a, d, rs.N, rs.is_last, sq);
-    return p.run_lab[e + r];
-}
-
-__global__ void __launch_bounds__(kTB) resolve_small_kernel(PipeArgs p)
-{
-    if (!ctl_active(p.ctl)) return;
-    const int nt = *((volatile int *)&p.ctl->tied_small);
-    unsigned long long changes = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += gridDim.x * blockDim.x) {
-        const int v = p.tied_small[i];
-        const int32_t nl = resolve_small(p, run_scope(p, v), SmallStateMem{p, v});
-        const int32_t old = __ldg(&p.lab_in[v]);
-        p.lab_out[v] = nl;
-        count_change(changes, nl, old);
-        note_change(p, v, nl, old);
-    }
-    flush_changes(changes, p.ctl);
+    from = e + r;
+    return 0;
 }
 
 // Unsorted spilled (label, count) entries of a mid/large vertex, one warp.
@@ -2188,6 +2166,157 @@ __device__ __forceinline__ int32_t resolve_mid(const PipeArgs &p, int v, const R
     return (r == rmin) ? p.sm_c0[v] : (r == rmax) ? p.sm_c1[v] : (int32_t)tq.select(r);
 }
 
+// Count a row of changed vertices (one per lane) for their graphs (batches): a warp's rows mostly
+// lie in one graph, whose changes it keeps until the graph is another one.
+struct GraphChanges {
+    int g = -1, n = 0;  // warp-uniform
+    __device__ __forceinline__ void flush(const PipeArgs &p)
+    {
+        if (n && (threadIdx.x & 31) == 0) atomicAdd(&p.g_changes[g], (unsigned long long)n);
+        n = 0;
+    }
+    __device__ __forceinline__ void add(const PipeArgs &p, bool chg, int gv)
+    {
+        const unsigned m = __ballot_sync(kFull, chg);
+        if (!m) return;
+        const int g0 = __shfl_sync(kFull, gv, __ffs(m) - 1);
+        if (__all_sync(kFull, !chg || gv == g0)) {
+            if (g0 != g) flush(p);
+            g = g0;
+            n += __popc(m);
+        } else if (chg) {
+            atomicAdd(&p.g_changes[gv], 1ull);
+        }
+    }
+};
+
+// The scope's vertices in order, with their run bases: ties of at most 32 neighbours are resolved
+// here, larger ones listed with their run base for resolve_mid_kernel, hubs (which have no
+// summary: sm_kw is 0) get their run base.  Batches: a graph that has ended keeps its labels,
+// the others count their changes.
+//
+// One pass where a reduction and a scan over all vertices, tied lists filled by the counting
+// kernels and, for batches, a pass of comparing and committing labels stood before: ten
+// iterations of 1,024 planted partitions (36 M vertices) 12.4 -> 6.5 ms with scan_kernel, and
+// five launches per iteration fewer.  Bound by the latency of its dependent loads (d and kw,
+// then the summary and offset, then the spilled label), which is why the rows' loads of one kind
+// go out together; 2 or 4 blocks per SM were 3 to 20 % slower.
+constexpr int kResolveBlocks = 3;  // resident blocks per SM
+template <bool BATCH>
+__global__ void __launch_bounds__(kTB, kResolveBlocks) resolve_kernel(PipeArgs p)
+{
+    constexpr int PER = kRunBlock / kTB;
+    __shared__ long long ws[kNW];
+    __shared__ int32_t tbuf[kNW][kWarpBuf];
+    if (!ctl_active(p.ctl)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t b0 = p.v0 + (int64_t)blockIdx.x * kRunBlock;
+    const int64_t v0 = b0 + w * (PER * 32) + lane;
+    // the rows' loads of one kind together, so that the chain of dependent loads is paid once
+    int d[PER], kw[PER], g[PER];
+    int32_t old[PER], nl[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int64_t v = v0 + u * 32;
+        const bool in = v < p.v1;
+        d[u] = in ? p.dcnt[v] : 0;
+        kw[u] = in ? p.sm_kw[v] : 1;
+        old[u] = BATCH && in ? __ldg(&p.lab_in[v]) : 0;
+        nl[u] = BATCH && in ? p.lab_out[v] : 0;
+        g[u] = BATCH && in ? __ldg(&p.gid[v]) : 0;
+    }
+    long long at[PER];  // runs of the warp's vertices before the vertex
+    {
+        bool hub = false;  // a row without one has less than 2^31 runs
+#pragma unroll
+        for (int u = 0; u < PER; ++u) hub |= d[u] > kXlMax;
+        const bool wide = !BATCH && __any_sync(kFull, hub);
+        long long s = 0;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            long long row, incl;
+            if (!wide) {
+                int x = d[u];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFull, x, o);
+                    if (lane >= o) x += y;
+                }
+                incl = x;
+                row = __shfl_sync(kFull, x, 31);
+            } else {
+                incl = d[u];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const long long y = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                row = __shfl_sync(kFull, incl, 31);
+            }
+            at[u] = s + incl - d[u];
+            s += row;
+        }
+        if (lane == 0) ws[w] = s;
+    }
+    // small tied vertices (small), larger ones and hubs (rest; k = 0 in hubs)
+    int64_t o0[PER];
+    int32_t c0[PER], c1[PER], rr[PER];
+    bool small[PER], rest[PER], runs[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int64_t v = v0 + u * 32;
+        const int k = kw[u] & 0xFFFF;
+        const bool pick = d[u] > 0 && k != 1;
+        small[u] = pick && kw[u] < 0;
+        rest[u] = pick && kw[u] >= 0;
+        o0[u] = small[u] ? __ldg(&p.off[v]) : 0;
+        c0[u] = small[u] ? p.sm_c0[v] : 0;
+        c1[u] = small[u] ? p.sm_c1[v] : 0;
+        rr[u] = small[u] && (k == 2 || p.small_sort != 2) ? p.sm_r[v] : 0;
+        if (!BATCH) old[u] = small[u] ? __ldg(&p.lab_in[v]) : 0;
+        runs[u] = !BATCH || __ldg(&p.g_active[g[u]]) != 0;
+    }
+    __syncthreads();
+    long long base = p.run_at[run_piece(p, (int)b0)];
+    for (int i = 0; i < w; ++i) base += ws[i];
+    int64_t from[PER];  // spill entry that holds the new label, or -1
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        from[u] = -1;
+        if (small[u]) {
+            const int64_t v = v0 + u * 32;
+            nl[u] = resolve_small(p, run_scope(p, (int)v, base + at[u]), kw[u], d[u], c0[u], c1[u], rr[u],
+                                  o0[u] - p.nbr_shift, from[u]);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u)
+        if (from[u] >= 0) nl[u] = p.run_lab[from[u]];
+    WarpBuf tb{tbuf[w]};
+    GraphChanges gc;
+    unsigned long long changes = 0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int64_t v = v0 + u * 32;
+        const bool listed = rest[u] && (kw[u] & 0xFFFF) != 0;
+        if (rest[u]) p.runbase[v] = base + at[u];
+        if (small[u]) {
+            if (runs[u]) p.lab_out[v] = nl[u];
+            count_change(changes, nl[u], old[u]);
+            note_change(p, (int32_t)v, nl[u], old[u]);
+        }
+        tb.append(listed, (int32_t)v, p.tied_mid, &p.ctl->tied_mid);
+        if (BATCH) {
+            if (v < p.v1 && !listed && !runs[u]) p.lab_out[v] = old[u];
+            gc.add(p, v < p.v1 && !listed && runs[u] && nl[u] != old[u], g[u]);
+        }
+    }
+    tb.flush(p.tied_mid, &p.ctl->tied_mid);
+    if (BATCH) gc.flush(p);
+    flush_changes(changes, p.ctl);
+}
+
+template <bool BATCH>
 __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
 {
     __shared__ int hist[kNW][256];
@@ -2197,12 +2326,19 @@ __global__ void __launch_bounds__(kTB) resolve_mid_kernel(PipeArgs p)
     unsigned long long changes = 0;
     for (int i = blockIdx.x * kNW + w; i < nt; i += gridDim.x * kNW) {
         const int v = p.tied_mid[i];
-        const int32_t nl = resolve_mid(p, v, run_scope(p, v), hist[w]);
+        const int32_t nl = resolve_mid(p, v, run_scope(p, v, p.runbase[v]), hist[w]);
         if (lane == 0) {
             const int32_t old = __ldg(&p.lab_in[v]);
-            p.lab_out[v] = nl;
             count_change(changes, nl, old);
             note_change(p, v, nl, old);
+            if (BATCH) {
+                const int g = __ldg(&p.gid[v]);
+                const bool runs = __ldg(&p.g_active[g]) != 0;
+                p.lab_out[v] = runs ? nl : old;
+                if (runs && nl != old) atomicAdd(&p.g_changes[g], 1ull);
+            } else {
+                p.lab_out[v] = nl;
+            }
         }
     }
     flush_changes(changes, p.ctl);
@@ -2252,28 +2388,42 @@ __global__ void __launch_bounds__(kTB) first_iteration_kernel(PipeArgs p, int64_
     if (!ctl_active(p.ctl)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) p.ctl->N = m;  // one run per CSR entry
     unsigned long long changes = 0;
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t o0 = __ldg(&p.off[v]);
-        const int64_t deg = __ldg(&p.off[v + 1]) - o0;
-        const int32_t old = __ldg(&p.lab_in[v]);
-        int32_t nl = old;
-        if (deg > 0) {
-            AllCandidates q{deg};
-            if (!p.g_v0) {
-                const int r = resolve_rank(o0, deg, m, v == p.last_v, q);
-                nl = __ldg(&p.nbr[o0 + r]);
-            } else {  // graph-local run positions and labels
-                const int g = __ldg(&p.gid[v]);
-                const int64_t vg = p.g_v0[g], e0 = __ldg(&p.off[vg]), e1 = __ldg(&p.off[p.g_v0[g + 1]]);
-                const int r = resolve_rank(o0 - e0, deg, e1 - e0, v == p.g_last[g], q);
-                nl = (int32_t)(__ldg(&p.nbr[o0 + r]) - vg);
+    GraphChanges gc;
+    const int lane = threadIdx.x & 31;
+    for (int64_t vb = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; vb < n;
+         vb += (int64_t)gridDim.x * blockDim.x) {  // warp-uniform
+        const int64_t v = vb + lane;
+        int g = 0;
+        bool chg = false;
+        if (v < n) {
+            const int64_t o0 = __ldg(&p.off[v]);
+            const int64_t deg = __ldg(&p.off[v + 1]) - o0;
+            const int32_t old = __ldg(&p.lab_in[v]);
+            int32_t nl = old;
+            if (deg > 0) {
+                AllCandidates q{deg};
+                if (!p.g_v0) {
+                    const int r = resolve_rank(o0, deg, m, v == p.last_v, q);
+                    nl = __ldg(&p.nbr[o0 + r]);
+                } else {  // graph-local run positions and labels
+                    g = __ldg(&p.gid[v]);
+                    const int64_t vg = p.g_v0[g], e0 = __ldg(&p.off[vg]), e1 = __ldg(&p.off[p.g_v0[g + 1]]);
+                    const int r = resolve_rank(o0 - e0, deg, e1 - e0, v == p.g_last[g], q);
+                    nl = (int32_t)(__ldg(&p.nbr[o0 + r]) - vg);
+                }
+            }
+            p.lab_out[v] = nl;
+            p.dcnt[v] = (int32_t)deg;  // every neighbour label distinct (insert-aggregation hint)
+            count_change(changes, nl, old);
+            note_change(p, (int32_t)v, nl, old);
+            if (p.g_v0) {
+                g = __ldg(&p.gid[v]);
+                chg = nl != old;
             }
         }
-        p.lab_out[v] = nl;
-        p.dcnt[v] = (int32_t)deg;  // every neighbour label distinct (insert-aggregation hint)
-        count_change(changes, nl, old);
-        note_change(p, (int32_t)v, nl, old);
+        if (p.g_v0) gc.add(p, chg, g);
     }
+    if (p.g_v0) gc.flush(p);
     flush_changes(changes, p.ctl);
 }
 
@@ -2419,60 +2569,29 @@ __global__ void __launch_bounds__(kTB) batch_init_labels_kernel(const int64_t *g
     }
 }
 
-// Per-graph run bases after the scan: g_base[g] = run base of graph g's first vertex,
-// g_base[ngraphs] = all runs.
-__global__ void batch_bases_kernel(const int64_t *g_v0, int ngraphs, const int64_t *runbase, int64_t n, const Ctl *ctl,
-                                   int64_t *g_base)
-{
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= ngraphs; g += gridDim.x * blockDim.x) {
-        const int64_t v = g_v0[g];
-        g_base[g] = v < n ? runbase[v] : ctl->N;
-    }
-}
-
-// After an iteration: per graph, the labels that changed and the reference's early exit
-// (count <= n_g * 1e-5, dpp.cuh:88) per graph.  A graph that had already exited keeps its
-// labels (lab_out = lab_in).  One block per graph (grid-stride).
-__global__ void __launch_bounds__(kTB) batch_commit_kernel(const Ctl *ctl, const int64_t *g_v0, int ngraphs,
-                                                           const int32_t *lab_in, int32_t *lab_out, int32_t *g_active,
-                                                           int32_t *g_iters, long long *g_counts, int max_iter, int it,
-                                                           int early_exit)
-{
-    __shared__ unsigned long long part[kTB / 32];
-    if (!ctl_active(ctl)) return;  // every graph exited earlier: the final buffer is settled
-    for (int g = blockIdx.x; g < ngraphs; g += gridDim.x) {
-        const int64_t v0 = g_v0[g], v1 = g_v0[g + 1];
-        if (!g_active[g]) {
-            for (int64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) lab_out[v] = lab_in[v];
-            continue;
-        }
-        unsigned long long c = 0;
-        for (int64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) c += lab_out[v] != lab_in[v];
-        c = __reduce_add_sync(kFull, (unsigned)c);
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long t = 0;
-            for (int w = 0; w < kTB / 32; ++w) t += part[w];
-            if (it < max_iter) g_counts[(int64_t)g * max_iter + it] = (long long)t;
-            g_iters[g] = it + 1;
-            if ((early_exit && (double)t <= (double)(v1 - v0) * 1e-5) || it + 1 >= max_iter) g_active[g] = 0;
-        }
-        __syncthreads();
-    }
-}
-
-// Global bookkeeping after batch_commit: the run goes on while some graph is active.
-__global__ void batch_finalize_kernel(Ctl *ctl, const int32_t *g_active, int ngraphs)
+// After an iteration of a batch: per graph, the labels that changed and the reference's early
+// exit (count <= n_g * 1e-5, dpp.cuh:88); the run goes on while some graph is active.
+// Also the next iteration's dispatch state, where there is one (a.out).
+__global__ void batch_finalize_kernel(Ctl *ctl, const int64_t *g_v0, int32_t *g_active, int32_t *g_iters,
+                                      long long *g_counts, unsigned long long *g_changes, int ngraphs, int max_iter,
+                                      int it, int early_exit, DispatchArgs a)
 {
     __shared__ int any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
-    for (int g = threadIdx.x; g < ngraphs; g += blockDim.x)
-        if (g_active[g]) any = 1;
+    const bool on = ctl_active(ctl);  // else every graph ended earlier: all is settled
+    for (int g = threadIdx.x; on && g < ngraphs; g += blockDim.x) {
+        if (!g_active[g]) continue;
+        const unsigned long long t = g_changes[g];
+        g_changes[g] = 0;
+        if (it < max_iter) g_counts[(int64_t)g * max_iter + it] = (long long)t;
+        g_iters[g] = it + 1;
+        if ((early_exit && (double)t <= (double)(g_v0[g + 1] - g_v0[g]) * 1e-5) || it + 1 >= max_iter) g_active[g] = 0;
+        else any = 1;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (ctl->active) {
+        if (on) {
             const unsigned long long c = ctl->changes;
             if (ctl->iter < 64) ctl->counts[ctl->iter] = c;
             ctl->iter += 1;
@@ -2481,13 +2600,19 @@ __global__ void batch_finalize_kernel(Ctl *ctl, const int32_t *g_active, int ngr
         ctl->changes = 0;
         ctl->ticket = 0;
     }
+    if (a.out) {
+        __syncthreads();
+        dispatch_step(a);
+    }
 }
 
-__global__ void batch_init_kernel(int32_t *g_active, int32_t *g_iters, int ngraphs, int active)
+__global__ void batch_init_kernel(int32_t *g_active, int32_t *g_iters, unsigned long long *g_changes, int ngraphs,
+                                  int active)
 {
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngraphs; g += gridDim.x * blockDim.x) {
         g_active[g] = active;
         g_iters[g] = 0;
+        g_changes[g] = 0;
     }
 }
 

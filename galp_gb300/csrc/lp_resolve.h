@@ -24,8 +24,16 @@ constexpr int64_t kChunk = 17;
 constexpr int64_t kTile = 256 * 17;
 constexpr int64_t kSpine = 256;
 constexpr int64_t kSpine2 = 256;
+static_assert(kTile == kChunk << 8 && kSpine == 256 && kSpine2 == 256, "resolve_rank shifts by 8");
 
 GALP_HD int64_t imax64(int64_t a, int64_t b) { return a > b ? a : b; }
+
+// x / kChunk for x >= 0: unsigned, and in 32 bits where x is that small
+GALP_HD int64_t div_chunk(int64_t x)
+{
+    const uint64_t u = (uint64_t)x;
+    return (u >> 32) ? (int64_t)(u / (uint64_t)kChunk) : (int64_t)((uint32_t)u / (uint32_t)kChunk);
+}
 
 // Priority of position i (0 <= i < kTile) inside a tile that lies wholly within one
 // vertex's runs.  The reference reduces such a tile (segmented_reduce.cuh:263-304)
@@ -69,8 +77,8 @@ GALP_HD int resolve_rank(int64_t a, int64_t d, int64_t N, bool is_last, Q &q)
 {
     const int64_t b = a + d;
     const int64_t e = is_last ? ((N + kTile - 1) / kTile) * kTile - 1 : b - 1;
-    const int64_t ke = e / kTile, ce = e / kChunk, sb = ke / kSpine, qe = sb / kSpine2;
-    const int64_t ka = a / kTile;
+    // a tile is kTile / kChunk = 256 chunks: one division gives chunk, tile and spine blocks
+    const int64_t ce = div_chunk(e), ke = ce >> 8, sb = ke >> 8, qe = sb >> 8;
 
     const int64_t rho = imax64(0, ce * kChunk - a);
     if (rho < d) {
@@ -83,6 +91,7 @@ GALP_HD int resolve_rank(int64_t a, int64_t d, int64_t N, bool is_last, Q &q)
         if (r >= 0) return r;
     }
     // no candidate in the last tile: the segment spans earlier tiles (ka < ke)
+    const int64_t ka = div_chunk(a) >> 8;
     auto pick_in_tile = [&](int c) -> int {
         const int64_t j = (a + c) / kTile;
         if (a > j * kTile) return c;           // partial first tile: leftmost candidate
@@ -93,7 +102,7 @@ GALP_HD int resolve_rank(int64_t a, int64_t d, int64_t N, bool is_last, Q &q)
         int c = q.first_ge(lo1);
         if (c >= 0 && c < tau) return pick_in_tile(c);
     }
-    const int64_t qa = (ka / kSpine) / kSpine2;
+    const int64_t qa = ka >> 16;
     const int64_t chunk_runs = kSpine2 * kSpine * kTile;
     if (qa < qe) {
         int cl = q.last_lt(qe * chunk_runs - a);

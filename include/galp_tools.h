@@ -38,8 +38,8 @@ typedef struct {
     double pipe_ms;        /* count + scan + resolve kernels: summed device time */
     int32_t pipe_groups;   /* scopes timed */
     int32_t big_pre_groups;
-    double big_pre_ms;     /* big_insert + big_stats + big_dcnt: summed device time */
-    double big_post_ms;    /* big_resolve + big_clear + big_reset */
+    double big_pre_ms;     /* hub pre-pass (big_insert ... big_stats): summed device time */
+    double big_post_ms;    /* big_resolve */
     int32_t big_post_groups;
     int32_t first_groups;  /* first-iteration shortcuts timed */
     double first_ms;       /* first_iteration_kernel (labels = IDs, sorted adjacency): summed
