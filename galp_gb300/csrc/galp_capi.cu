@@ -341,6 +341,13 @@ Engine::~Engine()
         if (ev_consumed[i]) cudaEventDestroy(ev_consumed[i]);
     }
     if (copy_stream) cudaStreamDestroy(copy_stream);
+    for (cudaStream_t s : side_stream)
+        if (s) {
+            cudaStreamSynchronize(s);  // a run that failed half-way may not have joined it
+            cudaStreamDestroy(s);
+        }
+    for (cudaEvent_t e : {ev_fork, ev_side[0], ev_side[1]})
+        if (e) cudaEventDestroy(e);
     if (registered) cudaHostUnregister((void *)h_nbr);
 }
 
@@ -755,6 +762,27 @@ int Engine::launch_limits()
     return GALP_OK;
 }
 
+// Whether this scope's three kernel groups (hubs; CTA tables; small and lane-group sorts) go to
+// streams of their own.  Profiling spans one stream; a captured call stays on the caller's.
+bool Engine::forks(cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (prof.on || batched || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+        return false;
+    if (!ev_side[1]) {
+        bool ok = true;
+        for (cudaStream_t &x : side_stream)
+            ok = ok && (x || cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking) == cudaSuccess);
+        for (cudaEvent_t *e : {&ev_fork, &ev_side[0], &ev_side[1]})
+            ok = ok && (*e || cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess);
+        if (!ok) {  // one stream does as well
+            (void)cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
+}
+
 int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, const int32_t *lab_in,
                           int32_t *lab_out, const uint8_t *dirty, int32_t *changed)
 {
@@ -774,27 +802,41 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     q.dirty = dirty;
     q.changed = changed;
     int e0 = -1;
+    const int ncta = sc.nms + sc.nml + sc.nmx - sc.gcut[5];
+    const bool fork = sc.e1 - sc.e0 <= kForkMaxEntries && (a.nbig || ncta > 0) && forks(st);
+    cudaStream_t hub_st = st, cta_st = st;
+    if (fork) {
+        GALP_CUDA(cudaEventRecord(ev_fork, st));
+        if (a.nbig) {
+            hub_st = side_stream[0];
+            GALP_CUDA(cudaStreamWaitEvent(hub_st, ev_fork, 0));
+        }
+        if (ncta > 0) {
+            cta_st = side_stream[1];
+            GALP_CUDA(cudaStreamWaitEvent(cta_st, ev_fork, 0));
+        }
+    }
     if (a.nbig) {
         if (prof.on) e0 = prof.mark(st);
-        big_insert_kernel<<<a.nchunks, kTB, 0, st>>>(a);
-        launched("big_insert_kernel", st);
+        big_insert_kernel<<<a.nchunks, kTB, 0, hub_st>>>(a);
+        launched("big_insert_kernel", hub_st);
         // smaller partitions (hub_part_shift), smaller tables and more CTAs per SM
         if (sched.hub_shift >= 2)
             hub_count_kernel<kHubCountThreads / 4, kHubTab / 4>
                 <<<std::min(a.nparts, hub_count_blocks_quarter), kHubCountThreads / 4,
-                   sizeof(uint32_t) * kHubTab / 2, st>>>(a);
+                   sizeof(uint32_t) * kHubTab / 2, hub_st>>>(a);
         else if (sched.hub_shift == 1)
             hub_count_kernel<kHubCountThreads / 2, kHubTab / 2>
                 <<<std::min(a.nparts, hub_count_blocks_half), kHubCountThreads / 2, sizeof(uint32_t) * kHubTab,
-                   st>>>(a);
+                   hub_st>>>(a);
         else
             hub_count_kernel<kHubCountThreads, kHubTab>
-                <<<std::min(a.nparts, hub_count_blocks), kHubCountThreads, sizeof(uint32_t) * 2 * kHubTab, st>>>(a);
-        launched("hub_count_kernel", st);
-        big_combine_kernel<<<(a.nbig + 7) / 8, 256, 0, st>>>(a, q);
-        launched("big_combine_kernel", st);
-        big_stats_kernel<<<a.nschunks, kTB, 0, st>>>(a);
-        launched("big_stats_kernel", st);
+                <<<std::min(a.nparts, hub_count_blocks), kHubCountThreads, sizeof(uint32_t) * 2 * kHubTab, hub_st>>>(a);
+        launched("hub_count_kernel", hub_st);
+        big_combine_kernel<<<(a.nbig + 7) / 8, 256, 0, hub_st>>>(a, q);
+        launched("big_combine_kernel", hub_st);
+        big_stats_kernel<<<a.nschunks, kTB, 0, hub_st>>>(a);
+        launched("big_stats_kernel", hub_st);
         if (prof.on) prof.spans[1].push_back({e0, prof.mark(st)});
     }
     if (prof.on) e0 = prof.mark(st);
@@ -832,26 +874,34 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
             if (variant.cta_stage)  // neighbour IDs staged by bulk copies (the stage follows the table)
                 count_cta_kernel<kTB, 2 * kLargeMax, true>
                     <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax + sizeof(int32_t) * (kLargeMax + 8),
-                       st>>>(q, 1);
+                       cta_st>>>(q, 1);
             else
                 count_cta_kernel<kTB, 2 * kLargeMax>
-                    <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax, st>>>(q, 1);
-            launched("count_cta_kernel<256>", st);
+                    <<<g256, kTB, sizeof(unsigned long long) * 2 * kLargeMax, cta_st>>>(q, 1);
+            launched("count_cta_kernel<256>", cta_st);
         }
         // rows with a CTA split at 1024 (forced or learned) send 1025..2048 here
         const bool rows = policy == 0 && disp_mode != 0;
         const int nxla = sc.n6144 - sc.gcut[rows ? 5 : 6];
         if (nxla > 0) {
             count_cta_kernel<512, 2 * kXlAMax><<<(int)std::min<int64_t>(nxla, (int64_t)sms * 2), 512,
-                                                 sizeof(unsigned long long) * 2 * kXlAMax, st>>>(q, 2);
-            launched("count_cta_kernel<512>", st);
+                                                 sizeof(unsigned long long) * 2 * kXlAMax, cta_st>>>(q, 2);
+            launched("count_cta_kernel<512>", cta_st);
         }
         if (nmid > sc.n6144) {
             count_cta_kernel<kXlThreads, kXlSlots>
                 <<<(int)std::min<int64_t>(nmid - sc.n6144, (int64_t)sms), kXlThreads,
-                   sizeof(unsigned long long) * kXlSlots, st>>>(q, 3);
-            launched("count_cta_kernel<1024>", st);
+                   sizeof(unsigned long long) * kXlSlots, cta_st>>>(q, 3);
+            launched("count_cta_kernel<1024>", cta_st);
         }
+    }
+    if (hub_st != st) {
+        GALP_CUDA(cudaEventRecord(ev_side[0], hub_st));
+        GALP_CUDA(cudaStreamWaitEvent(st, ev_side[0], 0));
+    }
+    if (cta_st != st) {
+        GALP_CUDA(cudaEventRecord(ev_side[1], cta_st));
+        GALP_CUDA(cudaStreamWaitEvent(st, ev_side[1], 0));
     }
     const int64_t nv = sc.v1 - sc.v0;
     if (nv > 0) {
