@@ -978,8 +978,9 @@ DispatchArgs Engine::dispatch_args(int it) const
 // iterations the launches of the separate kernels would bound.
 bool Engine::fused_fits() const
 {
-    return policy == 0 && (batched ? G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries : m <= kFusedMaxEntries) &&
-           n > 0 && n <= kFusedMaxVertices && sched.big_v.empty();
+    if (policy != 0 || n < 1 || n > kFusedMaxVertices || !sched.big_v.empty()) return false;
+    if (batched) return G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries;
+    return m <= kFusedMaxEntries && (n <= kFusedAnyVertices || m >= kFusedDense * n);
 }
 
 // ... and whether this run is: under the default kernels and the fixed rule, not in a stream
@@ -1009,7 +1010,7 @@ int Engine::setup_fused(cudaStream_t st)
     for (int g = 1; g <= 5; ++g) tiles += (sc.gcut[g] - sc.gcut[g - 1] + (32 >> g) - 1) / (32 >> g);
     fused_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, std::min(sms, kFusedMaxBlocks)));
     GALP_CUDA(cudaFuncSetAttribute(fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(unsigned long long) * kXlSlots)));
+                                   (int)std::max(kFusedSmem<kFusedWide>, sizeof(unsigned long long) * kXlSlots)));
     const size_t graphs = batched ? (size_t)G : 1;
     GALP_CUDA(b_fused.alloc(sizeof(FusedState) + sizeof(long long) * 3 * (kFusedMaxBlocks + graphs) +
                             (batched ? sizeof(unsigned long long) * 3 * graphs : 0)));

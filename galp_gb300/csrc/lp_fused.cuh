@@ -6,9 +6,9 @@
 // barriers per iteration:
 //
 //   count    vertices of more than 1024 neighbours by the block (hash table in shared
-//            memory), lane-group and small tiles by its warps (the code of the separate
-//            kernels); each warp adds its vertices' distinct counts to the sums of the
-//            chunks of vertices they belong to
+//            memory), lane-group and small tiles by warps (the code of the separate
+//            kernels), one list of tiles for all warps of the grid; each warp adds its
+//            vertices' distinct counts to the sums of the chunks of vertices they belong to
 //   barrier
 //   resolve  each block scans the distinct counts of its own chunk from the chunk sums and
 //            resolves the chunk's tied vertices where it meets them
@@ -17,6 +17,14 @@
 // Batches of graphs run the same way, with run positions, change counts and early exits per
 // graph: the sums are then those of the pieces in which graphs and chunks cut the vertices.
 //
+// Bound by the latency of a tile (two round trips to L2 per eight rows of gathers) and of the
+// barriers (1.7 us each) on the smallest graphs; a warp's first tile is therefore the same in every
+// iteration, with its neighbours in shared memory, and its gathers are 16 in flight.  On skewed
+// graphs bound by the balance between the blocks: the other tiles are claimed from the list.
+// Passes of ten iterations, tiles dealt out in fixed order, each kind by itself and gathered by the
+// separate kernels' code -> this (us): planted partitions of 10 K entries 158 -> 124, 294 K 230 ->
+// 160; R-MAT 16 423 -> 342; LFR of 560 K entries 309 -> 200; batch of 96 graphs 432 -> 400.
+//
 // Labels, change counts, run counts and the dispatch log are those of the separate kernels.
 #pragma once
 
@@ -24,18 +32,29 @@
 
 namespace galp {
 
-// Block shapes: 512 threads where latency is all there is (up to kFusedNarrowEntries), 768 above,
-// for more of the gathers in flight.
+// Block shapes: 512 threads where latency is all there is (up to kFusedNarrowEntries), with plans of
+// the fixed tiles; 768 above, for more of the gathers in flight, without (their 96 KB would come out
+// of the L1 cache: LFR of 5.5 M entries 663 -> 886 us).  768 threads have 80 registers: they store a
+// gathered row before the next is loaded (tile_gather), all eight loaded first would spill (planted
+// partitions of 3.8 M entries 454 -> 519).  512 against 768 threads (us): R-MAT 16 (1.8 M) 342 and
+// 380, LFR of 1.9 M 357 and 362, R-MAT 18 with edge factor 4 (2.0 M) 437 and 436, planted partitions
+// of 3.8 M 466 and 454, LFR of 5.5 M 691 and 663.
 constexpr int kFusedNarrow = 512, kFusedWide = 768;
+constexpr int64_t kFusedNarrowEntries = 1 << 21;
 constexpr int kFusedMaxBlocks = 256;
-// Up to these sizes a run is one kernel.  Passes of ten iterations, separate kernels against one
-// (us): planted partitions of 10 K entries 458 and 147, 294 K 691 and 220, 3.8 M 906 and 545;
-// R-MAT 16 (1.8 M) 1123 and 393; LFR of 5.5 M entries 1030 and 757, of 18 M 2093 and 2077;
-// 1.5 M vertices with 7.5 M entries 1693 and 1638.  Batches, whose separate kernels are one
-// CUDA-graph launch: 96 graphs with 1.8 M entries 574 and 417, 1,000 graphs with 3.9 M entries
-// 775 and 870.
-constexpr int64_t kFusedMaxEntries = 1 << 23, kFusedMaxVertices = 1 << 21;
-constexpr int64_t kFusedMaxBatchEntries = 1 << 21, kFusedNarrowEntries = 1 << 20;
+// Up to these sizes a run is one kernel (above kFusedAnyVertices only with kFusedDense entries per
+// vertex: of a sparse graph's run the resolve phase is the larger part, and its separate kernel has
+// more threads).  Passes of ten iterations, separate kernels against one (us): planted partitions of
+// 10 K entries 336 and 124, 294 K 496 and 160, 3.8 M 713 and 454; R-MAT 16 (1.8 M) 699 and 342; LFR
+// of 5.5 M entries 916 and 663, 18 M 1964 and 1768, 24 M (700 K vertices) 2131 and 1865; planted
+// partitions of a million vertices with 5 M entries 1078 and 1071, 15 M 1516 and 1458, 25 M 1825 and
+// 1846; 1.5 M vertices with 7.5 M entries 1367 and 1446, with 21 M (LFR) 2386 and 2165.  Batches,
+// whose separate kernels are one CUDA-graph launch (the context's first pass, with the capture, and
+// a later one): 16 graphs with 312 K entries 440 / 286 and 234 / 197, 96 graphs with 738 K entries
+// 478 / 319 and 341 / 296, 96 with 1.8 M 600 / 383 and 467 / 400, 1,000 with 3.9 M 665 and 877 later.
+constexpr int64_t kFusedMaxEntries = 1 << 25, kFusedMaxVertices = 1 << 21;
+constexpr int64_t kFusedAnyVertices = 1 << 20, kFusedDense = 8;
+constexpr int64_t kFusedMaxBatchEntries = 1 << 21;
 constexpr int kFusedMaxGraphs = 4096;
 constexpr long long kFusedSpinLimit = 1ll << 21;  // polls of a barrier wait (about a second)
 
@@ -46,6 +65,7 @@ struct FusedState {
     unsigned left;                           // blocks that have ended it
     unsigned long long changes[3];           // of iteration i in entry i % 3
     unsigned long long runs[3];              // distinct labels, likewise
+    int claimed[3];                          // tiles handed out beyond the fixed ones, likewise
 };
 
 struct FusedArgs {
@@ -112,9 +132,14 @@ union FusedTile {
     GroupBuf group;
 };
 template <int THREADS>
-constexpr size_t kFusedSmem = sizeof(FusedTile) * (THREADS / 32);
-static_assert(sizeof(FusedResolve<kFusedNarrow>) <= kFusedSmem<kFusedNarrow> &&
-                  sizeof(FusedResolve<kFusedWide>) <= kFusedSmem<kFusedWide>,
+constexpr size_t kFusedTiles = sizeof(FusedTile) * (THREADS / 32);  // the plans lie behind
+template <int THREADS>
+constexpr int kFusedPlan = THREADS > kFusedNarrow ? 0 : 16;
+template <int THREADS>
+constexpr size_t kFusedSmem =
+    kFusedTiles<THREADS> + (kFusedPlan<THREADS> ? sizeof(int32_t) * kPlanWords * (THREADS / 32) : 0);
+static_assert(sizeof(FusedResolve<kFusedNarrow>) <= kFusedTiles<kFusedNarrow> &&
+                  sizeof(FusedResolve<kFusedWide>) <= kFusedTiles<kFusedWide>,
               "the resolve buffers fit the tile buffers");
 
 // State of a vertex in the resolve phase, loaded in one round trip whether it is tied or not.
@@ -209,19 +234,38 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
     };
     unsigned barriers = 0;
     __syncthreads();
-    // tiles: consecutive ones on different blocks; the blocks' offsets turn with the warp so that
-    // no block has only one quarter of the small vertices' degree windows
-    const int ngroup = T.count(), nsmall = (p.nsmall + 31) >> 5;
-    auto tile_of = [&](int r) { return r * nb + (b + r) % nb; };
-    auto small_head = [&](int r) {
+    // tiles: the lane groups' (largest degrees first), then the small vertices'.  Every warp of a
+    // block without vertices above kGroupMax has its first tile fixed, consecutive ones on different
+    // blocks, with its vertices and offsets in registers for all iterations; the other tiles are
+    // claimed one by one.
+    const int ngroup = T.count(), ntiles = ngroup + ((p.nsmall + 31) >> 5);
+    const int nfree = max(nb - ncta, 0), nfixed = nfree * kFusedWarps;
+    auto head_of = [&](int t) {
+        if (t < ngroup) return group_head<true>(p, T, t, false);
         TileHead h{-1, 0, 0, 0, 0, 1};
-        const int i = tile_of(r) * 32 + lane;
-        if (i < p.nsmall) tile_head<true>(p, h, p.small_v[i], false);
+        const int i = (t - ngroup) * 32 + lane;
+        if (t < ntiles && i < p.nsmall) tile_head<true>(p, h, p.small_v[i], false);
         return h;
     };
-    // the warp's first tiles: their vertices and offsets stay in registers for all iterations
-    const TileHead group0 = group_head<true>(p, T, w * nb < ngroup ? tile_of(w) : ngroup, false);
-    const TileHead small0 = small_head(w);
+    const int tile0 = b >= ncta ? w * nfree + b - ncta : -1;
+    const TileHead head0 = head_of(tile0 >= 0 ? tile0 : ntiles);
+    // its plan: the block's table is never used, so it stays
+    constexpr int kPlanPer = kFusedPlan<kFusedThreads>;
+    int32_t *plan = reinterpret_cast<int32_t *>(fused_smem + kFusedTiles<kFusedThreads>) + w * kPlanWords;
+    if (!kPlanPer || tile0 < 0 || tile0 >= ntiles) {
+        plan = nullptr;
+    } else {
+        int first = 0, n = 32;  // the lane's part of its vertex's neighbours
+        if (tile0 < ngroup) {
+            n = group_shape_of(head0.deg, head0.g).N;
+            first = (lane & ((1 << head0.g) - 1)) * n;
+        }
+        const int cnt = head0.v >= 0 ? head0.deg - first : 0;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j)
+            plan[j * 32 + lane] = j < n && j < cnt ? __ldg(&p.nbr[head0.o0 - p.nbr_shift + first + j]) : -1;
+        __syncwarp();
+    }
     if (!a.shortcut && !grid_barrier(st, ctl, &failed, ++barriers)) return;  // labels gathered by other blocks
     int it = 0;
     long long runs = 0, last_changes = 0;
@@ -318,21 +362,24 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 }
                 __syncthreads();
             }
-            for (int r = w; r * nb < ngroup; r += kFusedWarps) {
-                TileHead hd = group0;
-                if (r != w) hd = group_head<true>(p, T, tile_of(r), false);
+            auto claim = [&] {
+                if (ntiles <= nfixed) return ntiles;
+                int c = 0;
+                if (lane == 0) c = atomicAdd(&st->claimed[it % 3], 1);
+                return nfixed + __shfl_sync(kFull, c, 0);
+            };
+            for (int t = tile0 >= 0 ? tile0 : claim(); t < ntiles; t = claim()) {
+                TileHead hd = head0;
+                if (t != tile0) hd = head_of(t);
                 else if (hd.v >= 0) hd.old = get_label<true>(&p.lab_in[hd.v]);
-                const int d = group_tile<true>(p, tiles[w].group, hd, changes);
-                const bool leader = (lane & ((1 << hd.g) - 1)) == 0;
-                add_runs(sums, piece_of(hd.v), leader && hd.v >= 0 ? d : 0);
-                if (leader && hd.v >= 0) counted += (unsigned)d;
-            }
-            for (int r = w; r * nb < nsmall; r += kFusedWarps) {
-                TileHead hd = small0;
-                if (r != w) hd = small_head(r);
-                else if (hd.v >= 0) hd.old = get_label<true>(&p.lab_in[hd.v]);
-                bool chg;
-                const int d = small_tile<true>(p, tiles[w].small, hd, changes, chg);
+                int d;
+                if (t < ngroup) {
+                    d = group_tile<true, kPlanPer>(p, tiles[w].group, hd, changes, t == tile0 ? plan : nullptr);
+                    if ((lane & ((1 << hd.g) - 1)) || hd.v < 0) d = 0;  // the group's first lane counts
+                } else {
+                    bool chg;
+                    d = small_tile<true, kPlanPer>(p, tiles[w].small, hd, changes, chg, t == tile0 ? plan : nullptr);
+                }
                 add_runs(sums, piece_of(hd.v), d);
                 counted += (unsigned)d;
             }
@@ -353,6 +400,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             if (b == 0 && tid == 0) {
                 st->changes[(it + 1) % 3] = 0;
                 st->runs[(it + 2) % 3] = 0;
+                st->claimed[(it + 1) % 3] = 0;
             }
             if (BATCH)
                 for (int g = b * kFusedThreads + tid; g < p.ngraphs; g += nb * kFusedThreads)
@@ -582,7 +630,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             ctl->iter = it;
             ctl->N = runs;
             // (st->runs of other blocks' last read lies before the last barrier)
-            for (int i = 0; i < 3; ++i) st->runs[i] = 0;
+            for (int i = 0; i < 3; ++i) {
+                st->runs[i] = 0;
+                st->claimed[i] = 0;
+            }
         }
     }
 }

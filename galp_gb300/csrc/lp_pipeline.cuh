@@ -153,6 +153,22 @@ __device__ __forceinline__ int32_t gather_label(const int32_t *p)
     }
 }
 
+// The label of vertex id, INT_MAX where id < 0.  LIVE loads are volatile, so a condition around one
+// would be a branch that the compiler moves no other load across: the condition is in the load.
+template <bool LIVE>
+__device__ __forceinline__ int32_t gather_label_if(const int32_t *lab, int id)
+{
+    if constexpr (LIVE) {
+        int32_t v;
+        asm volatile("{\n\t.reg .b64 pol;\n\t.reg .pred some;\n\tsetp.ge.s32 some, %2, 0;\n\tmov.b32 %0, 0x7fffffff;\n\t"
+            "createpolicy.fractional.L2::evict_last.b64 pol, 1.0;\n\t"
+            "@some ld.global.L2::cache_hint.b32 %0, [%1], pol;\n\t}" : "=&r"(v) : "l"(lab + id), "r"(id));
+        return v;
+    } else {
+        return id >= 0 ? gather_label<false>(&lab[id]) : INT_MAX;
+    }
+}
+
 // Record a changed vertex for the next iteration's frontier (single thread).
 __device__ __forceinline__ void note_change(const PipeArgs &p, int32_t v, int32_t nl, int32_t old)
 {
@@ -737,7 +753,8 @@ struct TileBuf {
 
 // Gather a tile of one vertex per lane: the lane's `deg` labels, whose first entry is at e0
 // of the neighbour buffer, go to its row, padded to n words (a multiple of 4).
-template <bool LIVE>
+// SLIM (where registers are short): a row's labels are stored before the next row's are loaded.
+template <bool LIVE, bool SLIM>
 __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int deg, int64_t e0, int n)
 {
     const int lane = threadIdx.x & 31;
@@ -784,9 +801,21 @@ __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int d
                 at[u] = B.at[own] + s;
             }
         }
+        if constexpr (SLIM) {
 #pragma unroll
-        for (int u = 0; u < PER; ++u)
-            if (id[u] >= 0) B.rows[at[u]] = gather_label<LIVE>(&p.lab_in[id[u]]);
+            for (int u = 0; u < PER; ++u)
+                if (id[u] >= 0) B.rows[at[u]] = gather_label<LIVE>(&p.lab_in[id[u]]);
+        } else {  // all loads before the first store: the warp waits once for the eight rows
+            int32_t lb[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                if (LIVE && (r0 + u) * 32 >= total) continue;  // warp-uniform
+                lb[u] = gather_label_if<LIVE>(p.lab_in, id[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u)
+                if (id[u] >= 0) B.rows[at[u]] = lb[u];
+        }
     }
     __syncwarp();
 }
@@ -830,17 +859,43 @@ __device__ __forceinline__ void tile_head(const PipeArgs &p, TileHead &h, int v,
     h.dirty = fr ? (int)p.dirty[v] : 1;
 }
 
-// Count the warp's 32 small vertices (one per lane), with the tile buffer B.  Writes their state
-// and the labels of untied ones (chg: it changed); returns the lane's distinct count.
-template <bool LIVE>
+// Plan of a tile that a warp counts again and again: word j * 32 + lane is the neighbour whose
+// label is the j-th of the lane's row, -1 = none.
+constexpr int kPlanWords = 32 * 32;
+
+// Fill the rows (`stride` words apart) by a plan, the first n labels of each (a multiple of 4),
+// PER of them in flight.
+template <int PER>
+__device__ __forceinline__ void plan_gather(const PipeArgs &p, const int32_t *plan, int32_t *rows, int stride, int n)
+{
+    const int lane = threadIdx.x & 31;
+    for (int j0 = 0; j0 < n; j0 += PER) {
+        int32_t x[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) x[u] = j0 + u < n ? plan[(j0 + u) * 32 + lane] : -1;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) x[u] = gather_label_if<true>(p.lab_in, x[u]);
+#pragma unroll
+        for (int u = 0; u < PER; u += 4)
+            if (j0 + u < n)
+                *reinterpret_cast<int4 *>(rows + lane * stride + j0 + u) = make_int4(x[u], x[u + 1], x[u + 2], x[u + 3]);
+    }
+    __syncwarp();
+}
+
+// Count the warp's 32 small vertices (one per lane), with the tile buffer B (PLAN: rows in flight
+// by the tile's plan, 0 = it has none).  Writes their state and the labels of untied ones (chg: it
+// changed); returns the lane's distinct count.
+template <bool LIVE, int PLAN = 0>
 __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const TileHead &hd,
-                                          unsigned long long &changes, bool &chg)
+                                          unsigned long long &changes, bool &chg, const int32_t *plan = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const int v = hd.v;
     const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
     const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
-    tile_gather<LIVE>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
+    if (PLAN && plan) plan_gather<PLAN ? PLAN : 4>(p, plan, B.rows, kSmallRow, 4 * n4);
+    else tile_gather<LIVE, LIVE && PLAN == 0>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
     int32_t *row = B.rows + lane * kSmallRow;
     uint32_t h = 0u;
     switch (n4) {  // warp-uniform
@@ -891,7 +946,18 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
             }
         }
     }
-    if (__any_sync(kFull, k > 2)) {
+    unsigned spill = __ballot_sync(kFull, k > 2);
+    if (PLAN && plan) {
+        // one vertex after the other (the owners of slots are not at hand)
+#pragma unroll 1
+        while (spill) {
+            const int src = __ffs(spill) - 1;
+            spill &= spill - 1;
+            const int64_t e = __shfl_sync(kFull, hd.o0 - p.nbr_shift, src);
+            const int dg = __shfl_sync(kFull, deg, src);
+            if (lane < dg) p.run_lab[e + lane] = B.rows[src * kSmallRow + lane];
+        }
+    } else if (spill) {
         const int total = __reduce_add_sync(kFull, deg);
         const unsigned nz = __ballot_sync(kFull, deg > 0);
         if (deg > 0 && k <= 2) B.dlt[__popc(nz & ((1u << lane) - 1u))] = LLONG_MIN;
@@ -1146,44 +1212,66 @@ __device__ __forceinline__ TileHead group_head(const PipeArgs &p, const GroupTil
     return h;
 }
 
-// Count the warp's tile of vertices (one per group of lanes).  Writes their state and the
-// labels of untied ones; returns the group's distinct count.
-template <bool LIVE>
+// The shape for a tile whose lanes belong to vertices of `deg` labels to count.
+__device__ __forceinline__ GroupShape group_shape_of(int deg, int g)
+{
+    const int n = (__reduce_max_sync(kFull, deg) + (1 << g) - 1) >> g;
+    return n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
+}
+
+// Count the warp's tile of vertices (one per group of lanes; PLAN and plan as for small tiles).
+// Writes their state and the labels of untied ones; returns the group's distinct count.
+template <bool LIVE, int PLAN = 0>
 __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const TileHead &hd,
-                                          unsigned long long &changes)
+                                          unsigned long long &changes, const int32_t *plan = nullptr)
 {
     const int lane = threadIdx.x & 31;
     int32_t *rows = B.rows;
     const int v = hd.v, g = hd.g, G = 1 << g, sub = lane & (G - 1);
     const bool leader = sub == 0;
     const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-    const int n = (__reduce_max_sync(kFull, deg) + G - 1) >> g;
-    const GroupShape sh = n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
+    const GroupShape sh = group_shape_of(deg, g);
     const int N = sh.N, stride = sh.stride;
-    if (leader) {
-        B.ent[lane >> g] = hd.o0 - p.nbr_shift;
-        B.deg[lane >> g] = deg;
-    }
-    for (int j = 0; j < N; j += 4)
-        *reinterpret_cast<int4 *>(rows + lane * stride + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
-    __syncwarp();
-    // gather: row r holds entries 32 (r mod G) ... of the tile's vertex r / G
-    constexpr int PER = 8;  // rows in flight
-    for (int r0 = 0; r0 < 32; r0 += PER) {
-        int id[PER];
-#pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
-            id[u] = j < B.deg[q] ? ld_nbr(&p.nbr[B.ent[q] + j]) : -1;
+    if (PLAN && plan) {
+        plan_gather<PLAN ? PLAN : 4>(p, plan, rows, stride, N);
+    } else {
+        if (leader) {
+            B.ent[lane >> g] = hd.o0 - p.nbr_shift;
+            B.deg[lane >> g] = deg;
         }
+        for (int j = 0; j < N; j += 4)
+            *reinterpret_cast<int4 *>(rows + lane * stride + j) = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+        __syncwarp();
+        // gather: row r holds entries 32 (r mod G) ... of the tile's vertex r / G
+        constexpr int PER = 8;  // rows in flight
+        for (int r0 = 0; r0 < 32; r0 += PER) {
+            int id[PER];
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
-            const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
-            if (id[u] >= 0)
-                rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] = gather_label<LIVE>(&p.lab_in[id[u]]);
+            for (int u = 0; u < PER; ++u) {
+                const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+                id[u] = j < B.deg[q] ? ld_nbr(&p.nbr[B.ent[q] + j]) : -1;
+            }
+            if constexpr (LIVE && PLAN == 0) {  // as for small tiles
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+                    if (id[u] >= 0)
+                        rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] =
+                            gather_label<LIVE>(&p.lab_in[id[u]]);
+                }
+            } else {
+                int32_t lb[PER];
+#pragma unroll
+                for (int u = 0; u < PER; ++u) lb[u] = gather_label_if<LIVE>(p.lab_in, id[u]);
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int q = (r0 + u) >> g, j = ((r0 + u) & (G - 1)) * 32 + lane;
+                    if (id[u] >= 0) rows[(q << g) * stride + j + (j * sh.rcp >> 16) * (stride - N)] = lb[u];
+                }
+            }
         }
+        __syncwarp();
     }
-    __syncwarp();
     uint32_t h;
     if (N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
     else if (N == 24) h = group_sort_rows<24>(rows, g);

@@ -1,0 +1,66 @@
+"""One-kernel runs: tiles fixed to a warp (counted by a plan kept in shared memory) and tiles
+claimed from the list, lane-group and small tiles of every row length, on both block shapes."""
+import numpy as np
+import pytest
+
+import galp_gb300
+import oracle
+from galp_gb300 import tools
+
+pytestmark = pytest.mark.gpu
+
+SMS, NARROW = 152, 16  # resident blocks, warps of the narrow shape
+FIXED = SMS * NARROW   # tiles fixed to a warp when no block has a larger vertex
+
+
+def _check(degs, seed, niter=4, one=True):
+    rng = np.random.default_rng(seed)
+    n = len(degs)
+    off = np.zeros(n + 1, np.int64)
+    off[1:] = np.cumsum(degs)
+    pool = rng.integers(0, n, max(n // 4, 3), dtype=np.int64)  # ties, repeated labels
+    nbr = pool[rng.integers(0, len(pool), off[-1])].astype(np.int32)
+    g = galp_gb300.Graph(off, nbr)
+    _, want, counts = oracle.run_par(g.offsets, g.neighbors, niter, early_exit=False)
+    with galp_gb300.Propagator(g, early_exit=0) as p:
+        for _ in range(2):
+            before = tools.schedule_info(p).launches
+            p.run(niter)
+            assert (tools.schedule_info(p).launches - before == 1) == one
+            assert np.array_equal(p.get_labels(), want) and list(p.updates) == list(counts)
+
+
+@pytest.mark.parametrize("extra", [-33, -1, 0, 1, 32, 1000])
+def test_fixed_and_claimed(extra):
+    # 32 small vertices a tile: just below and above one tile for every warp
+    n = FIXED * 32 + extra
+    _check(np.random.default_rng(extra + 99).integers(0, 12, n), 105 + extra)
+
+
+@pytest.mark.parametrize("deg", [1, 4, 5, 16, 17, 31, 32, 33, 40, 41, 48, 49, 64, 160, 161, 192, 193, 256, 640, 641,
+                                 768, 769, 1023, 1024])
+def test_row_lengths(deg):
+    n = 70 if deg > 32 else 131
+    _check(np.full(n, deg), deg)
+    rng = np.random.default_rng(deg)
+    _check(rng.permutation(np.concatenate([np.full(n, deg), rng.integers(0, deg + 1, n)])), deg + 1)
+
+
+@pytest.mark.parametrize("large", [1, 100, SMS - 1, SMS, 2 * SMS + 5])
+def test_few_free_blocks(large):
+    rng = np.random.default_rng(large)
+    _check(rng.permutation(np.concatenate([rng.integers(1025, 1400, large), rng.integers(33, 200, 500),
+                                           rng.integers(0, 33, 9000)])), large)
+
+
+def test_wide():
+    # above 2 M entries: no plans
+    rng = np.random.default_rng(3)
+    _check(rng.permutation(np.concatenate([rng.integers(1025, 3000, 60), rng.integers(33, 1025, 3000),
+                                           rng.integers(0, 33, 60000)])), 3)
+
+
+@pytest.mark.parametrize("n, deg, one", [(1 << 20, 2, True), ((1 << 20) + 7, 8, True), ((1 << 20) + 7, 7, False),
+                                         ((1 << 21) + 1, 9, False)])
+def test_size_rule(n, deg, one):
+    _check(np.full(n, deg), deg, niter=2, one=one)
