@@ -994,6 +994,26 @@ bool Engine::fused_run(cudaStream_t st, int niter) const
     return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
+cudaLaunchConfig_t Engine::fused_launch(cudaStream_t st, cudaLaunchAttribute &attr) const
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)fused_blocks);
+    cfg.blockDim = dim3((unsigned)fused_threads);
+    cfg.dynamicSmemBytes = fused_smem;
+    cfg.stream = st;
+    if (fused_cluster) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)fused_cluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 // Buffers and launch shape of one-kernel runs (once per graph).
 int Engine::setup_fused(cudaStream_t st)
 {
@@ -1009,8 +1029,23 @@ int Engine::setup_fused(cudaStream_t st)
     int64_t tiles = (sc.nsv + 31) / 32 + ncta;
     for (int g = 1; g <= 5; ++g) tiles += (sc.gcut[g] - sc.gcut[g - 1] + (32 >> g) - 1) / (32 >> g);
     fused_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, std::min(sms, kFusedMaxBlocks)));
+    fused_cluster = 0;
+    if (narrow && !ncta && tiles <= kFusedClusterTiles) {
+        fused_blocks = 1;
+        while (fused_blocks < tiles && fused_blocks < kFusedClusterBlocks) fused_blocks *= 2;
+        fused_cluster = fused_blocks;
+    }
     GALP_CUDA(cudaFuncSetAttribute(fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)std::max(kFusedSmem<kFusedWide>, sizeof(unsigned long long) * kXlSlots)));
+    if (fused_cluster) {  // where the device has room for such a cluster
+        if (fused_cluster > 8)
+            GALP_CUDA(cudaFuncSetAttribute(fused_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute attr{};
+        const cudaLaunchConfig_t cfg = fused_launch(st, attr);
+        int room = 0;
+        if (cudaOccupancyMaxActiveClusters(&room, fused_kernel, &cfg) != cudaSuccess) (void)cudaGetLastError();
+        if (room < 1) fused_cluster = 0;
+    }
     const size_t graphs = batched ? (size_t)G : 1;
     GALP_CUDA(b_fused.alloc(sizeof(FusedState) + sizeof(long long) * 3 * (kFusedMaxBlocks + graphs) +
                             (batched ? sizeof(unsigned long long) * 3 * graphs : 0)));
@@ -1052,17 +1087,22 @@ int Engine::enqueue_run_fused(cudaStream_t st, int niter, long long thr)
         a.g_max_iter = batch_max_iter;
         a.early_exit = early_exit;
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)fused_blocks);
-    cfg.blockDim = dim3((unsigned)fused_threads);
-    cfg.dynamicSmemBytes = fused_smem;
-    cfg.stream = st;
     cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeCooperative;
-    attr.val.cooperative = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+    cudaError_t e = cudaSuccess;
+    if (fused_cluster) {
+        const cudaLaunchConfig_t cfg = fused_launch(st, attr);
+        a.cluster = 1;
+        e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+        if (e != cudaSuccess) {  // no room for the cluster (any more)
+            (void)cudaGetLastError();
+            fused_cluster = 0;
+            a.cluster = 0;
+        }
+    }
+    if (!a.cluster) {
+        const cudaLaunchConfig_t cfg = fused_launch(st, attr);
+        e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+    }
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // not all of the device is ours
         (void)cudaGetLastError();
         b_fused.release();

@@ -210,6 +210,7 @@ struct Engine {
     DevBuf b_fused;
     void (*fused_kernel)(FusedArgs) = nullptr;
     int fused_blocks = 0, fused_threads = 0, fused_slots = 0;
+    int fused_cluster = 0;  // blocks of the one cluster that the grid is, or 0
     size_t fused_smem = 0;
     DevBuf b_static_feat, b_vtab, b_disp, b_feat_log, b_var_log, b_weights;  // dispatch
     float static_feat[kDegBins + 3] = {};
@@ -285,6 +286,7 @@ struct Engine {
                       int32_t *lab_out, const uint8_t *dirty = nullptr, int32_t *changed = nullptr);
     int enqueue_run_incore(cudaStream_t st, int niter, long long thr);
     bool fused_fits() const;
+    cudaLaunchConfig_t fused_launch(cudaStream_t st, cudaLaunchAttribute &attr) const;
     bool fused_run(cudaStream_t st, int niter) const;
     int setup_fused(cudaStream_t st);
     int reset_fused(cudaStream_t st);

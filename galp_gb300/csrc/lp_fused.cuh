@@ -22,7 +22,7 @@
 // iteration, with its neighbours in shared memory, and its gathers are 16 in flight.  On skewed
 // graphs bound by the balance between the blocks: the other tiles are claimed from the list.
 // Passes of ten iterations, tiles dealt out in fixed order, each kind by itself and gathered by the
-// separate kernels' code -> this (us): planted partitions of 10 K entries 158 -> 124, 294 K 230 ->
+// separate kernels' code -> this (us): planted partitions of 10 K entries 158 -> 124 (115 as a cluster), 294 K 230 ->
 // 160; R-MAT 16 423 -> 342; LFR of 560 K entries 309 -> 200; batch of 96 graphs 432 -> 400.
 //
 // Labels, change counts, run counts and the dispatch log are those of the separate kernels.
@@ -45,7 +45,7 @@ constexpr int kFusedMaxBlocks = 256;
 // Up to these sizes a run is one kernel (above kFusedAnyVertices only with kFusedDense entries per
 // vertex: of a sparse graph's run the resolve phase is the larger part, and its separate kernel has
 // more threads).  Passes of ten iterations, separate kernels against one (us): planted partitions of
-// 10 K entries 336 and 124, 294 K 496 and 160, 3.8 M 713 and 454; R-MAT 16 (1.8 M) 699 and 342; LFR
+// 10 K entries 336 and 115, 294 K 496 and 160, 3.8 M 713 and 454; R-MAT 16 (1.8 M) 699 and 342; LFR
 // of 5.5 M entries 916 and 663, 18 M 1964 and 1768, 24 M (700 K vertices) 2131 and 1865; planted
 // partitions of a million vertices with 5 M entries 1078 and 1071, 15 M 1516 and 1458, 25 M 1825 and
 // 1846; 1.5 M vertices with 7.5 M entries 1367 and 1446, with 21 M (LFR) 2386 and 2165.  Batches,
@@ -55,6 +55,14 @@ constexpr int kFusedMaxBlocks = 256;
 constexpr int64_t kFusedMaxEntries = 1 << 25, kFusedMaxVertices = 1 << 21;
 constexpr int64_t kFusedAnyVertices = 1 << 20, kFusedDense = 8;
 constexpr int64_t kFusedMaxBatchEntries = 1 << 21;
+// Runs of up to kFusedClusterTiles tiles, all small or lane-group ones, are one thread-block cluster:
+// its hardware barrier replaces the counter in global memory (0.6 us less each), and the launch is
+// not cooperative.  One block per tile and the counter against the cluster (us): 512 vertices with
+// 5 K entries 133 and 117, 1,024 with 10 K 133 and 115, 2,048 with 20 K (64 tiles) 139 and 122,
+// 1,349 with 24 K (R-MAT 11) 141 and 140, four graphs of together 1,070 vertices 162 and 151; with
+// more tiles 16 SMs are too few for the work: 2,700 vertices with 51 K (R-MAT 12) 156 and 165,
+// 4,096 with 113 K 143 and 148.
+constexpr int kFusedClusterBlocks = 16, kFusedClusterTiles = 64;
 constexpr int kFusedMaxGraphs = 4096;
 constexpr long long kFusedSpinLimit = 1ll << 21;  // polls of a barrier wait (about a second)
 
@@ -82,6 +90,7 @@ struct FusedArgs {
     int chunk;                // vertices per block in the resolve phase
     int slots;                // table slots for vertices above kGroupMax
     int agg_mode;
+    int cluster;              // the grid is one cluster
     // batches
     unsigned long long *g_changes;  // [3][graphs]: labels changed, likewise
     int32_t *g_active, *g_iters;
@@ -90,11 +99,16 @@ struct FusedArgs {
 };
 
 // The run's k-th barrier (k = 1, 2, ...) of all blocks; false when the wait ran out
-// (kErrLookback is set, and the block must return: the others give up in the same way).  The
+// (kErrLookback is set, and the block must return: the others give up in the same way).  In a run
+// that is one cluster no wait can run out: all its blocks are resident, and none returns early.  The
 // arrivals only count up, so a block waits for one number and nobody resets anything until the
 // last block leaves the run.
-__device__ __forceinline__ bool grid_barrier(FusedState *st, Ctl *ctl, int *failed, unsigned k)
+__device__ __forceinline__ bool grid_barrier(FusedState *st, Ctl *ctl, int *failed, unsigned k, int cluster)
 {
+    if (cluster) {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->arrived) : "memory");
@@ -266,7 +280,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             plan[j * 32 + lane] = j < n && j < cnt ? __ldg(&p.nbr[head0.o0 - p.nbr_shift + first + j]) : -1;
         __syncwarp();
     }
-    if (!a.shortcut && !grid_barrier(st, ctl, &failed, ++barriers)) return;  // labels gathered by other blocks
+    if (!a.shortcut && !grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;  // labels gathered by other blocks
     int it = 0;
     long long runs = 0, last_changes = 0;
     for (;;) {
@@ -392,7 +406,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 if (tid == 0 && sruns) atomicAdd(&st->runs[it % 3], sruns);
             }
         }
-        if (!grid_barrier(st, ctl, &failed, ++barriers)) return;
+        if (!grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;
         // entries of the iterations to come: their last readers passed the barrier before this one
         {
             long long *later = a.sums + (size_t)((it + 2) % 3) * a.pieces;
@@ -594,7 +608,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
             if (lane == 0 && c) atomicAdd(&st->changes[it % 3], c);
         }
-        if (!grid_barrier(st, ctl, &failed, ++barriers)) return;
+        if (!grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;
         last_changes = (long long)*((volatile unsigned long long *)&st->changes[it % 3]);
         if (b == 0 && tid == 0 && it < 64) ctl->counts[it] = (unsigned long long)last_changes;
         ++it;

@@ -64,3 +64,10 @@ def test_wide():
                                          ((1 << 21) + 1, 9, False)])
 def test_size_rule(n, deg, one):
     _check(np.full(n, deg), deg, niter=2, one=one)
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 300, 511, 2047, 2048, 2049])  # one cluster up to 64 tiles
+def test_cluster(n):
+    rng = np.random.default_rng(n)
+    _check(rng.integers(0, 20, n), n, niter=9)
+    _check(np.concatenate([rng.integers(0, 20, n), rng.integers(33, 1025, 9)]), n + 1, niter=9)
