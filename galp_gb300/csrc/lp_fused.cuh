@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
     } else {
         int first = 0, n = 32;  // the lane's part of its vertex's neighbours
         if (tile0 < ngroup) {
-            n = group_shape_of(head0.deg, head0.g).N;
+            n = group_shape_of<true>(head0.deg, head0.g).N;  // as group_tile with a plan
             first = (lane & ((1 << head0.g) - 1)) * n;
         }
         const int cnt = head0.v >= 0 ? head0.deg - first : 0;

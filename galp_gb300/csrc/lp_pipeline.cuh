@@ -883,6 +883,12 @@ __device__ __forceinline__ void plan_gather(const PipeArgs &p, const int32_t *pl
     __syncwarp();
 }
 
+// Kernels that keep plans have few tiles per warp, and the straight-line code of the networks is
+// mostly fetched for one tile: they use fewer of them (rows of 8, 16, 24, 32; group rows of 32).
+// Passes with all networks and with these (us): R-MAT 14 188 and 176, R-MAT 17 with edge factor 4
+// 297 and 277, LFR of 1.9 M entries 357 and 331.  R-MAT 24, whose warps run the same code over and
+// over, would lose: 49.9 and 50.6 ms.
+
 // Count the warp's 32 small vertices (one per lane), with the tile buffer B (PLAN: rows in flight
 // by the tile's plan, 0 = it has none).  Writes their state and the labels of untied ones (chg: it
 // changed); returns the lane's distinct count.
@@ -893,20 +899,22 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
     const int lane = threadIdx.x & 31;
     const int v = hd.v;
     const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-    const int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
+    constexpr bool FEW = PLAN > 0;
+    int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
+    if (FEW) n4 = (n4 + 1) & ~1;
     if (PLAN && plan) plan_gather<PLAN ? PLAN : 4>(p, plan, B.rows, kSmallRow, 4 * n4);
     else tile_gather<LIVE, LIVE && PLAN == 0>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
     int32_t *row = B.rows + lane * kSmallRow;
     uint32_t h = 0u;
     switch (n4) {  // warp-uniform
     case 0: break;
-    case 1: h = small_sort_row<4>(row); break;
+    case 1: if (!FEW) h = small_sort_row<4>(row); break;
     case 2: h = small_sort_row<8>(row); break;
-    case 3: h = small_sort_row<12>(row); break;
+    case 3: if (!FEW) h = small_sort_row<12>(row); break;
     case 4: h = small_sort_row<16>(row); break;
-    case 5: h = small_sort_row<20>(row); break;
+    case 5: if (!FEW) h = small_sort_row<20>(row); break;
     case 6: h = small_sort_row<24>(row); break;
-    case 7: h = small_sort_row<28>(row); break;
+    case 7: if (!FEW) h = small_sort_row<28>(row); break;
     default: h = small_sort_row<32>(row); break;
     }
     const uint32_t valid = deg >= 32 ? kFull : (1u << deg) - 1u;
@@ -1212,9 +1220,12 @@ __device__ __forceinline__ TileHead group_head(const PipeArgs &p, const GroupTil
     return h;
 }
 
-// The shape for a tile whose lanes belong to vertices of `deg` labels to count.
+// The shape for a tile whose lanes belong to vertices of `deg` labels to count.  FEW: one length
+// for all, 32 labels per lane.
+template <bool FEW>
 __device__ __forceinline__ GroupShape group_shape_of(int deg, int g)
 {
+    if (FEW) return group_shape(32);
     const int n = (__reduce_max_sync(kFull, deg) + (1 << g) - 1) >> g;
     return n <= 20 ? group_shape(20) : n <= 24 ? group_shape(24) : group_shape(32);
 }
@@ -1230,7 +1241,8 @@ __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const 
     const int v = hd.v, g = hd.g, G = 1 << g, sub = lane & (G - 1);
     const bool leader = sub == 0;
     const int deg = (v >= 0 && hd.dirty) ? hd.deg : 0;  // neighbours to count
-    const GroupShape sh = group_shape_of(deg, g);
+    constexpr bool FEW = PLAN > 0;
+    const GroupShape sh = group_shape_of<FEW>(deg, g);
     const int N = sh.N, stride = sh.stride;
     if (PLAN && plan) {
         plan_gather<PLAN ? PLAN : 4>(p, plan, rows, stride, N);
@@ -1273,8 +1285,8 @@ __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const 
         __syncwarp();
     }
     uint32_t h;
-    if (N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
-    else if (N == 24) h = group_sort_rows<24>(rows, g);
+    if (!FEW && N == 20) h = group_sort_rows<20>(rows, g);  // warp-uniform
+    else if (!FEW && N == 24) h = group_sort_rows<24>(rows, g);
     else h = group_sort_rows<32>(rows, g);
     const int cnt = min(max(deg - sub * N, 0), N);  // labels in this lane
     const uint32_t valid = cnt >= 32 ? kFull : (1u << cnt) - 1u;
@@ -1335,8 +1347,8 @@ __device__ __forceinline__ int group_tile(const PipeArgs &p, GroupBuf &B, const 
     }
     unsigned spill = __ballot_sync(kFull, leader && deg > 0 && k > 2);
     if (spill) {
-        if (N == 20) group_compact<20>(rows, g, h, m, rank0);
-        else if (N == 24) group_compact<24>(rows, g, h, m, rank0);
+        if (!FEW && N == 20) group_compact<20>(rows, g, h, m, rank0);
+        else if (!FEW && N == 24) group_compact<24>(rows, g, h, m, rank0);
         else group_compact<32>(rows, g, h, m, rank0);
         const int64_t e0 = hd.o0 - p.nbr_shift;
         while (spill) {  // one vertex after the other, coalesced
