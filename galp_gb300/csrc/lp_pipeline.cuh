@@ -1174,9 +1174,10 @@ __device__ __forceinline__ void group_compact(int32_t *rows, int g, uint32_t h, 
 // About 4.5 warp instructions per entry in tie-heavy iterations, none of them divergent or
 // behind a barrier, where tables in shared memory (one warp, 64 or 128 threads per vertex)
 // took 8 to 10 at 13 to 22 active lanes; half of them are the networks' minima and maxima,
-// which run at half rate.  Ten iterations of R-MAT 24: 20.0 -> 16.6 ms here and, the spilled
-// runs being in order, 2.6 -> 0.85 ms in resolve_mid; R-MAT 26 with edge factor 4: 28.9 ->
-// 23.2 and 6.0 -> 1.8.  Longer lists stay with the tables: a warp sorting 2048 labels, 64 to
+// which run at half rate.  Ten iterations of R-MAT 24: 20.0 -> 16.6 ms here (15.6 since all
+// eight rows of a gather are loaded before the first is stored) and, the spilled runs being in
+// order, 2.6 -> 0.85 ms in resolve_mid; R-MAT 26 with edge factor 4: 28.9 -> 23.2 and 6.0 -> 1.8.
+// Longer lists stay with the tables: a warp sorting 2048 labels, 64 to
 // a lane, gained 16 % where there are tens of thousands of such vertices and lost 80 % where
 // there are a few (one warp then takes 27 us for one).  Labels brought in by asynchronous
 // copies, the next tile's during the sort, were slower (4-byte copies run at half the rate
