@@ -1024,11 +1024,14 @@ int Engine::setup_fused(cudaStream_t st)
     fused_threads = narrow ? kFusedNarrow : kFusedWide;
     fused_smem = std::max(narrow ? kFusedSmem<kFusedNarrow> : kFusedSmem<kFusedWide>,
                           sizeof(unsigned long long) * (size_t)fused_slots);
-    fused_kernel = batched ? (narrow ? fused_run_kernel<true, kFusedNarrow> : fused_run_kernel<true, kFusedWide>)
-                           : (narrow ? fused_run_kernel<false, kFusedNarrow> : fused_run_kernel<false, kFusedWide>);
     int64_t tiles = (sc.nsv + 31) / 32 + ncta;
     for (int g = 1; g <= 5; ++g) tiles += (sc.gcut[g] - sc.gcut[g - 1] + (32 >> g) - 1) / (32 >> g);
     fused_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, std::min(sms, kFusedMaxBlocks)));
+    const int64_t chunk = (n + fused_blocks - 1) / fused_blocks;
+    fused_kernel = !batched ? (narrow ? fused_run_kernel<false, kFusedNarrow, 1> : fused_run_kernel<false, kFusedWide, 2>)
+                   : chunk > 2 * kFusedNarrow ? fused_run_kernel<true, kFusedNarrow, 3>
+                   : chunk > kFusedNarrow     ? fused_run_kernel<true, kFusedNarrow, 2>
+                                              : fused_run_kernel<true, kFusedNarrow, 1>;
     fused_cluster = 0;
     if (narrow && !ncta && tiles <= kFusedClusterTiles) {
         fused_blocks = 1;

@@ -23,7 +23,7 @@
 // graphs bound by the balance between the blocks: the other tiles are claimed from the list.
 // Passes of ten iterations, tiles dealt out in fixed order, each kind by itself and gathered by the
 // separate kernels' code -> this (us): planted partitions of 10 K entries 158 -> 124 (115 as a cluster), 294 K 230 ->
-// 160; R-MAT 16 423 -> 342; LFR of 560 K entries 309 -> 200; batch of 96 graphs 432 -> 400.
+// 160; R-MAT 16 423 -> 342; LFR of 560 K entries 309 -> 200; batch of 96 graphs 432 -> 400 (372 with three rows per round).
 //
 // Labels, change counts, run counts and the dispatch log are those of the separate kernels.
 #pragma once
@@ -51,10 +51,11 @@ constexpr int kFusedMaxBlocks = 256;
 // 1846; 1.5 M vertices with 7.5 M entries 1367 and 1446, with 21 M (LFR) 2386 and 2165.  Batches,
 // whose separate kernels are one CUDA-graph launch (the context's first pass, with the capture, and
 // a later one): 16 graphs with 312 K entries 440 / 286 and 234 / 197, 96 graphs with 738 K entries
-// 478 / 319 and 341 / 296, 96 with 1.8 M 600 / 383 and 467 / 400, 1,000 with 3.9 M 665 and 877 later.
+// 478 / 319 and 341 / 296, 96 with 1.8 M 600 / 383 and 444 / 372, 1,000 with 3.9 M 665 and 877 later.
 constexpr int64_t kFusedMaxEntries = 1 << 25, kFusedMaxVertices = 1 << 21;
 constexpr int64_t kFusedAnyVertices = 1 << 20, kFusedDense = 8;
 constexpr int64_t kFusedMaxBatchEntries = 1 << 21;
+static_assert(kFusedMaxBatchEntries <= kFusedNarrowEntries, "batches have the narrow shape only");
 // Runs of up to kFusedClusterTiles tiles, all small or lane-group ones, are one thread-block cluster:
 // its hardware barrier replaces the counter in global memory (0.6 us less each), and the launch is
 // not cooperative.  One block per tile and the counter against the cluster (us): 512 vertices with
@@ -129,10 +130,10 @@ __device__ __forceinline__ bool grid_barrier(FusedState *st, Ctl *ctl, int *fail
 
 // Dynamic shared memory: the warps' tile buffers, or the block's hash table, or the resolve
 // phase's buffers.
-template <int THREADS>
+template <int THREADS, int ROWS>
 struct FusedResolve {
     static constexpr int kWarps = THREADS / 32;
-    static constexpr int kPer = THREADS > 512 ? 2 : 1;  // vertices per thread and round
+    static constexpr int kPer = ROWS;  // vertices per thread and round
     static constexpr int kRound = kPer * THREADS;
     int hist[kWarps][256];
     long long qa[kRound];   // queue of tied vertices above 32 neighbours: run base,
@@ -152,8 +153,8 @@ constexpr int kFusedPlan = THREADS > kFusedNarrow ? 0 : 16;
 template <int THREADS>
 constexpr size_t kFusedSmem =
     kFusedTiles<THREADS> + (kFusedPlan<THREADS> ? sizeof(int32_t) * kPlanWords * (THREADS / 32) : 0);
-static_assert(sizeof(FusedResolve<kFusedNarrow>) <= kFusedTiles<kFusedNarrow> &&
-                  sizeof(FusedResolve<kFusedWide>) <= kFusedTiles<kFusedWide>,
+static_assert(sizeof(FusedResolve<kFusedNarrow, 3>) <= kFusedTiles<kFusedNarrow> &&
+                  sizeof(FusedResolve<kFusedWide, 2>) <= kFusedTiles<kFusedWide>,
               "the resolve buffers fit the tile buffers");
 
 // State of a vertex in the resolve phase, loaded in one round trip whether it is tied or not.
@@ -163,10 +164,16 @@ struct FusedVertex {
     int64_t o0;
 };
 
-template <bool BATCH, int kFusedThreads>
+// ROWS: vertices per thread and round of the resolve phase.  A round is a chain of loads, scans and
+// block barriers (about 5,000 cycles in batches), and rows beyond the block's vertices are paid for
+// too: batches in the narrow shape take the rows that their chunk of vertices fills, up to three.
+// One row against two or three (us): 96 graphs with 156 K vertices (1,030 a block) 400 and 369,
+// 200 graphs with 130 K (858) 351 and 340; with rows to spare 96 graphs with 22 K (142) 186, 195
+// and 212.
+template <bool BATCH, int kFusedThreads, int ROWS>
 __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a)
 {
-    using Resolve = FusedResolve<kFusedThreads>;
+    using Resolve = FusedResolve<kFusedThreads, ROWS>;
     constexpr int kFusedWarps = Resolve::kWarps, kPer = Resolve::kPer, kRound = Resolve::kRound;
     extern __shared__ __align__(16) unsigned char fused_smem[];
     __shared__ GroupTiles T;

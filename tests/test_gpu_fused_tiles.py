@@ -71,3 +71,26 @@ def test_cluster(n):
     rng = np.random.default_rng(n)
     _check(rng.integers(0, 20, n), n, niter=9)
     _check(np.concatenate([rng.integers(0, 20, n), rng.integers(33, 1025, 9)]), n + 1, niter=9)
+
+
+@pytest.mark.parametrize("sizes", [[511] * 152, [513] * 152, [700, 30, 1] * 151 + [5000], [1024] * 152, [1030] * 152,
+                                   [1, 60, 4000] * 58, [2000] * 152])
+def test_batch_rows(sizes):
+    # one, two and three vertices per thread and round, several rounds; graphs that end early
+    rng = np.random.default_rng(len(sizes) + sizes[0])
+    gs = []
+    for i, n in enumerate(sizes):
+        deg = rng.integers(0, 9, n) if i % 3 else np.full(n, min(n, 4))
+        off = np.zeros(n + 1, np.int64)
+        off[1:] = np.cumsum(deg)
+        gs.append(galp_gb300.Graph(off, rng.integers(0, max(n // (1 + i % 4), 1), off[-1]).astype(np.int32)))
+    with galp_gb300.Batch(gs) as b:
+        for k in (1, 6):
+            before = tools.schedule_info(b).launches
+            b.run(k)
+            assert tools.schedule_info(b).launches - before == 1
+            for i, g in enumerate(gs):
+                it, want, counts = oracle.run_par(g.offsets, g.neighbors, k)
+                got_it, got = b.graph_stats(i)
+                assert np.array_equal(b.labels(i), want), f"graph {i} of {k}"
+                assert got_it == it and got == list(counts)
