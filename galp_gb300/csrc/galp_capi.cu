@@ -979,7 +979,7 @@ DispatchArgs Engine::dispatch_args(int it) const
 bool Engine::fused_fits() const
 {
     if (policy != 0 || n < 1 || n > kFusedMaxVertices || !sched.big_v.empty()) return false;
-    if (batched) return G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries;
+    if (batched) return G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries && n <= kFusedMaxBatchVertices;
     return m <= kFusedMaxEntries && (n <= kFusedAnyVertices || m >= kFusedDense * n);
 }
 
@@ -1020,7 +1020,7 @@ int Engine::setup_fused(cudaStream_t st)
     const Scope &sc = sched.scopes[0];
     const int nmid = sc.nms + sc.nml + sc.nmx, ncta = nmid - sc.gcut[5];
     fused_slots = ncta ? std::min(kXlSlots, 4 * ((sched.mid_deg[(size_t)(sc.m0 + nmid - 1)] + 31) & ~31)) : 0;
-    const bool narrow = m <= kFusedNarrowEntries;
+    const bool narrow = batched || m <= kFusedNarrowEntries;
     fused_threads = narrow ? kFusedNarrow : kFusedWide;
     fused_smem = std::max(narrow ? kFusedSmem<kFusedNarrow> : kFusedSmem<kFusedWide>,
                           sizeof(unsigned long long) * (size_t)fused_slots);

@@ -39,7 +39,7 @@ namespace galp {
 // partitions of 3.8 M entries 454 -> 519).  512 against 768 threads (us): R-MAT 16 (1.8 M) 342 and
 // 380, LFR of 1.9 M 357 and 362, R-MAT 18 with edge factor 4 (2.0 M) 437 and 436, planted partitions
 // of 3.8 M 466 and 454, LFR of 5.5 M 691 and 663.
-constexpr int kFusedNarrow = 512, kFusedWide = 768;
+constexpr int kFusedNarrow = 512, kFusedWide = 768;  // batches: always narrow
 constexpr int64_t kFusedNarrowEntries = 1 << 21;
 constexpr int kFusedMaxBlocks = 256;
 // Up to these sizes a run is one kernel (above kFusedAnyVertices only with kFusedDense entries per
@@ -49,13 +49,14 @@ constexpr int kFusedMaxBlocks = 256;
 // of 5.5 M entries 916 and 663, 18 M 1964 and 1768, 24 M (700 K vertices) 2131 and 1865; planted
 // partitions of a million vertices with 5 M entries 1078 and 1071, 15 M 1516 and 1458, 25 M 1825 and
 // 1846; 1.5 M vertices with 7.5 M entries 1367 and 1446, with 21 M (LFR) 2386 and 2165.  Batches,
-// whose separate kernels are one CUDA-graph launch (the context's first pass, with the capture, and
-// a later one): 16 graphs with 312 K entries 440 / 286 and 234 / 197, 96 graphs with 738 K entries
-// 478 / 319 and 341 / 296, 96 with 1.8 M 600 / 383 and 444 / 372, 1,000 with 3.9 M 665 and 877 later.
+// whose separate kernels are one CUDA-graph launch and whose resolve phase does more per vertex (the
+// context's first pass, with the capture, and a later one): 16 graphs with 312 K entries 440 / 286
+// and 234 / 197, 96 with 1.8 M (156 K vertices) 600 / 383 and 444 / 372, 100 with 3.7 M (202 K)
+// 939 / 612 and 606 / 523, 60 with 3.4 M (254 K) 818 / 581 and 633 / 562; above the vertex limit
+// 220 with 3.2 M (278 K) 678 / 478 and 657 / 567, 300 with 1.7 M (362 K) 1113 / 480 and 761 / 572.
 constexpr int64_t kFusedMaxEntries = 1 << 25, kFusedMaxVertices = 1 << 21;
 constexpr int64_t kFusedAnyVertices = 1 << 20, kFusedDense = 8;
-constexpr int64_t kFusedMaxBatchEntries = 1 << 21;
-static_assert(kFusedMaxBatchEntries <= kFusedNarrowEntries, "batches have the narrow shape only");
+constexpr int64_t kFusedMaxBatchEntries = 1 << 22, kFusedMaxBatchVertices = 1 << 18;
 // Runs of up to kFusedClusterTiles tiles, all small or lane-group ones, are one thread-block cluster:
 // its hardware barrier replaces the counter in global memory (0.6 us less each), and the launch is
 // not cooperative.  One block per tile and the counter against the cluster (us): 512 vertices with

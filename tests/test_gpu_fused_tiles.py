@@ -74,7 +74,7 @@ def test_cluster(n):
 
 
 @pytest.mark.parametrize("sizes", [[511] * 152, [513] * 152, [700, 30, 1] * 151 + [5000], [1024] * 152, [1030] * 152,
-                                   [1, 60, 4000] * 58, [2000] * 152])
+                                   [1, 60, 4000] * 58, [1700] * 152])
 def test_batch_rows(sizes):
     # one, two and three vertices per thread and round, several rounds; graphs that end early
     rng = np.random.default_rng(len(sizes) + sizes[0])
@@ -94,3 +94,18 @@ def test_batch_rows(sizes):
                 got_it, got = b.graph_stats(i)
                 assert np.array_equal(b.labels(i), want), f"graph {i} of {k}"
                 assert got_it == it and got == list(counts)
+
+
+@pytest.mark.parametrize("n, deg, one", [((1 << 18) // 64, 16, True), ((1 << 18) // 64, 17, False),
+                                         ((1 << 18) // 64 + 1, 3, False)])
+def test_batch_size_rule(n, deg, one):
+    rng = np.random.default_rng(n + deg)
+    gs = [galp_gb300.Graph(np.arange(n + 1, dtype=np.int64) * deg, rng.integers(0, n // 2, n * deg).astype(np.int32))
+          for _ in range(64)]
+    with galp_gb300.Batch(gs, early_exit=0) as b:
+        before = tools.schedule_info(b).launches
+        b.run(3)
+        assert (tools.schedule_info(b).launches - before == 1) == one
+        for i, g in enumerate(gs):
+            _, want, counts = oracle.run_par(g.offsets, g.neighbors, 3, early_exit=False)
+            assert np.array_equal(b.labels(i), want) and b.graph_stats(i)[1] == list(counts)
