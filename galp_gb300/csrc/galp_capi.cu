@@ -1425,15 +1425,15 @@ int galp_enqueue(galp_ctx *ctx, int32_t niter)
     if (rc) return rc;
     GALP_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->pending = true;
+    ctx->have_labels = false;  // the host's copy is an older run's
     ctx->last_niter = niter;
     return GALP_OK;
 }
 
-int galp_sync(galp_ctx *ctx, galp_stats *st)
+// Wait for the enqueued runs and read the last one's iterations, change counts and errors.
+static int settle(galp_ctx *ctx, Ctl &c)
 {
-    if (!ctx) return GALP_EINVAL;
     GALP_CUDA(cudaStreamSynchronize(ctx->stream));
-    Ctl c;
     GALP_CUDA(cudaMemcpy(&c, ctx->eng.b_ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost));
     // a hub partition overflowed (its pairs were dropped): redo the run with twice the
     // partitions, up to 64x the default count (the labels of the redone run are exact)
@@ -1449,6 +1449,23 @@ int galp_sync(galp_ctx *ctx, galp_stats *st)
     ctx->err = c.err;
     ctx->runs_last = c.N;
     for (int i = 0; i < GALP_MAX_ITERS; ++i) ctx->counts[i] = (int64_t)c.counts[i];
+    return GALP_OK;
+}
+
+// Before results of the last run are read: a run enqueued since the last galp_sync counts (which
+// still reports its statistics and errors).
+static int settle_pending(galp_ctx *ctx)
+{
+    if (!ctx->pending) return GALP_OK;
+    Ctl c;
+    return settle(ctx, c);
+}
+
+int galp_sync(galp_ctx *ctx, galp_stats *st)
+{
+    if (!ctx) return GALP_EINVAL;
+    Ctl c;
+    if (const int rc = settle(ctx, c)) return rc;
     float ms = 0.f;
     if (ctx->pending) cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     ctx->pending = false;
@@ -1500,6 +1517,7 @@ int galp_get_labels(galp_ctx *ctx, int32_t *out, int64_t n)
     if (!ctx || n != ctx->n || (!out && n > 0)) return GALP_EINVAL;
     if (!ctx->have_labels) {
         // labels of the last enqueued run, if any, else the initial labels
+        if (const int rc = settle_pending(ctx)) return rc;
         const int32_t *src = ctx->eng.final_labels(ctx->iters);
         GALP_CUDA(cudaStreamSynchronize(ctx->stream));
         if (n) GALP_CUDA(cudaMemcpy(out, src, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
@@ -1633,6 +1651,7 @@ int galp_dispatch_log(galp_ctx *ctx, float *features, int32_t *variants, int32_t
 {
     if (!ctx || !count || cap_iters < 0) return GALP_EINVAL;
     galp::Engine &E = ctx->eng;
+    if (const int rc = settle_pending(ctx)) return rc;
     GALP_CUDA(cudaStreamSynchronize(ctx->stream));
     const int nlog = std::min(std::min(ctx->iters, (int)galp::kMaxLogIters), (int)cap_iters);
     *count = nlog;
@@ -1713,6 +1732,7 @@ int galp_batch_labels(galp_ctx *ctx, int32_t graph, int32_t *labels, int64_t n)
     galp::Engine &E = ctx->eng;
     const int64_t v0 = E.g_v0_h[graph], v1 = E.g_v0_h[graph + 1];
     if (n != v1 - v0 || (n > 0 && !labels)) return GALP_EINVAL;
+    if (const int rc = settle_pending(ctx)) return rc;
     GALP_CUDA(cudaStreamSynchronize(ctx->stream));
     if (n) GALP_CUDA(cudaMemcpy(labels, E.final_labels(ctx->iters) + v0, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
     return GALP_OK;
