@@ -32,6 +32,7 @@
 #include <utility>
 
 #include "rmat_rng.h"
+#include "lp_index.h"
 #include "lp_kernels.cuh"
 #include "lp_dispatch.cuh"
 
@@ -995,20 +996,19 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
     unsigned long long changes = 0;
     // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
     // window in turn, so that none has only the window's highest degrees
-    const int stride = gridDim.x * kSmallThreads;
-    int base = blockIdx.x * kSmallThreads;  // block-uniform
+    ListWalk walk(blockIdx.x, gridDim.x, kSmallThreads, p.nsmall);
     int turn = w;
-    auto ahead = [&](int from) {
+    auto head = [&](int rounds) {
         TileHead h{-1, 0, 0, 0, 0, 1};
-        const int i = from + turn * 32 + lane;
-        if (i < p.nsmall) tile_head<false>(p, h, p.small_v[i], fr);
+        const int i = walk.entry(rounds, turn * 32 + lane);
+        if (i >= 0) tile_head<false>(p, h, p.small_v[i], fr);
         turn = (turn + 1) & (NW - 1);
         return h;
     };
-    TileHead nxt = ahead(base);
-    for (; base < p.nsmall; base += stride) {
+    TileHead nxt = head(0);
+    for (; walk.more(); walk.next()) {
         const TileHead hd = nxt;
-        nxt = ahead(base + stride);
+        nxt = head(1);
         bool chg;
         int d = small_tile<false>(p, stile[w], hd, changes, chg);
         if (!hd.dirty) d = p.dcnt[hd.v];
@@ -2459,7 +2459,7 @@ __global__ void __launch_bounds__(kTB) mark_dirty_kernel(const int64_t *off, con
     const bool dense = !disp->frontier;
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->frontier_off = dense ? 1 : 0;
     if (dense) return;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += (gridDim.x * blockDim.x) >> 5) {
+    for (int64_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += (gridDim.x * blockDim.x) >> 5) {
         const int u = changed[i];
         const int64_t e0 = off[u], e1 = off[u + 1];
         for (int64_t e = e0 + lane; e < e1; e += 32) dirty[nbr[e]] = 1;
