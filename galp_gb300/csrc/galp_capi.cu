@@ -489,6 +489,7 @@ int Engine::setup(const galp_csr &g, const galp_opts &o, cudaStream_t st, int64_
     GALP_CUDA(b_lab0.alloc(sizeof(int32_t) * std::max<int64_t>(n, 1)));
     GALP_CUDA(b_lab1.alloc(sizeof(int32_t) * std::max<int64_t>(n, 1)));
     GALP_CUDA(b_ctl.alloc(sizeof(Ctl)));
+    GALP_CUDA(cudaMemsetAsync(b_ctl.p, 0, sizeof(Ctl), st));
     const size_t nbig = sched.big_v.size();
     GALP_CUDA(b_bstat.alloc(sizeof(BigStat) * std::max<size_t>(nbig, 1)));
     GALP_CUDA(b_big_a.alloc(sizeof(int64_t) * std::max<size_t>(nbig, 1)));
@@ -1058,7 +1059,8 @@ int Engine::setup_fused(cudaStream_t st)
 // The barriers and sums of one-kernel runs as the first run finds them.
 int Engine::reset_fused(cudaStream_t st)
 {
-    GALP_CUDA(cudaMemsetAsync(b_fused.p, 0, b_fused.bytes, st));
+    if (b_fused.p) GALP_CUDA(cudaMemsetAsync(b_fused.p, 0, b_fused.bytes, st));
+    GALP_CUDA(cudaMemsetAsync(&((Ctl *)b_ctl.p)->gave_up, 0, sizeof(int), st));
     return GALP_OK;
 }
 
@@ -1080,6 +1082,8 @@ int Engine::enqueue_run_fused(cudaStream_t st, int niter, long long thr)
     a.chunk = (int)((n + fused_blocks - 1) / fused_blocks);
     a.slots = fused_slots;
     a.agg_mode = variant.agg_mode;
+    a.spin_limit = fused_spin;
+    a.more = fused_more;
     a.pieces = kFusedMaxBlocks + (batched ? G : 1);
     a.sums = (long long *)((FusedState *)b_fused.p + 1);
     if (batched) {
@@ -1445,6 +1449,7 @@ static int settle(galp_ctx *ctx, Ctl &c)
         GALP_CUDA(cudaStreamSynchronize(ctx->stream));
         GALP_CUDA(cudaMemcpy(&c, ctx->eng.b_ctl.p, sizeof(Ctl), cudaMemcpyDeviceToHost));
     }
+    if (c.gave_up) c.err |= kErrLookback;  // in this run or in one enqueued before it
     ctx->iters = c.iter;
     ctx->err = c.err;
     ctx->runs_last = c.N;
@@ -1478,7 +1483,7 @@ int galp_sync(galp_ctx *ctx, galp_stats *st)
         st->runs_last = c.N;
         for (int i = 0; i < GALP_MAX_ITERS; ++i) st->updates[i] = (int64_t)c.counts[i];
     }
-    if ((c.err & kErrLookback) && ctx->eng.b_fused.p) {  // barriers given up half-way
+    if (c.gave_up) {  // barriers and sums left half-way
         const int rc = ctx->eng.reset_fused(ctx->stream);
         if (rc) return rc;
     }
@@ -1537,6 +1542,14 @@ void galp_destroy(galp_ctx *ctx)
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
+}
+
+int galp_debug_barrier(galp_ctx *ctx, int64_t spin_limit, int32_t wait_unset)
+{
+    if (!ctx) return GALP_EINVAL;
+    ctx->eng.fused_spin = spin_limit > 0 ? (long long)spin_limit : kFusedSpinLimit;
+    ctx->eng.fused_more = wait_unset ? 1 : 0;
+    return GALP_OK;
 }
 
 int galp_probe_gather(galp_ctx *ctx, int32_t reps, float *ms_per_pass)

@@ -212,6 +212,8 @@ struct Engine {
     int fused_blocks = 0, fused_threads = 0, fused_slots = 0;
     int fused_cluster = 0;  // blocks of the one cluster that the grid is, or 0
     size_t fused_smem = 0;
+    long long fused_spin = kFusedSpinLimit;  // galp_debug_barrier
+    unsigned fused_more = 0;
     DevBuf b_static_feat, b_vtab, b_disp, b_feat_log, b_var_log, b_weights;  // dispatch
     float static_feat[kDegBins + 3] = {};
     std::vector<DispatchState> vtab;   // variant table of the in-core scope

@@ -68,8 +68,9 @@ constexpr int kFusedClusterBlocks = 16, kFusedClusterTiles = 64;
 constexpr int kFusedMaxGraphs = 4096;
 constexpr long long kFusedSpinLimit = 1ll << 21;  // polls of a barrier wait (about a second)
 
-// Device memory of the run's barriers and sums, zero before the first run (every run leaves it
-// so, except after an error).
+// Device memory of the run's barriers and sums, zero before the first run.  Every run leaves it so,
+// except one whose wait ran out (Ctl::gave_up): runs enqueued behind it return at once, and
+// galp_sync clears both.
 struct FusedState {
     unsigned arrived;                        // blocks that have reached a barrier of this run
     unsigned left;                           // blocks that have ended it
@@ -93,6 +94,8 @@ struct FusedArgs {
     int slots;                // table slots for vertices above kGroupMax
     int agg_mode;
     int cluster;              // the grid is one cluster
+    long long spin_limit;     // polls before a barrier wait gives up
+    unsigned more;            // arrivals awaited beyond the blocks' own (0; tests only)
     // batches
     unsigned long long *g_changes;  // [3][graphs]: labels changed, likewise
     int32_t *g_active, *g_iters;
@@ -100,28 +103,29 @@ struct FusedArgs {
     int g_max_iter, early_exit;
 };
 
-// The run's k-th barrier (k = 1, 2, ...) of all blocks; false when the wait ran out
-// (kErrLookback is set, and the block must return: the others give up in the same way).  In a run
+// The run's k-th barrier (k = 1, 2, ...) of all blocks; false when the wait ran out (Ctl::gave_up
+// is set, and the block must return: the others give up in the same way).  In a run
 // that is one cluster no wait can run out: all its blocks are resident, and none returns early.  The
 // arrivals only count up, so a block waits for one number and nobody resets anything until the
 // last block leaves the run.
-__device__ __forceinline__ bool grid_barrier(FusedState *st, Ctl *ctl, int *failed, unsigned k, int cluster)
+__device__ __forceinline__ bool grid_barrier(const FusedArgs &a, Ctl *ctl, int *failed, unsigned k)
 {
-    if (cluster) {
+    FusedState *st = a.state;
+    if (a.cluster) {
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
         return true;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->arrived) : "memory");
-        const unsigned want = k * gridDim.x;
+        const unsigned want = k * gridDim.x + a.more;
         unsigned now = 0;
         long long i = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&st->arrived) : "memory");
-        } while (now < want && ++i < kFusedSpinLimit);
+        } while (now < want && ++i < a.spin_limit);
         if (now < want) {
-            atomicOr(&ctl->err, kErrLookback);
+            atomicExch(&ctl->gave_up, 1);
             *failed = 1;
         }
     }
@@ -193,12 +197,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
     FusedTile *tiles = reinterpret_cast<FusedTile *>(fused_smem);
     const BlockRed5<kFusedThreads> br{red, red2};
     if (tid == 0) {
-        failed = 0;
+        failed = *(volatile int *)&ctl->gave_up;
         T.set(p, p.gcut[5]);
     }
     if (b == 0) {  // the run's bookkeeping: nobody else touches it before the first barrier
         if (tid == 0) {
+            ctl->active = 0;
+            ctl->iter = 0;
             ctl->err = 0;
+            ctl->N = 0;
             ctl->thr = a.thr;
             ctl->max_iter = a.niter;
             ctl->ticket = 0;
@@ -256,6 +263,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
     };
     unsigned barriers = 0;
     __syncthreads();
+    if (failed) return;  // a run before this one left the barriers and sums half-way
     // tiles: the lane groups' (largest degrees first), then the small vertices'.  Every warp of a
     // block without vertices above kGroupMax has its first tile fixed, consecutive ones on different
     // blocks, with its vertices and offsets in registers for all iterations; the other tiles are
@@ -288,7 +296,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             plan[j * 32 + lane] = j < n && j < cnt ? __ldg(&p.nbr[head0.o0 - p.nbr_shift + first + j]) : -1;
         __syncwarp();
     }
-    if (!a.shortcut && !grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;  // labels gathered by other blocks
+    if (!a.shortcut && !grid_barrier(a, ctl, &failed, ++barriers)) return;  // labels gathered by other blocks
     int it = 0;
     long long runs = 0, last_changes = 0;
     for (;;) {
@@ -414,7 +422,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 if (tid == 0 && sruns) atomicAdd(&st->runs[it % 3], sruns);
             }
         }
-        if (!grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;
+        if (!grid_barrier(a, ctl, &failed, ++barriers)) return;
         // entries of the iterations to come: their last readers passed the barrier before this one
         {
             long long *later = a.sums + (size_t)((it + 2) % 3) * a.pieces;
@@ -616,7 +624,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(kFull, c, o);
             if (lane == 0 && c) atomicAdd(&st->changes[it % 3], c);
         }
-        if (!grid_barrier(st, ctl, &failed, ++barriers, a.cluster)) return;
+        if (!grid_barrier(a, ctl, &failed, ++barriers)) return;
         last_changes = (long long)*((volatile unsigned long long *)&st->changes[it % 3]);
         if (b == 0 && tid == 0 && it < 64) ctl->counts[it] = (unsigned long long)last_changes;
         ++it;
@@ -648,7 +656,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             st->arrived = 0;
         }
         if (b == 0) {
-            ctl->active = 0;
             ctl->iter = it;
             ctl->N = runs;
             // (st->runs of other blocks' last read lies before the last barrier)

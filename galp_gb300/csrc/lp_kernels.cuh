@@ -55,7 +55,7 @@ struct Ctl {
     int active;                 // 1 while iterations still run
     int iter;                   // iterations completed
     int err;                    // sticky error bits
-    int pad0;
+    int gave_up;                // a one-kernel run's wait ran out (until galp_sync has seen it)
     unsigned long long ticket;  // tile ticket of the running lp_tile_kernel
     unsigned long long changes; // labels changed in the current iteration
     long long N;                // runs in the scope (written by the tile of last_v)

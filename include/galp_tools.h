@@ -154,6 +154,12 @@ int galp_profile_kernels(galp_ctx *ctx, galp_kernel_stat *out, int32_t cap, int3
  * out and the call returns GALP_ETIMEOUT.  (0, 0) restores the defaults. */
 int galp_debug_noalloc_lookback(int64_t spin_limit, int32_t wait_unset);
 
+/* Test hook of the one-kernel runs' failure detection: every barrier wait of this context's later
+ * runs gives up after spin_limit polls (<= 0: the default bound), and with wait_unset != 0 the
+ * waits expect one more arrival than there are blocks, so that they run out and galp_sync returns
+ * GALP_ETIMEOUT.  Runs that are one cluster have no such wait.  (0, 0) restores the defaults. */
+int galp_debug_barrier(galp_ctx *ctx, int64_t spin_limit, int32_t wait_unset);
+
 /* Write nedges raw R-MAT edge keys (u << 32 | v) into device memory d_out, on
  * `stream` (cudaStream_t as void*), with the same sampler as galp_gen_rmat. */
 int galp_gen_rmat_keys_device(uint64_t seed, int32_t scale, int64_t nedges, double a, double b, double c,
