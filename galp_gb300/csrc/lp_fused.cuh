@@ -28,6 +28,7 @@
 // Labels, change counts, run counts and the dispatch log are those of the separate kernels.
 #pragma once
 
+#include "lp_index.h"
 #include "lp_pipeline.cuh"
 
 namespace galp {
@@ -118,13 +119,14 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs &a, Ctl *ctl, int *
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->arrived) : "memory");
-        const unsigned want = k * gridDim.x + a.more;
         unsigned now = 0;
+        bool waits;
         long long i = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&st->arrived) : "memory");
-        } while (now < want && ++i < a.spin_limit);
-        if (now < want) {
+            waits = barrier_waits(now - a.more, k, gridDim.x);
+        } while (waits && ++i < a.spin_limit);
+        if (waits) {
             atomicExch(&ctl->gave_up, 1);
             *failed = 1;
         }

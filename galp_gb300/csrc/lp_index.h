@@ -31,4 +31,12 @@ struct ListWalk {
     }
 };
 
+// Whether a barrier of `blocks` blocks, the k-th that a run comes to, still waits: `arrived` counts
+// every arrival of the run so far.  Both wrap around (152 blocks pass 2^32 arrivals after 14 M
+// iterations), and lie within one barrier of each other: the sign of their difference decides.
+GALP_INDEX bool barrier_waits(uint32_t arrived, uint32_t k, uint32_t blocks)
+{
+    return (int32_t)(arrived - k * blocks) < 0;
+}
+
 }  // namespace galp

@@ -30,6 +30,18 @@ WALK = """
     return puts("ok"), 0;
 """
 
+BARRIER = """
+    // barriers k ... of a run: arrivals before, at and up to one barrier after
+    const uint32_t k0 = (uint32_t)atoll(argv[1]), blocks = (uint32_t)atoll(argv[2]);
+    unsigned long long total = (unsigned long long)k0 * blocks;
+    for (uint32_t k = k0; k != k0 + 3; ++k, total += blocks)
+        for (uint32_t missing = 0; missing <= blocks; ++missing) {
+            if (barrier_waits((uint32_t)(total - missing), k, blocks) != (missing > 0)) return puts("waits"), 0;
+            if (barrier_waits((uint32_t)(total + missing), k, blocks)) return puts("closed"), 0;
+        }
+    return puts("ok"), 0;
+"""
+
 
 @pytest.fixture(scope="module")
 def program(tmp_path_factory):
@@ -58,3 +70,11 @@ def program(tmp_path_factory):
 @pytest.mark.parametrize("blocks", [1, 152 * 8, 2048])
 def test_list_walk(program, n, blocks):
     assert program("walk", WALK)(n, blocks) == ["ok"]
+
+
+@pytest.mark.parametrize("blocks", [1, 16, 152, 256])
+@pytest.mark.parametrize("k", [1, 2, 1000, 2**31 // 152, 2**32 // 152, 2**32 // 152 - 2, 2**32 // 256 - 1,
+                               2**32 // 16 - 1, 2**32 // 16, 2**32 - 2])
+def test_barrier_count_wraps(program, k, blocks):
+    # a run without early exit has two barriers an iteration and as many iterations as asked for
+    assert program("barrier", BARRIER)(k, blocks) == ["ok"]
