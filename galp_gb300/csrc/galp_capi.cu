@@ -14,9 +14,11 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <new>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/galp.h"
@@ -54,6 +56,34 @@ int cuda_status(cudaError_t e)
     } while (0)
 
 namespace {
+
+// part(t) for every t in [0, T), on T - 1 threads of their own and this one.  Where no thread (or
+// memory for one) is to be had, this one does the rest; an exception of a part is thrown on when
+// all have ended.
+template <class F>
+void run_parts(int T, F &&part)
+{
+    std::vector<std::thread> th;
+    std::vector<std::exception_ptr> failed;
+    auto guarded = [&](int t) {
+        try {
+            part(t);
+        } catch (...) {
+            failed[(size_t)t] = std::current_exception();
+        }
+    };
+    failed.resize((size_t)T);
+    int started = 1;
+    try {
+        for (; started < T; ++started) th.emplace_back(guarded, started);
+    } catch (...) {
+    }
+    guarded(0);
+    for (int t = started; t < T; ++t) guarded(t);
+    for (auto &x : th) x.join();
+    for (const std::exception_ptr &e : failed)
+        if (e) std::rethrow_exception(e);
+}
 
 // One thread's share of a scope: packs, mid-list vertices (unsorted), big vertices.
 struct ChunkPlan {
@@ -180,15 +210,7 @@ bool build_schedule(Schedule &S, int64_t n, const int64_t *off, const std::vecto
         // planned one after the other, most of them below it)
         const int T = nv >= (1 << 18) ? (int)std::min<int64_t>(hw, nv >> 15) : 1;
         std::vector<ChunkPlan> plans(T);
-        {
-            std::vector<std::thread> th;
-            for (int t = 0; t < T; ++t) {
-                const int64_t a = sc.v0 + nv * t / T, b = sc.v0 + nv * (t + 1) / T;
-                if (T == 1) plan_chunk(off, a, b, plans[t]);
-                else th.emplace_back(plan_chunk, off, a, b, std::ref(plans[t]));
-            }
-            for (auto &x : th) x.join();
-        }
+        run_parts(T, [&](int t) { plan_chunk(off, sc.v0 + nv * t / T, sc.v0 + nv * (t + 1) / T, plans[(size_t)t]); });
         int64_t nsmall = 0;
         std::vector<int32_t> big;
         size_t np = 0, nm = 0;
@@ -246,15 +268,14 @@ bool build_schedule(Schedule &S, int64_t n, const int64_t *off, const std::vecto
                     S.mid_deg[at] = P.mid_deg[i];
                 }
             };
-            std::vector<std::thread> th;
+            std::vector<std::pair<size_t, size_t>> at;  // each thread's first pack and small vertex
             size_t p0 = pb, s0 = sb;
-            for (int t = 0; t < T; ++t) {
-                if (T == 1) place(t, p0, s0);
-                else th.emplace_back(place, t, p0, s0);
-                p0 += plans[(size_t)t].pack_v0.size();
-                s0 += (size_t)plans[(size_t)t].nsmall;
+            for (const ChunkPlan &P : plans) {
+                at.push_back({p0, s0});
+                p0 += P.pack_v0.size();
+                s0 += (size_t)P.nsmall;
             }
-            for (auto &x : th) x.join();
+            run_parts(T, [&](int t) { place(t, at[(size_t)t].first, at[(size_t)t].second); });
         }
         {
             auto cut = [&](int t) {  // mid-list entries of degree <= t
