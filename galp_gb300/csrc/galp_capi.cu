@@ -1634,6 +1634,16 @@ int galp_schedule_info(galp_ctx *ctx, galp_sched_info *info)
     return GALP_OK;
 }
 
+// A batch's captured run is captured again: its kernels, grids or arguments have changed.
+static void drop_graph(galp_ctx *ctx)
+{
+    if (!ctx->graph_exec) return;
+    cudaStreamSynchronize(ctx->stream);  // its last launch
+    cudaGraphExecDestroy(ctx->graph_exec);
+    ctx->graph_exec = nullptr;
+    ctx->graph_iters = -1;
+}
+
 int galp_set_variant(galp_ctx *ctx, const galp_variant *v)
 {
     if (!ctx || !v || v->agg_mode < 0 || v->agg_mode > 2 || !(v->frontier_frac >= 0.f && v->frontier_frac <= 1.f) ||
@@ -1649,10 +1659,7 @@ int galp_set_variant(galp_ctx *ctx, const galp_variant *v)
         if (rc) return rc;
     }
     ctx->eng.variant = *v;
-    // a batched run is a captured CUDA graph: capture again with the new kernels
-    if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-    ctx->graph_exec = nullptr;
-    ctx->graph_iters = -1;
+    drop_graph(ctx);
     return GALP_OK;
 }
 
@@ -1678,6 +1685,7 @@ int galp_dispatch_set(galp_ctx *ctx, int32_t mode, int32_t forced_variant, const
     if (mode == 1 && !E.have_weights) return GALP_EINVAL;
     E.disp_mode = mode;
     E.disp_forced = forced_variant;
+    drop_graph(ctx);
     return GALP_OK;
 }
 
@@ -1886,9 +1894,7 @@ int galp_batch_tune(galp_ctx *ctx, int32_t niter, galp_tune_result *res)
     E.prof.spans[3].clear();
     E.prof.it_spans.clear();
     E.prof.used = 0;
-    if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);  // recapture with the chosen shapes
-    ctx->graph_exec = nullptr;
-    ctx->graph_iters = -1;
+    drop_graph(ctx);
     if (rc) return rc;
     if (res) {
         res->small_blocks_per_sm = E.small_bps;
