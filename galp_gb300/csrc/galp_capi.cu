@@ -1821,16 +1821,14 @@ int galp_run_batch(const galp_csr *graphs, int32_t count, const galp_opts *opts,
     return rc;
 }
 
-// Launch-shape autotuner for batched runs: coordinate descent over blocks per SM of the
-// small-vertex counting, mid-vertex counting and small-vertex resolve kernels, each
-// candidate timed on a probe run of niter iterations.
+// Launch-shape autotuner for batched runs.  First the run that the batch would take is timed as it
+// is, where that is one kernel; it has no shapes to choose.  Then, on the separate kernels, a
+// coordinate descent over the blocks per SM of the counting and resolve kernels that the batch
+// has, each candidate timed on a probe run of niter iterations.
 int galp_batch_tune(galp_ctx *ctx, int32_t niter, galp_tune_result *res)
 {
     if (!ctx || niter < 1) return GALP_EINVAL;
     galp::Engine &E = ctx->eng;
-    int *knob[3] = {&E.small_bps, &E.mid_bps, &E.resolve_bps};
-    const int cand[3][4] = {{8, 16, 24, 32}, {2, 4, 6, 8}, {2, 4, 8, 16}};
-    float best_ms = 0.f;
     int trials = 0;
     auto probe = [&](float &ms) -> int {  // best of two runs
         ms = 1e30f;
@@ -1845,47 +1843,70 @@ int galp_batch_tune(galp_ctx *ctx, int32_t niter, galp_tune_result *res)
         ++trials;
         return GALP_OK;
     };
+    int rc = GALP_OK;
+    float one_ms = 1e30f;
+    if (E.fused_run(ctx->stream, niter) && (rc = probe(one_ms))) return rc;
+    const bool one = E.fused_run(ctx->stream, niter);  // unless its launch was refused
     const bool was_on = E.prof.on;
-    E.prof.on = true;  // enqueue directly while probing (no graph capture)
+    E.prof.on = true;  // enqueue the separate kernels directly while probing (no graph capture)
     const int level = E.prof.level;
     E.prof.level = 0;
-    int rc = probe(best_ms);  // warm-up
+    float best_ms = 0.f;
+    rc = probe(best_ms);  // warm-up
     if (!rc) rc = probe(best_ms);
-    for (int k = 0; !rc && k < 3; ++k) {
-        int keep = *knob[k];
+    int64_t nmid = 0, ngroup = 0, ncta256 = 0;  // vertices above 32, up to 1024, of 1025..2048 neighbours
+    for (const galp::Scope &sc : E.sched.scopes) {
+        nmid += sc.nms + sc.nml + sc.nmx;
+        ngroup += sc.gcut[5];
+        ncta256 += sc.gcut[6] - sc.gcut[5];
+    }
+    struct Knob {
+        int *blocks;
+        int cand[4];
+        bool used;  // some kernel of this batch goes by it
+    };
+    const Knob knobs[3] = {{&E.small_bps, {8, 16, 24, 32}, E.variant.small_sort != 2},
+                           {&E.mid_bps, {2, 4, 6, 8}, ngroup > 0},
+                           {&E.resolve_bps, {2, 4, 8, 16}, nmid > 0}};
+    for (const Knob &k : knobs) {
+        if (!k.used) continue;
+        int keep = *k.blocks;
         for (int c = 0; !rc && c < 4; ++c) {
-            if (cand[k][c] == keep) continue;
-            const int old = *knob[k];
-            *knob[k] = cand[k][c];
+            if (k.cand[c] == *k.blocks) continue;  // timed already
+            const int old = *k.blocks;
+            *k.blocks = k.cand[c];
             float ms = 0.f;
             rc = probe(ms);
             if (!rc && ms < best_ms) {
                 best_ms = ms;
-                keep = cand[k][c];
+                keep = k.cand[c];
             }
-            *knob[k] = old;
+            *k.blocks = old;
         }
-        *knob[k] = keep;
+        *k.blocks = keep;
     }
-    // bucket shapes: the degree splits between warp and CTA counting (128 / 256) and
-    // between CTA sizes (1024 / 2048) and the insert aggregation, as fixed variant rows
-    // (frontier off); a row is kept only when it beats the per-iteration fixed rule by 1 %
+    // bucket shapes, as fixed variant rows (frontier off): the insert aggregation of vertices above
+    // 1024 neighbours and the CTA size of those up to 2048, where there are any; a row is kept only
+    // when it beats the per-iteration fixed rule, and the one-kernel run that it would end, by 1 %
     int best_row = -1;
-    if (!rc && !E.frontier) {
+    if (!rc && !E.frontier && nmid > ngroup) {
         const int mode0 = E.disp_mode, forced0 = E.disp_forced;
-        for (int row = 0; !rc && row < galp::kVar; row += 2) {
+        float to_beat = one ? std::min(one_ms, best_ms) : best_ms;
+        for (int row : {0, 2, 8, 10}) {
+            if (rc || ((row & 2) && !ncta256)) continue;
             E.disp_mode = 2;
             E.disp_forced = row;
             float ms = 0.f;
             rc = probe(ms);
-            if (!rc && ms < 0.99f * best_ms) {
-                best_ms = ms;
+            if (!rc && ms < 0.99f * to_beat) {
+                to_beat = best_ms = ms;
                 best_row = row;
             }
         }
         E.disp_mode = best_row >= 0 ? 2 : mode0;
         E.disp_forced = best_row >= 0 ? best_row : forced0;
     }
+    if (one && best_row < 0) best_ms = one_ms;  // the run that the batch goes on to take
     E.prof.on = was_on;
     E.prof.level = level;
     E.prof.spans[0].clear();
