@@ -1120,7 +1120,7 @@ int Engine::enqueue_run_fused(cudaStream_t st, int niter, long long thr)
     if (fused_cluster) {
         const cudaLaunchConfig_t cfg = fused_launch(st, attr);
         a.cluster = 1;
-        e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+        e = fused_refuse & 1 ? cudaErrorInvalidConfiguration : cudaLaunchKernelEx(&cfg, fused_kernel, a);
         if (e != cudaSuccess) {  // no room for the cluster (any more)
             (void)cudaGetLastError();
             fused_cluster = 0;
@@ -1129,7 +1129,7 @@ int Engine::enqueue_run_fused(cudaStream_t st, int niter, long long thr)
     }
     if (!a.cluster) {
         const cudaLaunchConfig_t cfg = fused_launch(st, attr);
-        e = cudaLaunchKernelEx(&cfg, fused_kernel, a);
+        e = fused_refuse & 2 ? cudaErrorCooperativeLaunchTooLarge : cudaLaunchKernelEx(&cfg, fused_kernel, a);
     }
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // not all of the device is ours
         (void)cudaGetLastError();
@@ -1570,6 +1570,13 @@ int galp_debug_barrier(galp_ctx *ctx, int64_t spin_limit, int32_t wait_unset)
     if (!ctx) return GALP_EINVAL;
     ctx->eng.fused_spin = spin_limit > 0 ? (long long)spin_limit : kFusedSpinLimit;
     ctx->eng.fused_more = wait_unset ? 1 : 0;
+    return GALP_OK;
+}
+
+int galp_debug_launch(galp_ctx *ctx, int32_t refuse)
+{
+    if (!ctx || refuse < 0 || refuse > 3) return GALP_EINVAL;
+    ctx->eng.fused_refuse = refuse;
     return GALP_OK;
 }
 

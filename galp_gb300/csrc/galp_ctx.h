@@ -214,6 +214,7 @@ struct Engine {
     size_t fused_smem = 0;
     long long fused_spin = kFusedSpinLimit;  // galp_debug_barrier
     unsigned fused_more = 0;
+    int fused_refuse = 0;  // galp_debug_launch
     DevBuf b_static_feat, b_vtab, b_disp, b_feat_log, b_var_log, b_weights;  // dispatch
     float static_feat[kDegBins + 3] = {};
     std::vector<DispatchState> vtab;   // variant table of the in-core scope

@@ -161,6 +161,11 @@ int galp_debug_noalloc_lookback(int64_t spin_limit, int32_t wait_unset);
  * GALP_ETIMEOUT.  Runs that are one cluster have no such wait.  (0, 0) restores the defaults. */
 int galp_debug_barrier(galp_ctx *ctx, int64_t spin_limit, int32_t wait_unset);
 
+/* Test hook of the one-kernel runs' launch: this context's later runs find their cluster launch (1),
+ * their cooperative launch (2) or both (3) refused, as on a device that another program occupies;
+ * 0 restores the launches. */
+int galp_debug_launch(galp_ctx *ctx, int32_t refuse);
+
 /* Write nedges raw R-MAT edge keys (u << 32 | v) into device memory d_out, on
  * `stream` (cudaStream_t as void*), with the same sampler as galp_gen_rmat. */
 int galp_gen_rmat_keys_device(uint64_t seed, int32_t scale, int64_t nedges, double a, double b, double c,
