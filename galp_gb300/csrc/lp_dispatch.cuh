@@ -84,8 +84,7 @@ __device__ __forceinline__ void dispatch_step(const DispatchArgs &a)
     __shared__ float x[kFeat], h1[kHid], h2[kHid], y[kVar];
     __shared__ int pick;
     const int t = threadIdx.x;
-    if (t < kFeat)
-        x[t] = dispatch_feature(a, t, a.it, a.it > 0 ? (long long)a.ctl->counts[a.it - 1] : 0, a.ctl->N);
+    if (t < kFeat) x[t] = dispatch_feature(a, t, a.it, (long long)a.ctl->last, a.ctl->N);
     __syncthreads();
     if (t == 0) {
         int v;

@@ -62,7 +62,8 @@ struct Ctl {
     long long thr;              // early-exit threshold: stop when changes <= thr
     int max_iter;               // iterations requested
     int pad1;
-    unsigned long long counts[64];  // changes per iteration
+    unsigned long long counts[64];  // changes per iteration (the first 64)
+    unsigned long long last;    // changes of the last iteration
     int tied_mid;               // tied vertices above 32 neighbours (per scope)
     int pad2;
     int changed_n;              // vertices whose label changed (frontier mode)
@@ -1124,6 +1125,7 @@ __device__ __forceinline__ void finalize_iteration(Ctl *ctl)  // one thread
 {
     if (ctl->active) {
         const unsigned long long c = ctl->changes;
+        ctl->last = c;
         if (ctl->iter < 64) ctl->counts[ctl->iter] = c;
         ctl->iter += 1;
         if ((long long)c <= ctl->thr || ctl->iter >= ctl->max_iter) ctl->active = 0;

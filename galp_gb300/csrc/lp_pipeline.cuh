@@ -2694,6 +2694,7 @@ __global__ void batch_finalize_kernel(Ctl *ctl, const int64_t *g_v0, int32_t *g_
     if (threadIdx.x == 0) {
         if (on) {
             const unsigned long long c = ctl->changes;
+            ctl->last = c;
             if (ctl->iter < 64) ctl->counts[ctl->iter] = c;
             ctl->iter += 1;
             if (!any || ctl->iter >= ctl->max_iter) ctl->active = 0;
