@@ -482,9 +482,10 @@ int Engine::setup(const galp_csr &g, const galp_opts &o, cudaStream_t st, int64_
     GALP_CUDA(b_run_lab.alloc(sizeof(int32_t) * ms));
     GALP_CUDA(b_run_cnt.alloc(sizeof(uint16_t) * ms));
     GALP_CUDA(b_tmid.alloc(sizeof(int32_t) * (size_t)std::max<int64_t>(sched.max_scope_mid, 1)));
-    const size_t pieces = (size_t)(sched.max_scope_vertices / kRunBlock + 1 + (batched ? G : 0));
-    GALP_CUDA(b_bsum.alloc(sizeof(long long) * 2 * pieces));
-    GALP_CUDA(cudaMemsetAsync(b_bsum.p, 0, sizeof(long long) * pieces, st));  // sums; then their scan
+    run_pieces = sched.max_scope_vertices / kRunBlock + 1 + (batched ? G : 0);
+    const size_t pieces = (size_t)run_pieces;
+    GALP_CUDA(b_bsum.alloc(sizeof(long long) * (2 * pieces + pieces / kScanRound + 1)));
+    GALP_CUDA(cudaMemsetAsync(b_bsum.p, 0, sizeof(long long) * pieces, st));  // sums; then their scan; then rounds
     GALP_CUDA(cudaStreamSynchronize(st));
     phase(2);
     // dispatch: static features, variant table, per-scope state, logs
@@ -761,7 +762,8 @@ PipeArgs Engine::pipe_args(const Scope &sc) const
     q.v0 = sc.v0;
     q.v1 = sc.v1;
     q.sums = (long long *)b_bsum.p;
-    q.run_at = q.sums + b_bsum.bytes / (2 * sizeof(long long));
+    q.run_at = q.sums + run_pieces;
+    q.round_sum = q.run_at + run_pieces;
     q.last_v = sc.last_v;
     for (int i = 0; i < 6; ++i) q.gcut[i] = sc.gcut[i];
     q.gstart = variant.mid_sort ? sc.gcut[3] : 0;
@@ -928,8 +930,18 @@ int Engine::enqueue_scope(cudaStream_t st, const Scope &sc, const int32_t *nbr, 
     const int64_t nv = sc.v1 - sc.v0;
     if (nv > 0) {
         const int blocks = (int)((nv + kRunBlock - 1) / kRunBlock);
-        scan_kernel<<<1, kScanThreads, 0, st>>>(q, blocks + (batched ? G : 0));
+        const int64_t pieces = (int64_t)blocks + (batched ? G : 0);
+        const int rounds = pieces > kScanOneBlock ? (int)((pieces + kScanRound - 1) / kScanRound) : 1;
+        if (rounds > 1) {
+            scan_sums_kernel<<<rounds, kScanThreads, 0, st>>>(q, (int)pieces);
+            launched("scan_sums_kernel", st);
+        }
+        scan_kernel<<<rounds, kScanThreads, 0, st>>>(q, (int)pieces);
         launched("scan_kernel", st);
+        if (rounds > 1 && batched) {
+            batch_bases_kernel<<<(unsigned)std::min<int64_t>((G + (int64_t)kTB) / kTB, (int64_t)sms * 8), kTB, 0, st>>>(q);
+            launched("batch_bases_kernel", st);
+        }
         if (batched) resolve_kernel<true><<<blocks, kTB, 0, st>>>(q);
         else resolve_kernel<false><<<blocks, kTB, 0, st>>>(q);
         launched("resolve_kernel", st);
@@ -1194,7 +1206,8 @@ int Engine::enqueue_run_incore(cudaStream_t st, int niter, long long thr)
             full_state = true;
         }
         if (batched) {  // per-graph change counts, early exits and frozen graphs
-            batch_finalize_kernel<<<1, 1024, 0, st>>>(ctl, (const int64_t *)b_g_v0.p, (int32_t *)b_g_active.p,
+            const unsigned fblocks = (unsigned)std::min<int64_t>((G + (int64_t)kFinalThreads - 1) / kFinalThreads, sms);
+            batch_finalize_kernel<<<fblocks, kFinalThreads, 0, st>>>(ctl, (const int64_t *)b_g_v0.p, (int32_t *)b_g_active.p,
                                                       (int32_t *)b_g_iters.p, (long long *)b_g_counts.p,
                                                       (unsigned long long *)b_g_changes.p, G, batch_max_iter, it,
                                                       early_exit, it + 1 < niter ? dispatch_args(it + 1) : DispatchArgs{});

@@ -234,6 +234,7 @@ struct Engine {
     int64_t *d_schunk_s0 = nullptr, *d_schunk_s1 = nullptr;
     int32_t *d_hub_p0 = nullptr, *d_hub_pcap = nullptr, *d_part_big = nullptr;
     int64_t *d_hub_pbase = nullptr;
+    int64_t run_pieces = 0;  // sums of distinct counts (PipeArgs::sums) in the largest scope
     int sms = 1;
     bool adj_sorted = false;  // every adjacency list strictly increasing (first-iteration shortcut)
     bool symmetric = false;   // edge multiset symmetric (frontier marking along out-edges)

@@ -61,7 +61,7 @@ struct Ctl {
     long long N;                // runs in the scope (written by the tile of last_v)
     long long thr;              // early-exit threshold: stop when changes <= thr
     int max_iter;               // iterations requested
-    int pad1;
+    int more;                   // batches: some graph goes on (within batch_finalize_kernel)
     unsigned long long counts[64];  // changes per iteration (the first 64)
     unsigned long long last;    // changes of the last iteration
     int tied_mid;               // tied vertices above 32 neighbours (per scope)
@@ -1152,6 +1152,7 @@ __global__ void init_ctl_kernel(Ctl *ctl, long long thr, int max_iter)
     ctl->N = 0;
     ctl->thr = thr;
     ctl->max_iter = max_iter;
+    ctl->more = 0;
     ctl->changed_n = 0;
     ctl->frontier_off = 0;
     for (int i = 0; i < 64; ++i) ctl->counts[i] = 0;

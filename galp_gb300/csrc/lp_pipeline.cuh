@@ -78,6 +78,7 @@ struct PipeArgs {
     // lies in one graph, see run_piece), zero between iterations; and their exclusive scan
     long long *sums;
     long long *run_at;
+    long long *round_sum;   // sums of kScanRound sums each, where several blocks scan
     int32_t last_v;
     // frontier mode (null = every vertex is recounted and no changes are recorded)
     const uint8_t *dirty;   // 1 = a neighbour's label changed in the previous iteration
@@ -1959,23 +1960,67 @@ __global__ void big_combine_kernel(IterArgs p, PipeArgs q)
 // scan of the distinct counts' sums
 // ---------------------------------------------------------------------------
 
-// One block: exclusive scan of the sums (which are zero again afterwards), the scope's number of
-// runs, the graphs' run bases, an empty tied list.
+// Exclusive scan of the sums (which are zero again afterwards), the scope's number of runs, the
+// graphs' run bases, an empty tied list.  Up to kScanOneBlock sums one block does it all, round
+// after round; more (whose rounds and graphs would follow one another) are scanned by a block per
+// round, from the rounds' sums (scan_sums_kernel), and the graphs' bases have a kernel of their own.
+// One block or several, us per iteration: 20 K graphs 29 and 23, 100 K 130 and 23, a million 1950
+// and 30; with fewer graphs two launches more are worth about two rounds.
 constexpr int kScanThreads = 1024;
+constexpr int kScanRound = kScanThreads * 8;
+constexpr int kScanOneBlock = 4 * kScanRound;
+
+// Run base of graph g, an empty one too: its first sum (empty graphs have one that nothing adds to)
+__device__ __forceinline__ int64_t graph_base(const PipeArgs &p, int g)
+{
+    return p.run_at[(int64_t)(p.g_v0[g] - p.v0) / kRunBlock + g];
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(PipeArgs p, int npieces)
+{
+    __shared__ long long ws[kScanThreads / 32];
+    if (!ctl_active(p.ctl)) return;
+    const int tid = threadIdx.x;
+    const int64_t i0 = (int64_t)blockIdx.x * kScanRound;
+    long long s = 0;
+#pragma unroll
+    for (int u = 0; u < kScanRound / kScanThreads; ++u) {
+        const int64_t i = i0 + u * kScanThreads + tid;
+        if (i < npieces) s += p.sums[i];
+    }
+    s = warp_sum_ll(s);
+    if ((tid & 31) == 0) ws[tid >> 5] = s;
+    __syncthreads();
+    if (tid < 32) {
+        s = warp_sum_ll(ws[tid]);
+        if (tid == 0) p.round_sum[blockIdx.x] = s;
+    }
+}
+
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(PipeArgs p, int npieces)
 {
-    constexpr int NW = kScanThreads / 32, PER = 8;
+    constexpr int NW = kScanThreads / 32, PER = kScanRound / kScanThreads;
     __shared__ long long ws[NW];
     if (!ctl_active(p.ctl)) return;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool several = gridDim.x > 1;
     long long base = 0;
-    // rounds of kScanThreads * PER sums; a warp takes 32 * PER consecutive ones, row after row
-    for (int i0 = 0; i0 < npieces; i0 += kScanThreads * PER) {
+    if (several) {  // the sums of the rounds before
+        for (int i = tid; i < (int)blockIdx.x; i += kScanThreads) base += p.round_sum[i];
+        base = warp_sum_ll(base);
+        if (lane == 0) ws[w] = base;
+        __syncthreads();
+        base = warp_sum_ll(ws[lane]);
+        __syncthreads();
+    }
+    const int64_t end = several ? min((int64_t)npieces, ((int64_t)blockIdx.x + 1) * kScanRound) : npieces;
+    // rounds of kScanRound sums; a warp takes 32 * PER consecutive ones, row after row
+    for (int64_t i0 = (int64_t)blockIdx.x * kScanRound; i0 < end; i0 += kScanRound) {
         long long x[PER], s = 0;
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-            const int i = i0 + (w * PER + u) * 32 + lane;
-            x[u] = i < npieces ? p.sums[i] : 0;
+            const int64_t i = i0 + (w * PER + u) * 32 + lane;
+            x[u] = i < end ? p.sums[i] : 0;
         }
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
@@ -1996,8 +2041,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(PipeArgs p, int npie
         all = warp_sum_ll(all);
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-            const int i = i0 + (w * PER + u) * 32 + lane;
-            if (i < npieces) {
+            const int64_t i = i0 + (w * PER + u) * 32 + lane;
+            if (i < end) {
                 p.run_at[i] = before + x[u];
                 p.sums[i] = 0;
             }
@@ -2005,15 +2050,19 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(PipeArgs p, int npie
         base += all;
         __syncthreads();
     }
-    if (tid == 0) {
+    if (blockIdx.x == gridDim.x - 1 && tid == 0) {
         p.ctl->N = base;
         p.ctl->tied_mid = 0;
     }
-    if (p.g_v0)
-        for (int g = tid; g <= p.ngraphs; g += kScanThreads) {
-            const int64_t v = p.g_v0[g];
-            p.g_base[g] = v < p.v1 ? p.run_at[run_piece(p, (int)v)] : base;
-        }
+    if (p.g_v0 && !several)
+        for (int g = tid; g <= p.ngraphs; g += kScanThreads) p.g_base[g] = g < p.ngraphs ? graph_base(p, g) : base;
+}
+
+__global__ void __launch_bounds__(kTB) batch_bases_kernel(PipeArgs p)
+{
+    if (!ctl_active(p.ctl)) return;
+    for (int64_t g = (int64_t)blockIdx.x * kTB + threadIdx.x; g <= p.ngraphs; g += (int64_t)gridDim.x * kTB)
+        p.g_base[g] = g < p.ngraphs ? graph_base(p, (int)g) : p.ctl->N;
 }
 
 // ---------------------------------------------------------------------------
@@ -2671,33 +2720,49 @@ __global__ void __launch_bounds__(kTB) batch_init_labels_kernel(const int64_t *g
 }
 
 // After an iteration of a batch: per graph, the labels that changed and the reference's early
-// exit (count <= n_g * 1e-5, dpp.cuh:88); the run goes on while some graph is active.
+// exit (count <= n_g * 1e-5, dpp.cuh:88); the run goes on while some graph is active.  One thread
+// per graph; the block that ends last keeps the run's books.
 // Also the next iteration's dispatch state, where there is one (a.out).
-__global__ void batch_finalize_kernel(Ctl *ctl, const int64_t *g_v0, int32_t *g_active, int32_t *g_iters,
-                                      long long *g_counts, unsigned long long *g_changes, int ngraphs, int max_iter,
-                                      int it, int early_exit, DispatchArgs a)
+constexpr int kFinalThreads = 1024;
+__global__ void __launch_bounds__(kFinalThreads) batch_finalize_kernel(Ctl *ctl, const int64_t *g_v0, int32_t *g_active,
+                                                                       int32_t *g_iters, long long *g_counts,
+                                                                       unsigned long long *g_changes, int ngraphs,
+                                                                       int max_iter, int it, int early_exit,
+                                                                       DispatchArgs a)
 {
-    __shared__ int any;
+    __shared__ int any, last;
+    const bool several = gridDim.x > 1;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
     const bool on = ctl_active(ctl);  // else every graph ended earlier: all is settled
-    for (int g = threadIdx.x; on && g < ngraphs; g += blockDim.x) {
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; on && g < ngraphs;
+         g += (int64_t)gridDim.x * blockDim.x) {
         if (!g_active[g]) continue;
         const unsigned long long t = g_changes[g];
         g_changes[g] = 0;
-        if (it < max_iter) g_counts[(int64_t)g * max_iter + it] = (long long)t;
+        if (it < max_iter) g_counts[g * max_iter + it] = (long long)t;
         g_iters[g] = it + 1;
         if ((early_exit && (double)t <= (double)(g_v0[g + 1] - g_v0[g]) * 1e-5) || it + 1 >= max_iter) g_active[g] = 0;
         else any = 1;
     }
     __syncthreads();
+    if (several) {
+        if (threadIdx.x == 0) {
+            if (any) atomicExch(&ctl->more, 1);
+            __threadfence();
+            last = atomicAdd(&ctl->ticket, 1ull) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+    }
     if (threadIdx.x == 0) {
         if (on) {
+            const bool more = several ? atomicExch(&ctl->more, 0) != 0 : any != 0;
             const unsigned long long c = ctl->changes;
             ctl->last = c;
             if (ctl->iter < 64) ctl->counts[ctl->iter] = c;
             ctl->iter += 1;
-            if (!any || ctl->iter >= ctl->max_iter) ctl->active = 0;
+            if (!more || ctl->iter >= ctl->max_iter) ctl->active = 0;
         }
         ctl->changes = 0;
         ctl->ticket = 0;
