@@ -137,16 +137,21 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs &a, Ctl *ctl, int *
 
 // Dynamic shared memory: the warps' tile buffers, or the block's hash table, or the resolve
 // phase's buffers.
-template <int THREADS, int ROWS>
+// The queue of tied vertices above 32 neighbours takes several rounds' worth of them: a vertex above
+// 1024 keeps its warp for up to 0.3 ms, which a block that empties the queue in every round waits
+// for in every round (600 K random vertices of 20 neighbours and 666 of 12,000, ten iterations
+// 14.2 -> 8.4 ms, separate kernels 7.6; without such vertices no change).
+template <bool BATCH, int THREADS, int ROWS>
 struct FusedResolve {
     static constexpr int kWarps = THREADS / 32;
     static constexpr int kPer = ROWS;  // vertices per thread and round
     static constexpr int kRound = kPer * THREADS;
+    static constexpr int kQueue = BATCH ? 6 * THREADS : 8 * THREADS;
     int hist[kWarps][256];
-    long long qa[kRound];   // queue of tied vertices above 32 neighbours: run base,
-    long long qN[kRound];   // (batches) its graph's runs,
-    int qv[kRound];         // vertex
-    uint8_t qf[kRound];     // (batches) 1 = last of its graph, 2 = its graph still runs
+    long long qa[kQueue];               // run base,
+    long long qN[BATCH ? kQueue : 1];   // (batches) its graph's runs,
+    int qv[kQueue];                     // vertex
+    uint8_t qf[BATCH ? kQueue : 1];     // (batches) 1 = last of its graph, 2 = its graph still runs
     uint8_t grun[THREADS];  // (batches) whether the chunk's graphs still run
 };
 union FusedTile {
@@ -160,8 +165,9 @@ constexpr int kFusedPlan = THREADS > kFusedNarrow ? 0 : 16;
 template <int THREADS>
 constexpr size_t kFusedSmem =
     kFusedTiles<THREADS> + (kFusedPlan<THREADS> ? sizeof(int32_t) * kPlanWords * (THREADS / 32) : 0);
-static_assert(sizeof(FusedResolve<kFusedNarrow, 3>) <= kFusedTiles<kFusedNarrow> &&
-                  sizeof(FusedResolve<kFusedWide, 2>) <= kFusedTiles<kFusedWide>,
+static_assert(sizeof(FusedResolve<true, kFusedNarrow, 3>) <= kFusedTiles<kFusedNarrow> &&
+                  sizeof(FusedResolve<false, kFusedNarrow, 1>) <= kFusedTiles<kFusedNarrow> &&
+                  sizeof(FusedResolve<false, kFusedWide, 2>) <= kFusedTiles<kFusedWide>,
               "the resolve buffers fit the tile buffers");
 
 // State of a vertex in the resolve phase, loaded in one round trip whether it is tied or not.
@@ -180,7 +186,7 @@ struct FusedVertex {
 template <bool BATCH, int kFusedThreads, int ROWS>
 __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a)
 {
-    using Resolve = FusedResolve<kFusedThreads, ROWS>;
+    using Resolve = FusedResolve<BATCH, kFusedThreads, ROWS>;
     constexpr int kFusedWarps = Resolve::kWarps, kPer = Resolve::kPer, kRound = Resolve::kRound;
     extern __shared__ __align__(16) unsigned char fused_smem[];
     __shared__ GroupTiles T;
@@ -500,6 +506,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
             // start of the current graph (the first graph's lies `base` runs before the chunk)
             long long start = BATCH ? -base : 0;
             if (BATCH) base = 0;
+            bool emptied = true;  // the queue, in the round before
             for (int64_t vb = v0; vb < v1; vb += kRound) {
                 if (vb > v0) load(x, vb);
                 int incl[kPer];  // distinct labels of the warp's vertices up to and with this one
@@ -517,7 +524,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                 }
                 __syncthreads();  // the sums of the round before are read
                 if (lane == 31) wsum[w] = wtotal;
-                if (tid == 0) qn = 0;
+                if (tid == 0 && emptied) qn = 0;
                 __syncthreads();
                 long long before = base;
                 for (int i = 0; i < kFusedWarps; ++i) {
@@ -597,7 +604,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a
                     }
                 }
                 __syncthreads();
-                for (int q = w; q < qn; q += kFusedWarps) {
+                emptied = vb + kRound >= v1 || qn > Resolve::kQueue - kRound;  // block-uniform
+                for (int q = w; emptied && q < qn; q += kFusedWarps) {
                     const int u = R.qv[q];
                     const RunScope rs{R.qa[q], BATCH ? R.qN[q] : runs_first, BATCH ? (R.qf[q] & 1) != 0 : u == p.last_v};
                     const bool run_u = !BATCH || (R.qf[q] & 2);

@@ -32,3 +32,12 @@ def test_few_free_blocks(blocks, times, extra):
 @pytest.mark.parametrize("size", [511, 513, 1024, 1030])
 def test_batch_rows(blocks, size):
     check_batch_rows([size] * blocks)
+
+
+@pytest.mark.parametrize("n, mid, deg", [(1 << 20, 60000, 33), (1 << 20, 15000, 130), (1 << 21, 530000, 35),
+                                         (1 << 21, 31000, 600)])
+def test_queue_of_tied_vertices(n, mid, deg):
+    # all vertices above 32 neighbours in the first blocks' chunks: more of them than the queue holds,
+    # and fewer over many rounds; both block shapes
+    degs = np.concatenate([np.full(mid, deg), np.zeros(n - mid, np.int64)])
+    _check(degs, mid, niter=3)
