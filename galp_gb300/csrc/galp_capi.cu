@@ -1013,6 +1013,8 @@ DispatchArgs Engine::dispatch_args(int it) const
 bool Engine::fused_fits() const
 {
     if (policy != 0 || n < 1 || n > kFusedMaxVertices || !sched.big_v.empty()) return false;
+    const Scope &sc = sched.scopes[0];
+    if (sc.nms + sc.nml + sc.nmx - sc.gcut[5] > kFusedLarge * std::min(sms, kFusedMaxBlocks)) return false;
     if (batched) return G <= kFusedMaxGraphs && m <= kFusedMaxBatchEntries && n <= kFusedMaxBatchVertices;
     return m <= kFusedMaxEntries && (n <= kFusedAnyVertices || m >= kFusedDense * n);
 }

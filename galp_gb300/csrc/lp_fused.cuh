@@ -58,6 +58,13 @@ constexpr int kFusedMaxBlocks = 256;
 constexpr int64_t kFusedMaxEntries = 1 << 25, kFusedMaxVertices = 1 << 21;
 constexpr int64_t kFusedAnyVertices = 1 << 20, kFusedDense = 8;
 constexpr int64_t kFusedMaxBatchEntries = 1 << 22, kFusedMaxBatchVertices = 1 << 18;
+// Vertices above kGroupMax neighbours, per multiprocessor: each takes a whole block here, four of
+// those up to 2048 share a multiprocessor in a kernel of their own.  Random graphs, ten iterations,
+// one kernel against the separate ones (ms): 4 M entries with 390 of 2,048 neighbours 1.08 and 1.27,
+// with 1,454 of 1,100 1.16 and 1.15, with 3,636 0.90 and 0.71; 20 M with 18,181 of 1,100 4.5 and 2.2,
+// with 333 of 12,000 8.0 and 7.4; LFR of 7 M with 782 0.75 and 0.94, of 24 M with 1,967 2.26 and
+// 2.17; batches of 2 M entries with 976 of 2,048 1.1 times as fast, with 1,816 of 1,100 0.88.
+constexpr int64_t kFusedLarge = 8;
 // Runs of up to kFusedClusterTiles tiles, all small or lane-group ones, are one thread-block cluster:
 // its hardware barrier replaces the counter in global memory (0.6 us less each), and the launch is
 // not cooperative.  One block per tile and the counter against the cluster (us): 512 vertices with
