@@ -991,10 +991,12 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
 {
     constexpr int NW = kSmallThreads / 32;
     __shared__ __align__(16) TileBuf stile[NW];
+    __shared__ int32_t cbuf[NW][kWarpBuf];
     if (!ctl_active(p.ctl)) return;
     const bool fr = frontier_on(p);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long changes = 0;
+    WarpBuf cb{cbuf[w]};  // changed vertices (frontier mode)
     // a block takes NW * 32 list entries per round; its warps take the quarters of a degree
     // window in turn, so that none has only the window's highest degrees
     ListWalk walk(blockIdx.x, gridDim.x, kSmallThreads, p.nsmall);
@@ -1014,8 +1016,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_
         int d = small_tile<false>(p, stile[w], hd, changes, chg);
         if (!hd.dirty) d = p.dcnt[hd.v];
         add_runs(p.sums, d ? run_piece(p, hd.v) : 0, d);
-        warp_note_changes(p, chg, hd.v);
+        if (p.changed) cb.append(chg, hd.v, p.changed, &p.ctl->changed_n);
     }
+    if (p.changed) cb.flush(p.changed, &p.ctl->changed_n);
     flush_changes(changes, p.ctl);
 }
 
@@ -2453,7 +2456,6 @@ __global__ void __launch_bounds__(kTB, kResolveBlocks) resolve_kernel(PipeArgs p
         if (small[u]) {
             if (runs[u]) p.lab_out[v] = nl[u];
             count_change(changes, nl[u], old[u]);
-            note_change(p, (int32_t)v, nl[u], old[u]);
         }
         tb.append(listed, (int32_t)v, p.tied_mid, &p.ctl->tied_mid);
         if (BATCH) {
@@ -2462,6 +2464,23 @@ __global__ void __launch_bounds__(kTB, kResolveBlocks) resolve_kernel(PipeArgs p
         }
     }
     tb.flush(p.tied_mid, &p.ctl->tied_mid);
+    if (!BATCH && p.changed) {  // the warp's changed vertices, with one addition to the list's length
+        unsigned m[PER];
+        int n = 0;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            m[u] = __ballot_sync(kFull, small[u] && nl[u] != old[u]);
+            n += __popc(m[u]);
+        }
+        int to = 0;
+        if (lane == 0 && n) to = atomicAdd(&p.ctl->changed_n, n);
+        to = __shfl_sync(kFull, to, 0);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            if ((m[u] >> lane) & 1u) p.changed[to + __popc(m[u] & ((1u << lane) - 1u))] = (int32_t)(v0 + u * 32);
+            to += __popc(m[u]);
+        }
+    }
     if (BATCH) gc.flush(p);
     flush_changes(changes, p.ctl);
 }
