@@ -891,6 +891,23 @@ __device__ __forceinline__ void plan_gather(const PipeArgs &p, const int32_t *pl
 // 297 and 277, LFR of 1.9 M entries 357 and 331.  R-MAT 24, whose warps run the same code over and
 // over, would lose: 49.9 and 50.6 ms.
 
+// A lane's at most 4 labels, gathered by itself and sorted into its row; the mask of run heads as
+// small_sort_row.  Lanes of a tile lie close together in the neighbour list, and setting up the
+// common gather costs more than the gather: ten iterations over 20 M vertices in pairs 3.6 -> 2.8 ms
+// in this kernel, in a ring 4.0 -> 3.2, in a torus 5.1 -> 3.7, with two random neighbours 6.1 -> 6.3.
+__device__ __forceinline__ uint32_t small_direct_row(const PipeArgs &p, int32_t *row, int deg, int64_t e0)
+{
+    int id[4];
+    int32_t x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) id[j] = j < deg ? ld_nbr(&p.nbr[e0 + j]) : -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = gather_label_if<false>(p.lab_in, id[j]);
+    SortNet<4>::sort(x);
+    *reinterpret_cast<int4 *>(row) = make_int4(x[0], x[1], x[2], x[3]);
+    return 1u | (x[1] != x[0] ? 2u : 0u) | (x[2] != x[1] ? 4u : 0u) | (x[3] != x[2] ? 8u : 0u);
+}
+
 // Count the warp's 32 small vertices (one per lane), with the tile buffer B (PLAN: rows in flight
 // by the tile's plan, 0 = it has none).  Writes their state and the labels of untied ones (chg: it
 // changed); returns the lane's distinct count.
@@ -904,11 +921,13 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
     constexpr bool FEW = PLAN > 0;
     int n4 = (__reduce_max_sync(kFull, deg) + 3) >> 2;
     if (FEW) n4 = (n4 + 1) & ~1;
+    const bool direct = !LIVE && n4 <= 1;  // every lane gathers its own
     if (PLAN && plan) plan_gather<PLAN ? PLAN : 4>(p, plan, B.rows, kSmallRow, 4 * n4);
-    else tile_gather<LIVE, LIVE && PLAN == 0>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
+    else if (!direct) tile_gather<LIVE, LIVE && PLAN == 0>(p, B, deg, hd.o0 - p.nbr_shift, 4 * n4);
     int32_t *row = B.rows + lane * kSmallRow;
     uint32_t h = 0u;
-    switch (n4) {  // warp-uniform
+    if (!LIVE && direct) h = small_direct_row(p, row, deg, hd.o0 - p.nbr_shift);
+    else switch (n4) {  // warp-uniform
     case 0: break;
     case 1: if (!FEW) h = small_sort_row<4>(row); break;
     case 2: h = small_sort_row<8>(row); break;
@@ -967,6 +986,9 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
             const int dg = __shfl_sync(kFull, deg, src);
             if (lane < dg) p.run_lab[e + lane] = B.rows[src * kSmallRow + lane];
         }
+    } else if (direct) {
+        if (k > 2)
+            for (int j = 0; j < deg; ++j) p.run_lab[hd.o0 - p.nbr_shift + j] = row[j];
     } else if (spill) {
         const int total = __reduce_add_sync(kFull, deg);
         const unsigned nz = __ballot_sync(kFull, deg > 0);
