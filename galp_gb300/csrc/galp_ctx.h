@@ -43,18 +43,20 @@ struct DevBuf {
     }
 };
 
-// One scope of run positions: the whole graph (policy 0) or one out-of-core batch
-// (policies 1/2; batch j = vertices [v0, v1) per OutOfCore::compute_batch_boundaries,
-// label_propagation/src/common/outofcore.cuh:38-60).
 // Scopes of up to this many CSR entries run their hub kernels, their CTA-table kernels and their
 // sorting kernels on three streams, joined before the scan.  Up to there the chain of kernels that
 // leave the chip partly idle (few hubs, last waves, launch gaps) costs more than the three slow one
 // another down; above it every kernel fills the chip and they compete for L2.  Ten iterations, one
 // stream -> three: R-MAT of 8 M entries 1.65 -> 1.21 ms, 32 M 3.6 -> 3.2, 64 M 7.1 -> 6.3, 128 M
 // 11.4 -> 10.9, 259 M 23.9 -> 24.1; sparser ones (edge factor 4) of 33 M 4.4 -> 3.8, 133 M
-// 16.3 -> 15.5, 530 M 74.6 -> 76.2; 310 out-of-core batches of 4 M entries 48.8 -> 35.7.
+// 16.3 -> 15.5, 530 M 74.6 -> 76.2; 310 out-of-core batches of 4 M entries 46.3 -> 34.5 (medians of 48
+// passes in turn on one machine; one pass in twelve takes up to four times as long on the shared
+// link, with either).
 constexpr int64_t kForkMaxEntries = 1ll << 27;
 
+// One scope of run positions: the whole graph (policy 0) or one out-of-core batch
+// (policies 1/2; batch j = vertices [v0, v1) per OutOfCore::compute_batch_boundaries,
+// label_propagation/src/common/outofcore.cuh:38-60).
 struct Scope {
     int64_t v0 = 0, v1 = 0;    // vertices
     int64_t e0 = 0, e1 = 0;    // CSR entries

@@ -25,6 +25,10 @@
 // separate kernels' code -> this (us): planted partitions of 10 K entries 158 -> 124 (115 as a cluster), 294 K 230 ->
 // 160; R-MAT 16 423 -> 342; LFR of 560 K entries 309 -> 200; batch of 96 graphs 432 -> 400 (372 with three rows per round).
 //
+// Shares of a run's time, count / wait at the barrier after it / resolve / wait: R-MAT 16 60 / 20 /
+// 13 / 8 %, the batch of 96 graphs 51 / 12 / 27 / 11, LFR of a million vertices 80 / 2 / 15 / 2,
+// planted partitions of 294 K entries 38 / 20 / 24 / 17, of 10 K 36 / 15 / 34 / 15.
+//
 // Labels, change counts, run counts and the dispatch log are those of the separate kernels.
 #pragma once
 
@@ -187,9 +191,9 @@ struct FusedVertex {
 // ROWS: vertices per thread and round of the resolve phase.  A round is a chain of loads, scans and
 // block barriers (about 5,000 cycles in batches), and rows beyond the block's vertices are paid for
 // too: batches in the narrow shape take the rows that their chunk of vertices fills, up to three.
-// One row against two or three (us): 96 graphs with 156 K vertices (1,030 a block) 400 and 369,
-// 200 graphs with 130 K (858) 351 and 340; with rows to spare 96 graphs with 22 K (142) 186, 195
-// and 212.
+// One, two and three rows (us, on the device): 96 graphs with 165 K vertices (1,086 a block) 348, 344
+// and 320, 150 with 180 K (1,186) 357, 352 and 328; 96 with 146 K (960) 285, 270 and 281, 200 with
+// 132 K (871) 287, 271 and 284; 96 with 22 K (145) 137, 145 and 160.
 template <bool BATCH, int kFusedThreads, int ROWS>
 __global__ void __launch_bounds__(kFusedThreads, 1) fused_run_kernel(FusedArgs a)
 {

@@ -822,27 +822,6 @@ __device__ __forceinline__ void tile_gather(const PipeArgs &p, TileBuf &B, int d
     __syncwarp();
 }
 
-// Small vertices (at most 32 neighbours; `small_sort` 2): a warp takes 32 vertices of about
-// equal degree (small_window_kernel), gathers their labels together and sorts each vertex's
-// labels in one lane's registers.
-//
-//   gather  32 CSR entries per row whatever vertices they belong to, eight rows in flight;
-//           the owner of an entry follows from the mask of vertex starts in its row; labels
-//           go to the owner's row of shared memory (padded with INT_MAX, no label).
-//   sort    a network sized to the warp's largest degree in steps of 4; the mask h of run
-//           heads gives everything else: d = popc(h), and the heads m of runs of maximum
-//           length W by W steps of m & (continuations >> W).
-//   spill   vertices with more than two candidates keep their sorted labels at their CSR
-//           positions and h, m in place of the candidate labels (SmallMaskQuery).
-//
-// Bound by the load/store pipe (70 % of its wavefronts on planted partitions of degree 15:
-// the label gathers alone are 32 per row), then by the latency of the two dependent loads.
-// A warp has the order of its vertices to itself, so there is no barrier between warps: a
-// version that ordered 128 vertices inside the block, with three barriers and per-lane
-// result selects, took 42 ms where this one takes 25.  Ten iterations, this kernel's share
-// (an insertion sort per thread in shared memory before): 1,024 planted partitions of
-// together 526 M entries 55.5 -> 24.9 ms, R-MAT 24 9.8 -> 4.4 ms, R-MAT 26 with edge
-// factor 4 20.2 -> 11.5 ms, LFR of a million vertices 2.0 -> 0.73 ms.
 // What a lane needs of its vertex before counting it: loaded one tile ahead.
 struct TileHead {
     int v, deg, g;  // vertex (-1 = none), its neighbours, log2 of its lanes
@@ -885,12 +864,6 @@ __device__ __forceinline__ void plan_gather(const PipeArgs &p, const int32_t *pl
     __syncwarp();
 }
 
-// Kernels that keep plans have few tiles per warp, and the straight-line code of the networks is
-// mostly fetched for one tile: they use fewer of them (rows of 8, 16, 24, 32; group rows of 32).
-// Passes with all networks and with these (us): R-MAT 14 188 and 176, R-MAT 17 with edge factor 4
-// 297 and 277, LFR of 1.9 M entries 357 and 331.  R-MAT 24, whose warps run the same code over and
-// over, would lose: 49.9 and 50.6 ms.
-
 // A lane's at most 4 labels, gathered by itself and sorted into its row; the mask of run heads as
 // small_sort_row.  Lanes of a tile lie close together in the neighbour list, and setting up the
 // common gather costs more than the gather: ten iterations over 20 M vertices in pairs 3.6 -> 2.8 ms
@@ -911,6 +884,12 @@ __device__ __forceinline__ uint32_t small_direct_row(const PipeArgs &p, int32_t 
 // Count the warp's 32 small vertices (one per lane), with the tile buffer B (PLAN: rows in flight
 // by the tile's plan, 0 = it has none).  Writes their state and the labels of untied ones (chg: it
 // changed); returns the lane's distinct count.
+//
+// Kernels that keep plans have few tiles per warp, and the straight-line code of the networks is
+// mostly fetched for one tile: they use fewer of them (rows of 8, 16, 24, 32; group rows of 32).
+// Passes with all networks and with these (us): R-MAT 14 188 and 176, R-MAT 17 with edge factor 4
+// 297 and 277, LFR of 1.9 M entries 357 and 331.  R-MAT 24, whose warps run the same code over and
+// over, would lose: 49.9 and 50.6 ms.
 template <bool LIVE, int PLAN = 0>
 __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const TileHead &hd,
                                           unsigned long long &changes, bool &chg, const int32_t *plan = nullptr)
@@ -1007,6 +986,28 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
     return __popc(h);
 }
 
+// Small vertices (at most 32 neighbours; `small_sort` 2): a warp takes 32 vertices of about
+// equal degree (small_window_kernel), gathers their labels together and sorts each vertex's
+// labels in one lane's registers.
+//
+//   gather  32 CSR entries per row whatever vertices they belong to, eight rows in flight;
+//           the owner of an entry follows from the mask of vertex starts in its row; labels
+//           go to the owner's row of shared memory (padded with INT_MAX, no label).  Tiles of
+//           at most four neighbours each: small_direct_row.
+//   sort    a network sized to the warp's largest degree in steps of 4; the mask h of run
+//           heads gives everything else: d = popc(h), and the heads m of runs of maximum
+//           length W by W steps of m & (continuations >> W).
+//   spill   vertices with more than two candidates keep their sorted labels at their CSR
+//           positions and h, m in place of the candidate labels (SmallMaskQuery).
+//
+// Bound by the load/store pipe (70 % of its wavefronts on planted partitions of degree 15:
+// the label gathers alone are 32 per row), then by the latency of the two dependent loads.
+// A warp has the order of its vertices to itself, so there is no barrier between warps: a
+// version that ordered 128 vertices inside the block, with three barriers and per-lane
+// result selects, took 42 ms where this one takes 25.  Ten iterations, this kernel's share
+// (an insertion sort per thread in shared memory before): 1,024 planted partitions of
+// together 526 M entries 55.5 -> 24.9 ms, R-MAT 24 9.8 -> 4.4 ms, R-MAT 26 with edge
+// factor 4 20.2 -> 11.5 ms, LFR of a million vertices 2.0 -> 0.73 ms.
 constexpr int kSmallThreads = 128;
 constexpr int kSmallBlocks = 8;  // resident blocks per SM
 __global__ void __launch_bounds__(kSmallThreads, kSmallBlocks) count_small_sort_kernel(PipeArgs p)
