@@ -957,6 +957,7 @@ __device__ __forceinline__ int small_tile(const PipeArgs &p, TileBuf &B, const T
     unsigned spill = __ballot_sync(kFull, k > 2);
     if (PLAN && plan) {
         // one vertex after the other (the owners of slots are not at hand)
+        __syncwarp();  // every lane's row is sorted (the vote does not order shared memory)
 #pragma unroll 1
         while (spill) {
             const int src = __ffs(spill) - 1;
